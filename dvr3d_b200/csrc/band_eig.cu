@@ -15,10 +15,9 @@
 //                    entry, is applied from the left to the rest of O_s, from both sides to
 //                    D_s and from the right to O_{s+1}; the remainder of the bulge is
 //                    eliminated by later sweeps.
-// One CTA owns a whole sweep (five warps with fixed roles, 32 x 32 blocks in shared memory,
-// lane = row), keeping O_{s+1} between its tasks. Sweep j+1 may start task s once sweep j has
-// written the beta of its task s + 2 (the only entry the two share), published through
-// per-sweep progress counters with release / acquire ordering and bounded waits.
+// One CTA owns a whole sweep, keeping O_{s+1} between its tasks. Sweep j+1 may start task s once
+// sweep j has written the beta of its task s + 2 (the only entry the two share), published
+// through per-sweep progress counters with release / acquire ordering and bounded waits.
 // Back-transformation: Q = prod over sweeps (in order) of prod over tasks of H; the
 // reflectors of one sweep act on disjoint rows, so a CTA holding a slab of eigenvector
 // columns in shared memory applies sweep after sweep (last first), its warps taking the
@@ -34,9 +33,7 @@ namespace {
 
 constexpr int kBW = kBandMaxBw;
 constexpr int kTS = kBW + 1;            // shared-memory row stride of a block
-constexpr int kChaseThreads = 160;      // five warps per sweep in flight
 constexpr int kBlk = kBW * kTS;         // doubles of one 32 x 32 block in shared memory
-constexpr size_t kChaseSmem = ((size_t)6 * kBlk + 3 * kBW) * sizeof(double);
 constexpr unsigned long long kSpinLimit = 1ull << 24;
 constexpr unsigned kFull = 0xffffffffu;
 
@@ -78,234 +75,319 @@ __global__ void band_prepare_kernel(double *A, long long lda, int n, int b, unsi
     }
 }
 
-// Householder reflector of x (lanes 0..L-1): H x = beta e_0, v[0] = 1.
-__device__ __forceinline__ void warp_house(double x, int lane, int L, double &v, double &tau, double &beta) {
-    const double alpha = __shfl_sync(kFull, x, 0);
-    const double sig = warp_sum((lane >= 1 && lane < L) ? x * x : 0.0);
+// Reflector of a task from its column x (x_0 = alpha, sig = sum of the other squares):
+// H = I - tau v v^T, v = (1, sc x_1, sc x_2, ...), H x = beta e_0.
+__device__ __forceinline__ void house_scalars(double alpha, double sig, double &tau, double &beta, double &sc) {
     tau = 0.0;
     beta = alpha;
-    v = (lane == 0) ? 1.0 : 0.0;
+    sc = 0.0;
     if (sig != 0.0) {
         beta = -copysign(sqrt(alpha * alpha + sig), alpha);
+        sc = 1.0 / (alpha - beta);
         tau = (beta - alpha) / beta;
-        const double sc = 1.0 / (alpha - beta);
-        v = (lane == 0) ? 1.0 : ((lane < L) ? x * sc : 0.0);
     }
 }
 
-// One CTA per sweep in flight, five warps with fixed roles per task s:
-//   warp 0: the reflector (from column j or the bulge's first column); its beta is written
-//           and the task published to the next sweep at once (the next sweep's task s-2,
-//           which this publication releases, shares only that entry with task s); then
-//           O_s <- H O_s, written back;
-//   warp 1: D_s <- H D_s H, written back (lower triangle);
-//   warp 2: O_{s+1} <- O_{s+1} H, kept in shared memory for task s+1;
-//   warps 3, 4: wait for the previous sweep and load task s+1's O_{s+2} and D_{s+1}.
-// Warps 0-2 start after the reflector is in shared memory; all five meet at the end of the
-// task, so a publication also covers everything of the earlier tasks. The last task of a
-// sweep is published only when all its parts are written.
-__global__ void __launch_bounds__(kChaseThreads) band_chase_kernel(BandTri t) {
-    extern __shared__ double sm[];
-    double *Ob = sm;                   // [2] O_s (held from the previous task) / O_{s+1}
-    double *Dr = sm + 2 * kBlk;        // [2] D_s as loaded (lower triangle, zeros elsewhere)
-    double *Orw = sm + 4 * kBlk;       // [2] O_{s+1} as loaded
-    double *Xr = sm + 6 * kBlk;        // column j below the diagonal (task 0)
-    double *vsm = Xr + kBW;            // reflector
-    double *wsm = vsm + kBW;           // w of the diagonal-block update
-    __shared__ double s_tau, s_beta;
-    __shared__ int s_abort;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+// One CTA per sweep in flight. The band lives in compact storage (kBandLd doubles a column, both
+// triangles within b of the diagonal, bulge space below): element (i, j) at C[j (kBandLd - 1) + i +
+// kBW], so a column window is contiguous, nothing is clamped at the matrix end (zero padding) and
+// the whole band stays in L2.
+// The chase is a dependency chain, so everything is arranged around its length. Task s needs the
+// column x that task s - 1 leaves in the bulge; all matrix-vector products of the task are formed
+// with x itself (O x, D x, O^T x) beside the norm of x, and the reflector's three scalars are
+// computed by every warp for itself, so one barrier (X) a task is all that stands between x and
+// the next x. 18 warps:
+//   L D (4)  wait for the previous sweep's flag, load task s+1's D and O into registers, then into
+//            the raw buffer that task s-1 has left (barrier E);
+//   O (4)    O_{s+1} <- O_{s+1} H: eight rows a warp, four lanes a row; the first column is the
+//            next x, written first with its partial norms; the whole block goes to shared memory;
+//   D (4)    D_s <- H D_s H, kept as a full symmetric block, to global memory;
+//   L (4)    O_s <- H O_s (the bulge), to global memory, its first row mirrored above the diagonal;
+//   P1       the reflector for the back-transformation, beta;
+//   P2       publishes: flag f = reflector f-1 known (beta written) and tasks < f-1 complete
+//            (counters in shared memory), the release off the chain.
+// Sweep j+1 runs task s once sweep j's flag reaches s + 3: its blocks were completed by task s+1
+// and the one entry that task s+2 changes is its beta. Sweeps follow one another at
+// (task time) + (flag, fence and load latency): 2656 columns of half-bandwidth 32 (the projected
+// matrix of 500 levels) take 17.7 ms, against 27.8 ms for five warps with the reflector broadcast
+// through a second barrier and the blocks at the matrix's own stride; 12202 columns 119 ms. Of a
+// task's 3400 cycles the D warps need 3000; fence, flag and loads take 1000 + 1900 + 1500.
+constexpr int kChaseThreads = 18 * 32;
+constexpr int kBarX = 1, kBarE = 3, kBarD = 5;
+
+__device__ __forceinline__ void bar_sync(int id, int count) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(count) : "memory"); }
+__device__ __forceinline__ void bar_arrive(int id, int count) { asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(count) : "memory"); }
+
+struct ChaseSmem {
+    double raw[2][2][kBlk];  // [buffer][D, O_{s+1}] as loaded
+    double bulge[2][kBlk];   // O_s after the right-hand update
+    double x[2][kBW];        // the task's column
+    double part[2][4];       // its sum of squares without x_0, eight rows each
+    double ya[kBW], p2[4];   // D x and x^T D x (without x_0)
+    volatile int done[8];    // tasks completed by each of the D and L warps
+    volatile int refl;       // reflectors known
+    volatile int abort;
+};
+
+__global__ void __launch_bounds__(kChaseThreads, 1) band_chase_kernel(BandTri t) {
+    extern __shared__ __align__(16) unsigned char chase_sm[];
+    ChaseSmem &S = *reinterpret_cast<ChaseSmem *>(chase_sm);
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, role = warp >> 2, w = warp & 3;
     const int n = t.n, b = t.b;
-    const long long ld = t.lda;
+    constexpr long long ld = kBandLd - 1;
+    constexpr int nX = 17 * 32, nE = 12 * 32;  // X: all but P2; E: O, D and the loaders
     const unsigned long long spin_limit = t.wait_limit ? t.wait_limit : kSpinLimit;
-    double *A = t.A;
-    for (int q = tid; q < 6 * kBlk + 3 * kBW; q += kChaseThreads) sm[q] = 0.0;
-    if (tid == 0) s_abort = 0;
-    __syncthreads();
-    long long pc[5] = {0, 0, 0, 0, 0};
-    long long tlast = clock64();
-    auto mark = [&](int ph) {
-        if (t.prof) {
-            const long long now = clock64();
-            pc[ph] += now - tlast;
-            tlast = now;
-        }
-    };
-    // warps 3 (which = 0: O_{s+1}, and column j for task 0) and 4 (which = 1: D_s): wait
-    // until sweep j-1 has published `need` tasks, then load task s's block
-    auto load_task = [&](int j, int s, int buf, int need, int which) {
-        if (j > 0) {
-            int ok = 1;
-            if (lane == 0) {
-                unsigned long long spins = 0;
-                while (ld_acquire_u32(t.progress + j - 1) < (unsigned)need) {
-                    if (++spins > spin_limit) {
-                        atomicExch(t.err, (int)kDevBarrierTimeout);
-                        ok = 0;
-                        break;
-                    }
-                    if ((spins & 255ull) == 0 && *(volatile int *)t.err != 0) {
-                        ok = 0;
-                        break;
-                    }
-                    if (spins > 32) __nanosleep(32);
-                }
-            }
-            ok = __shfl_sync(kFull, ok, 0);
-            if (!ok) {
-                if (lane == 0) s_abort = 1;
-                return;
-            }
-        }
-        __syncwarp();
-        const int r0 = j + 1 + s * b, L = min(b, n - r0);
-        const int r1 = r0 + b, L1 = (r1 < n) ? min(b, n - r1) : 0;
-        const int rl = min(r0 + lane, n - 1), rl1 = min(r1 + lane, n - 1);
-        double val[kBW];
-        if (which == 1) {
-#pragma unroll
-            for (int c = 0; c < kBW; ++c) {
-                const double a0 = __ldcg(A + (size_t)min(r0 + c, n - 1) * ld + rl);
-                val[c] = (c < L && lane >= c && lane < L) ? a0 : 0.0;
-            }
-            double *D = Dr + buf * kBlk;
-#pragma unroll
-            for (int c = 0; c < kBW; ++c) D[lane * kTS + c] = val[c];
-        } else {
-#pragma unroll
-            for (int c = 0; c < kBW; ++c) {
-                const double a1 = __ldcg(A + (size_t)min(r0 + c, n - 1) * ld + rl1);
-                val[c] = (c < b && lane < L1) ? a1 : 0.0;
-            }
-            if (s == 0) {
-                const double xv = __ldcg(A + (size_t)j * ld + rl);
-                Xr[lane] = (lane < L) ? xv : 0.0;
-            }
-            double *O = Orw + buf * kBlk;
-#pragma unroll
-            for (int c = 0; c < kBW; ++c) O[lane * kTS + c] = val[c];
-        }
-    };
+    double *A = t.C + kBW;
+    if (tid == 0) S.abort = 0;
+    int q = 0;  // tasks of this CTA so far: the parity of buffers and barriers
     for (int j = blockIdx.x; j <= n - 3; j += gridDim.x) {
         const int nt = band_ntask(n, b, j);
         const int ntp = (j > 0) ? band_ntask(n, b, j - 1) : 0;
-        if (warp >= 3) load_task(j, 0, 0, min(3, ntp), warp - 3);
+        if (tid < 8) S.done[tid] = 0;
+        if (tid == 8) S.refl = 0;
         __syncthreads();
-        if (s_abort) return;
-        mark(0);
-        for (int s = 0; s < nt; ++s) {
-            const int cur = s & 1;
-            const int r0 = j + 1 + s * b, L = min(b, n - r0);
-            const int r1 = r0 + b, L1 = (r1 < n) ? min(b, n - r1) : 0;
-            double *Oc = Ob + cur * kBlk, *On = Ob + (cur ^ 1) * kBlk;
-            const double *Dc = Dr + cur * kBlk, *Oraw = Orw + cur * kBlk;
-            if (warp == 0) {
-                const double x = (s == 0) ? Xr[lane] : ((lane < L) ? Oc[lane * kTS] : 0.0);
-                double v, tau, beta;
-                warp_house(x, lane, L, v, tau, beta);
-                vsm[lane] = v;
-                // beta at once, then the publication (the rest of O_s follows below). The
-                // release store is cumulative over the earlier tasks' writes of every warp,
-                // which the end-of-task barrier ordered before it.
-                if (lane == 0) {
-                    s_tau = tau;
-                    s_beta = beta;
-                    if (s == 0) A[(size_t)j * ld + r0] = beta;
-                    else A[(size_t)(r0 - b) * ld + r0] = beta;
-                    if (s + 1 < nt) st_release_u32(t.progress + j, (unsigned)(s + 1));
-                    t.taus[(size_t)j * t.ntmax + s] = tau;
+        if (S.abort) return;
+        if (role == 0) {
+            // ---- loaders: columns 8w .. 8w+7, lane = row
+            unsigned seen = (j > 0) ? 0u : 0xffffffffu;
+            for (int s = 0; s < nt; ++s) {
+                const int pb = (q + s) & 1;
+                const unsigned need = (unsigned)min(s + 3, ntp + 1);
+                if (seen < need && !S.abort) {
+                    unsigned f = 0;
+                    int ok = 1;
+                    if (lane == 0) {
+                        unsigned long long spins = 0;
+                        while ((f = ld_acquire_u32(t.progress + j - 1)) < need) {
+                            if (++spins > spin_limit) {
+                                atomicExch(t.err, (int)kDevBarrierTimeout);
+                                ok = 0;
+                                break;
+                            }
+                            if ((spins & 255ull) == 0 && *(volatile int *)t.err != 0) {
+                                ok = 0;
+                                break;
+                            }
+                        }
+                        if (!ok) S.abort = 1;  // this sweep runs on without waits; all leave at its end
+                    }
+                    seen = __shfl_sync(kFull, f, 0);
                 }
-                t.vs[((size_t)j * t.ntmax + s) * kBW + lane] = v;
-            }
-            __syncthreads();
-            mark(1);
-            const double tau = s_tau;
-            const double vme = vsm[lane];
-            if (warp == 0) {
+                __syncwarp();
+                const int r0 = j + 1 + s * b, L = min(b, n - r0), r1 = r0 + b, L1 = min(b, n - r1);
+                double dv[8], ov[8], xv = 0.0;
+#pragma unroll
+                for (int k = 0; k < 8; ++k) {
+                    const int c = 8 * w + k;
+                    const double *col = A + (long long)(r0 + c) * ld;
+                    dv[k] = (c < L && lane < L) ? __ldcg(col + r0 + lane) : 0.0;
+                    ov[k] = (c < L && lane < L1) ? __ldcg(col + r1 + lane) : 0.0;
+                }
+                if (s == 0 && lane < 8 && 8 * w + lane < L) xv = __ldcg(A + (long long)j * ld + r0 + 8 * w + lane);
+                if (q + s >= 2) bar_sync(kBarE + pb, nE);
+                double *D = S.raw[pb][0], *O = S.raw[pb][1];
+#pragma unroll
+                for (int k = 0; k < 8; ++k) {
+                    D[lane * kTS + 8 * w + k] = dv[k];
+                    O[lane * kTS + 8 * w + k] = ov[k];
+                }
                 if (s == 0) {
-                    if (lane < L) A[(size_t)j * ld + r0 + lane] = (lane == 0) ? s_beta : 0.0;
-                } else {
-                    // O_s <- H O_s (lane = column; v is zero past row L)
-                    double z0 = 0.0, z1 = 0.0, z2 = 0.0, z3 = 0.0;
-#pragma unroll
-                    for (int l = 0; l < kBW; l += 4) {
-                        z0 += vsm[l] * Oc[l * kTS + lane];
-                        z1 += vsm[l + 1] * Oc[(l + 1) * kTS + lane];
-                        z2 += vsm[l + 2] * Oc[(l + 2) * kTS + lane];
-                        z3 += vsm[l + 3] * Oc[(l + 3) * kTS + lane];
-                    }
-                    const double z = (lane >= 1 && lane < b) ? tau * ((z0 + z1) + (z2 + z3)) : 0.0;
-#pragma unroll
-                    for (int l = 0; l < kBW; ++l) Oc[l * kTS + lane] -= vsm[l] * z;
-                    __syncwarp();
-                    if (lane < L) Oc[lane * kTS] = (lane == 0) ? s_beta : 0.0;
-                    __syncwarp();
-                    if (lane < L) {
-                        double *dst = A + (size_t)(r0 - b) * ld + r0 + lane;
-                        for (int c = 0; c < b; ++c) dst[(size_t)c * ld] = Oc[lane * kTS + c];
-                    }
+                    if (lane < 8) S.x[pb][8 * w + lane] = xv;
+                    double sq = (w == 0 && lane == 0) ? 0.0 : xv * xv;
+                    sq += __shfl_xor_sync(kFull, sq, 4);
+                    sq += __shfl_xor_sync(kFull, sq, 2);
+                    sq += __shfl_xor_sync(kFull, sq, 1);
+                    if (lane == 0) S.part[pb][w] = sq;
                 }
-            } else if (warp == 1) {
-                if (tau != 0.0) {
-                    // y_l = sum_c (D[l][c] + D[c][l]) v_c - D[l][l] v_l
-                    double y0 = 0.0, y1 = 0.0, y2 = 0.0, y3 = 0.0;
-#pragma unroll
-                    for (int c = 0; c < kBW; c += 4) {
-                        y0 += (Dc[lane * kTS + c] + Dc[c * kTS + lane]) * vsm[c];
-                        y1 += (Dc[lane * kTS + c + 1] + Dc[(c + 1) * kTS + lane]) * vsm[c + 1];
-                        y2 += (Dc[lane * kTS + c + 2] + Dc[(c + 2) * kTS + lane]) * vsm[c + 2];
-                        y3 += (Dc[lane * kTS + c + 3] + Dc[(c + 3) * kTS + lane]) * vsm[c + 3];
-                    }
-                    const double y = ((y0 + y1) + (y2 + y3)) - Dc[lane * kTS + lane] * vme;
-                    const double K = warp_sum(vme * y);
-                    const double w = tau * y - 0.5 * tau * tau * K * vme;
-                    wsm[lane] = w;
-                    __syncwarp();
-                    if (lane < L) {
-                        double *dst = A + (size_t)r0 * ld + r0 + lane;
-#pragma unroll
-                        for (int c = 0; c < kBW; ++c)
-                            if (c <= lane) dst[(size_t)c * ld] = Dc[lane * kTS + c] - (vme * wsm[c] + w * vsm[c]);
-                    }
-                }
-            } else if (warp == 2) {
-                if (L1 > 0) {
-                    double u0 = 0.0, u1 = 0.0, u2 = 0.0, u3 = 0.0;
-#pragma unroll
-                    for (int c = 0; c < kBW; c += 4) {
-                        u0 += Oraw[lane * kTS + c] * vsm[c];
-                        u1 += Oraw[lane * kTS + c + 1] * vsm[c + 1];
-                        u2 += Oraw[lane * kTS + c + 2] * vsm[c + 2];
-                        u3 += Oraw[lane * kTS + c + 3] * vsm[c + 3];
-                    }
-                    const double u = tau * ((u0 + u1) + (u2 + u3));
-#pragma unroll
-                    for (int c = 0; c < kBW; ++c) On[lane * kTS + c] = Oraw[lane * kTS + c] - u * vsm[c];
-                }
-            } else {
-                if (s + 1 < nt) load_task(j, s + 1, cur ^ 1, min(s + 4, ntp), warp - 3);
+                bar_arrive(kBarX + pb, nX);
             }
-            mark(2);
-            __syncthreads();
-            if (s_abort) return;
-            mark(3);
-            if (s + 1 == nt && tid == 0) {
-                __threadfence();
-                st_release_u32(t.progress + j, (unsigned)nt);
+        } else if (warp < 17) {
+            const int rr = lane & 7, cg = lane >> 3, r = 8 * w + rr;
+            for (int s = 0; s < nt; ++s) {
+                const int pb = (q + s) & 1;
+                const int r0 = j + 1 + s * b, L = min(b, n - r0);
+                bar_sync(kBarX + pb, nX);
+                const double *x = S.x[pb];
+                const double alpha = x[0], sig = (S.part[pb][0] + S.part[pb][1]) + (S.part[pb][2] + S.part[pb][3]);
+                if (role == 1) {
+                    // ---- O_{s+1} <- O_{s+1} H
+                    const double *R = S.raw[pb][1] + r * kTS;
+                    double o[8], xc[8], a0 = 0.0, a1 = 0.0;
+                    const double o0 = R[0];
+#pragma unroll
+                    for (int k = 0; k < 8; ++k) {
+                        o[k] = R[8 * cg + k];
+                        xc[k] = (k == 0 && cg == 0) ? 0.0 : x[8 * cg + k];
+                    }
+#pragma unroll
+                    for (int k = 0; k < 8; k += 2) {
+                        a0 = fma(o[k], xc[k], a0);
+                        a1 = fma(o[k + 1], xc[k + 1], a1);
+                    }
+                    double a = a0 + a1;
+                    a += __shfl_xor_sync(kFull, a, 8);
+                    a += __shfl_xor_sync(kFull, a, 16);
+                    double tau, beta, sc;
+                    house_scalars(alpha, sig, tau, beta, sc);
+                    const double tu = tau * fma(sc, a, o0);
+                    const double xn = o0 - tu;
+                    if (cg == 0) S.x[pb ^ 1][r] = xn;
+                    double sq = (r == 0) ? 0.0 : xn * xn;
+                    sq += __shfl_xor_sync(kFull, sq, 4);
+                    sq += __shfl_xor_sync(kFull, sq, 2);
+                    sq += __shfl_xor_sync(kFull, sq, 1);
+                    if (lane == 0) S.part[pb ^ 1][w] = sq;
+                    double *B = S.bulge[pb ^ 1] + r * kTS + 8 * cg;
+                    const double tus = tu * sc;
+#pragma unroll
+                    for (int k = 0; k < 8; ++k) B[k] = (k == 0 && cg == 0) ? xn : fma(-tus, xc[k], o[k]);
+                    bar_arrive(kBarE + pb, nE);
+                } else if (role == 2) {
+                    // ---- D_s <- H D_s H
+                    const double *R = S.raw[pb][0];
+                    double d[8], xc[8], a0 = 0.0, a1 = 0.0;
+                    const double xr = (r == 0) ? 0.0 : x[r], d0 = R[r * kTS], d00 = R[0];
+#pragma unroll
+                    for (int k = 0; k < 8; ++k) {
+                        d[k] = R[r * kTS + 8 * cg + k];
+                        xc[k] = (k == 0 && cg == 0) ? 0.0 : x[8 * cg + k];
+                    }
+#pragma unroll
+                    for (int k = 0; k < 8; k += 2) {
+                        a0 = fma(d[k], xc[k], a0);
+                        a1 = fma(d[k + 1], xc[k + 1], a1);
+                    }
+                    double a = a0 + a1;
+                    a += __shfl_xor_sync(kFull, a, 8);
+                    a += __shfl_xor_sync(kFull, a, 16);
+                    if (cg == 0) S.ya[r] = a;
+                    double p = xr * a;
+                    p += __shfl_xor_sync(kFull, p, 4);
+                    p += __shfl_xor_sync(kFull, p, 2);
+                    p += __shfl_xor_sync(kFull, p, 1);
+                    if (lane == 0) S.p2[w] = p;
+                    bar_sync(kBarD, 4 * 32);
+                    double tau, beta, sc;
+                    house_scalars(alpha, sig, tau, beta, sc);
+                    const double p2 = (S.p2[0] + S.p2[1]) + (S.p2[2] + S.p2[3]);
+                    // v^T D v with v = e_0 + sc x
+                    const double K = fma(sc, fma(sc, p2, 2.0 * S.ya[0]), d00);
+                    const double hk = 0.5 * tau * tau * K;
+                    const double vr = (r == 0) ? 1.0 : sc * xr;
+                    const double wr = fma(-hk, vr, tau * fma(sc, a, d0));
+                    double *dst = A + (long long)(r0 + 8 * cg) * ld + r0 + r;
+#pragma unroll
+                    for (int k = 0; k < 8; ++k) {
+                        const double vc = (k == 0 && cg == 0) ? 1.0 : sc * xc[k];
+                        const double wc = fma(-hk, vc, tau * fma(sc, S.ya[8 * cg + k], R[(8 * cg + k) * kTS]));
+                        // the same rounding for (r, c) and (c, r): the block stays symmetric
+                        const double g = __dadd_rn(__dmul_rn(vr, wc), __dmul_rn(wr, vc));
+                        if (r < L && 8 * cg + k < L) dst[(long long)k * ld] = d[k] - g;
+                    }
+                    bar_arrive(kBarE + pb, nE);
+                    __syncwarp();
+                    if (lane == 0) {
+                        __threadfence_block();
+                        S.done[w] = s + 1;
+                    }
+                } else if (role == 3) {
+                    // ---- O_s <- H O_s: columns 8w .. 8w+7, four lanes a column
+                    if (s > 0) {
+                        const int c = 8 * w + (lane >> 2), rg = lane & 3;
+                        const double *B = S.bulge[pb] + c;
+                        double o[8], xk[8], z0 = 0.0, z1 = 0.0;
+                        const double o0 = B[0];
+#pragma unroll
+                        for (int k = 0; k < 8; ++k) {
+                            o[k] = B[(rg + 4 * k) * kTS];
+                            xk[k] = (k == 0 && rg == 0) ? 0.0 : x[rg + 4 * k];
+                        }
+#pragma unroll
+                        for (int k = 0; k < 8; k += 2) {
+                            z0 = fma(o[k], xk[k], z0);
+                            z1 = fma(o[k + 1], xk[k + 1], z1);
+                        }
+                        double z = z0 + z1;
+                        z += __shfl_xor_sync(kFull, z, 1);
+                        z += __shfl_xor_sync(kFull, z, 2);
+                        double tau, beta, sc;
+                        house_scalars(alpha, sig, tau, beta, sc);
+                        const double tz = tau * fma(sc, z, o0);
+                        const double tzs = tz * sc;
+                        if (c < b) {
+                            double *dst = A + (long long)(r0 - b + c) * ld + r0;
+#pragma unroll
+                            for (int k = 0; k < 8; ++k) {
+                                const int row = rg + 4 * k;
+                                double v = (row == 0) ? o[k] - tz : fma(-tzs, xk[k], o[k]);
+                                if (c == 0) v = (row == 0) ? beta : 0.0;
+                                if (row < L) dst[row] = v;
+                                if (row == 0) A[(long long)r0 * ld + (r0 - b + c)] = v;
+                            }
+                        }
+                        __syncwarp();
+                    }
+                    if (lane == 0) {
+                        __threadfence_block();
+                        S.done[4 + w] = s + 1;
+                    }
+                } else {
+                    // ---- P1: the reflector and beta
+                    double tau, beta, sc;
+                    house_scalars(alpha, sig, tau, beta, sc);
+                    if (s == 0) {
+                        if (lane < L) A[(long long)j * ld + r0 + lane] = (lane == 0) ? beta : 0.0;
+                    } else if (lane == 0) {
+                        A[(long long)(r0 - b) * ld + r0] = beta;
+                    }
+                    __syncwarp();
+                    if (lane == 0) {
+                        __threadfence_block();
+                        S.refl = s + 1;
+                    }
+                    if (t.vs) {
+                        t.vs[((size_t)j * t.ntmax + s) * kBW + lane] = (lane == 0) ? 1.0 : sc * x[lane];
+                        if (lane == 0) t.taus[(size_t)j * t.ntmax + s] = tau;
+                    }
+                }
+            }
+        } else {
+            // ---- P2: publication
+            int pub = 0;
+            while (pub <= nt) {
+                int v = (lane < 8) ? S.done[lane] : 0x7fffffff;
+                v = __reduce_min_sync(kFull, v);
+                const int refl = S.refl;
+                const int f = __shfl_sync(kFull, (v >= nt) ? nt + 1 : min(refl, v + 1), 0);
+                if (f > pub) {
+                    pub = f;
+                    if (lane == 0) {
+                        __threadfence_block();  // the counters' values before the release, which covers their writers' stores
+                        st_release_u32(t.progress + j, (unsigned)f);
+                    }
+                }
             }
         }
-    }
-    if (t.prof && tid == 0) {
-#pragma unroll
-        for (int q = 0; q < 5; ++q) atomicAdd(reinterpret_cast<unsigned long long *>(t.prof + q), (unsigned long long)pc[q]);
+        q += nt;
+        __syncthreads();
     }
 }
 
-__global__ void band_diag_kernel(const double *A, long long lda, int n, double *d, double *e) {
+// The band of a symmetric matrix (lower triangle read) into the chase's compact storage: both
+// triangles within b of the diagonal, zeros elsewhere, kBW zero columns at the end.
+__global__ void band_compact_kernel(const double *A, long long lda, int n, int b, double *C) {
+    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= (long long)(n + kBW) * kBandLd) return;
+    const int j = (int)(t / kBandLd), i = j + (int)(t % kBandLd) - kBW;
+    const int lo = min(i, j), hi = max(i, j);
+    C[t] = (lo >= 0 && hi < n && hi - lo <= b) ? A[(size_t)lo * lda + hi] : 0.0;
+}
+
+__global__ void band_diag_kernel(const double *C, int n, double *d, double *e) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    d[i] = A[(size_t)i * lda + i];
-    e[i] = (i + 1 < n) ? A[(size_t)i * lda + i + 1] : 0.0;
+    d[i] = C[(size_t)i * kBandLd + kBW];
+    e[i] = (i + 1 < n) ? C[(size_t)i * kBandLd + kBW + 1] : 0.0;
 }
 
 // Back-transformation, COLS eigenvector columns per CTA held in shared memory (column c at
@@ -424,16 +506,25 @@ cudaError_t launch_band_prepare(double *A, long long lda, int n, int b, unsigned
     return cudaGetLastError();
 }
 
+size_t band_compact_doubles(int n) { return (size_t)(n + kBW) * kBandLd; }
+
+cudaError_t launch_band_compact(const double *A, long long lda, int n, int b, double *C, cudaStream_t st) {
+    const long long tot = (long long)(n + kBW) * kBandLd;
+    DVR3D_COUNT_LAUNCH(1);
+    band_compact_kernel<<<(unsigned)((tot + 255) / 256), 256, 0, st>>>(A, lda, n, b, C);
+    return cudaGetLastError();
+}
+
 cudaError_t launch_band_chase(BandTri &t, cudaStream_t st) {
     if (t.b < 1 || t.b > kBW || t.n < 3) return cudaErrorInvalidValue;
     t.ntmax = band_ntask(t.n, t.b, 0);
     cudaError_t e = cudaMemsetAsync(t.progress, 0, sizeof(unsigned) * t.n, st);
     if (e != cudaSuccess) return e;
-    const size_t smem = kChaseSmem;
+    const size_t smem = sizeof(ChaseSmem);
     e = cudaFuncSetAttribute(band_chase_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    // one CTA per sweep in flight: sweeps start about three tasks apart and a CTA is busy
-    // for ntask tasks, so ntask / 3 plus slack keeps every sweep's successor supplied
+    // one CTA per sweep in flight: sweeps follow at least three tasks apart and a CTA is busy
+    // for ntask tasks, so ntask / 2 plus slack keeps every sweep's successor supplied
     int grid = std::min(t.n - 2, std::max(8, t.ntmax / 2 + 8));
     int dev = 0, nsm = 0, per = 0;
     cudaGetDevice(&dev);
@@ -445,7 +536,7 @@ cudaError_t launch_band_chase(BandTri &t, cudaStream_t st) {
     e = cudaLaunchCooperativeKernel((void *)band_chase_kernel, dim3(grid), dim3(kChaseThreads), args, smem, st);
     if (e != cudaSuccess) return e;
     DVR3D_COUNT_LAUNCH(1);
-    band_diag_kernel<<<(t.n + 255) / 256, 256, 0, st>>>(t.A, t.lda, t.n, t.d, t.e);
+    band_diag_kernel<<<(t.n + 255) / 256, 256, 0, st>>>(t.C, t.n, t.d, t.e);
     return cudaGetLastError();
 }
 

@@ -9,19 +9,18 @@ namespace dvr3d {
 
 constexpr int kBandMaxBw = 32;  // widest band handled (one warp lane per row of a block)
 
+constexpr int kBandLd = 3 * kBandMaxBw;  // doubles a column of the chase's compact band storage
+
 struct BandTri {
-    double *A;              // n x n, lower triangle holds the band; rows up to 2b below the
-    long long lda;          // diagonal are used as bulge space (zeroed by launch_band_prepare)
+    double *C;              // the band in compact storage (launch_band_compact); overwritten
     int n, b;
-    int ntmax;              // tasks per sweep at most: (n - 2) / b + 1
+    int ntmax;              // tasks per sweep at most: (n - 2) / b + 1 (set by launch_band_chase)
     double *d, *e;          // out: tridiagonal (d[i] = A[i][i], e[i] = A[i+1][i])
-    double *vs;             // out: reflectors, [n - 2][ntmax][kBandMaxBw] (v[0] = 1 stored)
+    double *vs;             // out: reflectors, [n - 2][ntmax][kBandMaxBw] (v[0] = 1 stored); null
+                            // when no back-transformation follows
     double *taus;           // out: [n - 2][ntmax]
-    unsigned int *progress; // [n] tasks finished per sweep (zeroed by the launcher)
+    unsigned int *progress; // [n] hand-off flags (zeroed by the launcher)
     int *err;
-    long long *prof;        // optional [5]: clock cycles of the chase's thread 0 summed over
-                            // CTAs (sweep start, reflector, O_s part with the hand-off,
-                            // end-of-task wait, unused), or null
     unsigned long long wait_limit;  // polls of one hand-off wait before it gives up (0: 2^24)
 };
 
@@ -31,6 +30,8 @@ cudaError_t launch_band_prepare(double *A, long long lda, int n, int b, unsigned
                                 cudaStream_t st);
 size_t band_reflector_doubles(int n, int b);  // vs
 size_t band_tau_doubles(int n, int b);        // taus
+size_t band_compact_doubles(int n);           // C
+cudaError_t launch_band_compact(const double *A, long long lda, int n, int b, double *C, cudaStream_t st);
 // Bulge chasing (one CTA per sweep in flight, sweeps pipelined through progress flags),
 // then d and e from the reduced matrix.
 cudaError_t launch_band_chase(BandTri &t, cudaStream_t st);

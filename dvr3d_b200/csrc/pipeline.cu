@@ -738,8 +738,8 @@ bool band_lowest(dvr3d_ctx *ctx, double *A, long long lda, int n, int b, int nev
     if (dropped_rel) *dropped_rel = rel;
     if (!(rel <= drop_rel)) return false;
     BandTri t{};
-    t.A = A;
-    t.lda = lda;
+    t.C = ctx->arena.get_t<double>("bd_C", band_compact_doubles(n));
+    CK(launch_band_compact(A, lda, n, b, t.C, st));
     t.n = n;
     t.b = b;
     t.d = ctx->arena.get_t<double>("bd_d", n);
