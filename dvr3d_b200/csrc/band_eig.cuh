@@ -35,6 +35,7 @@ cudaError_t launch_band_compact(const double *A, long long lda, int n, int b, do
 // Bulge chasing (one CTA per sweep in flight, sweeps pipelined through progress flags),
 // then d and e from the reduced matrix.
 cudaError_t launch_band_chase(BandTri &t, cudaStream_t st);
+constexpr int kBandBackMax = 22000;  // largest order launch_band_backtransform takes
 // Z (n x nev, ldz) <- Q Z with Q the product of the chase's reflectors (A = Q T Q^T).
 cudaError_t launch_band_backtransform(const BandTri &t, double *Z, long long ldz, int nev, cudaStream_t st);
 

@@ -1,7 +1,9 @@
 // eig_dense.cu -- FP64 eigensolver for the final N x N Hamiltonian (lowest K levels).
 //
 // Replaces diag3d -> diag -> dsyev('V','L') of the reference (:2661-2764, :2638-2659) for
-// the plain FP64 path. Same structure as the batched solver (Householder reduction,
+// the plain FP64 path. The one-stage reduction below serves what the two-stage one of
+// band_reduce.cu does not take; eigenvalues and tridiagonal eigenvectors serve both. Same
+// structure as the batched solver (Householder reduction,
 // bisection, inverse iteration, back-transformation) but spread over the whole GPU:
 //   - the reduction is blocked like LAPACK's dsytrd/dlatrd: a cooperative kernel forms
 //     the 32 reflectors of a panel (one symmetric product over the lower triangle of the

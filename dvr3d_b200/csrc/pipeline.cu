@@ -15,6 +15,7 @@
 #include "blocks.cuh"
 #include "eig_batched.cuh"
 #include "band_eig.cuh"
+#include "band_reduce.cuh"
 #include "eig_dense.cuh"
 #include "gemm64.cuh"
 #include "learned_precond.cuh"
@@ -631,8 +632,88 @@ void channel_setup(dvr3d_ctx *ctx, const H3Op &op, const Contracted &C, ChanPrec
 }
 
 // ---------------------------------------------------------------- dense eigensolver
+namespace {
+// Lowest eigenpairs in two stages: dense -> band (band_reduce.cu) -> tridiagonal (band_eig.cu).
+void dense_lowest_two_stage(dvr3d_ctx *ctx, double *A, long long lda, int n, int nev, bool vecs, double *w, double *Z,
+                            long long ldz, const char *tag, bool time_panels, DenseOut *out) {
+    cudaStream_t st = ctx->stream;
+    const std::string t(tag);
+    if (time_panels && ctx->panel_ev.size() < 2) {
+        const size_t old = ctx->panel_ev.size();
+        ctx->panel_ev.resize(2);
+        for (size_t q = old; q < 2; ++q) CK(cudaEventCreate(&ctx->panel_ev[q]));
+    }
+    BandReduce br{};
+    br.A = A;
+    br.lda = lda;
+    br.n = n;
+    br.keep = vecs;
+    br.C = ctx->arena.get_t<double>(t + "bandC", band_compact_doubles(n));
+    br.T = ctx->arena.get_t<double>(t + "bandT", (size_t)band_reduce_panels(n) * kBandMaxBw * kBandMaxBw);
+    br.work = ctx->arena.get_t<double>(t + "bandwork", band_reduce_work_doubles(n));
+    if (time_panels) CK(cudaEventRecord(ctx->panel_ev[0], st));
+    const long long launches0 = g_kernel_launches;
+    CK(launch_band_reduce(br, st));
+    const int reduce_launches = (int)(g_kernel_launches - launches0);
+    if (time_panels) CK(cudaEventRecord(ctx->panel_ev[1], st));
+    BandTri bt{};
+    bt.C = br.C;
+    bt.n = n;
+    bt.b = kBandMaxBw;
+    bt.d = ctx->arena.get_t<double>(t + "d", n);
+    bt.e = ctx->arena.get_t<double>(t + "e", n);
+    if (vecs) {
+        bt.vs = ctx->arena.get_t<double>(t + "bandvs", band_reflector_doubles(n, bt.b));
+        bt.taus = ctx->arena.get_t<double>(t + "bandtau", band_tau_doubles(n, bt.b));
+    }
+    bt.progress = ctx->arena.get_t<unsigned int>(t + "bandprog", n);
+    bt.err = ctx->arena.get_t<int>(t + "err", 1);
+    bt.wait_limit = ctx->wait_limit;
+    CK(cudaMemsetAsync(bt.err, 0, sizeof(int), st));
+    CK(launch_band_chase(bt, st));
+    double *e2s = ctx->arena.get_t<double>(t + "e2", n);
+    double *info = ctx->arena.get_t<double>(t + "info", 4);
+    launch_dense_eigvals(bt.d, bt.e, n, nev, e2s, info, w, st);
+    CK(cudaGetLastError());
+    if (vecs) {
+        const int T = std::min(nev, 1024);
+        const bool smem = invit_smem_bytes(n) <= (size_t)kInvitSmemMax;
+        double *fac = smem ? nullptr : ctx->arena.get_t<double>(t + "fac", (size_t)5 * n * T);
+        double *X = smem ? nullptr : ctx->arena.get_t<double>(t + "x", (size_t)n * nev);
+        int *cs = ctx->arena.get_t<int>(t + "cs", nev + 1);
+        int *ncl = ctx->arena.get_t<int>(t + "ncl", 1);
+        // the products of the back-transformation take 16-byte rows
+        const bool even = (ldz & 1) == 0 && (reinterpret_cast<uintptr_t>(Z) & 15) == 0;
+        const long long ldw = even ? ldz : round_up(n, 2);
+        double *Zw = even ? Z : ctx->arena.get_t<double>(t + "zw", (size_t)ldw * nev);
+        launch_tridiag_eigvecs(bt.d, bt.e, n, w, nev, info, cs, ncl, fac, T, X, Zw, ldw, 1.0e-6, st);
+        CK(cudaGetLastError());
+        CK(launch_band_backtransform(bt, Zw, ldw, nev, st));
+        CK(launch_band_reduce_back(br, Zw, ldw, nev, ctx->arena.get_t<double>(t + "bandback", band_reduce_back_doubles(nev)), st));
+        if (!even)
+            CK(cudaMemcpy2DAsync(Z, (size_t)ldz * sizeof(double), Zw, (size_t)ldw * sizeof(double), (size_t)n * sizeof(double),
+                                 nev, cudaMemcpyDeviceToDevice, st));
+    }
+    check_dev_err(ctx, bt.err, "dense tridiagonal reduction");
+    if (out && time_panels) {
+        float m = 0.f;
+        CK(cudaEventElapsedTime(&m, ctx->panel_ev[0], ctx->panel_ev[1]));
+        out->panel_ms = m;
+        out->npanel = reduce_launches;
+        out->two_stage = true;
+    }
+}
+}  // namespace
+
 void dense_lowest(dvr3d_ctx *ctx, double *A, long long lda, int n, int nev, bool vecs, double *w, double *Z,
                   long long ldz, const char *tag, bool time_panels, DenseOut *out) {
+    // Two stages at every order: 12: 0.19 -> 0.10 ms, 128: 1.83 -> 1.07, 913: 14.1 -> 9.2, 3960: 96.6
+    // -> 47.4, 12241: 984 -> 317 ms; one stage for orders that need no reflector, and for vectors
+    // whose columns the chase's back-transformation cannot hold in shared memory (over kBandBackMax).
+    if (n >= 3 && (!vecs || n <= kBandBackMax) && band_reduce_available()) {
+        dense_lowest_two_stage(ctx, A, lda, n, nev, vecs, w, Z, ldz, tag, time_panels, out);
+        return;
+    }
     cudaStream_t st = ctx->stream;
     const std::string t(tag);
     DenseTri dt{};
@@ -1240,16 +1321,17 @@ void solve_contracted(dvr3d_ctx *ctx, const BlockPlan &p, const Contracted &C, c
     finish_times(ms1, ms2, ms3);
     // dominant kernel: the panel kernel of the Householder reduction; its algorithmic
     // traffic is one read of the trailing lower triangle per column
+    // (one-stage), or the 4/3 N^3 flop of the reduction to band form (two-stage)
     double bytes = 0.0;
     for (int k = 0; k + 2 < N; ++k) {
         const double m = (double)(N - k - 1);
         bytes += 8.0 * m * (m + 1.0) * 0.5;
     }
     res.dom_ms = dout.panel_ms;
-    res.dom_bytes = bytes;
-    res.dom_flops = 0.0;
+    res.dom_bytes = dout.two_stage ? 0.0 : bytes;
+    res.dom_flops = dout.two_stage ? 4.0 / 3.0 * (double)N * N * N : 0.0;
     res.dom_launches = dout.npanel;
-    std::snprintf(res.dom_kernel, sizeof(res.dom_kernel), "dense_panel_kernel");
+    std::snprintf(res.dom_kernel, sizeof(res.dom_kernel), dout.two_stage ? "syr2k_band_kernel" : "dense_panel_kernel");
     res.launches = (int)(g_kernel_launches - launches0);
     res.h2d_bytes = t_h2d;
     res.d2h_bytes = t_d2h;

@@ -173,6 +173,7 @@ void note_d2h(long long bytes);
 // the reduction). Device scratch is taken from the arena under names starting with `tag`.
 // When time_panels is set, the reduction's panel launches are timed into *out.
 struct DenseOut {
+    bool two_stage = false;  // panel_ms / npanel: the reduction to band form
     double panel_ms = 0.0;
     int npanel = 0;
 };
