@@ -121,11 +121,15 @@ void copy_cols(double *dst, long long ldd, const double *src, long long lds, int
                          cudaMemcpyDeviceToDevice, st));
 }
 
+int split_for(int M, int N, int K, int target) {
+    const int tiles = ((M + 63) / 64) * ((N + 63) / 64);
+    const int s = std::max(1, std::min({(target + tiles - 1) / tiles, 64, (K + 15) / 16}));
+    return (s > 8 && tiles * 8 >= 296) ? 8 : s;
+}
+
 void gemm_split(GemmOp g, int target, double *work, cudaStream_t st) {
     if (target > 1) {
-        const int tiles = ((g.M + 63) / 64) * ((g.N + 63) / 64);
-        g.splitk = std::max(1, std::min({(target + tiles - 1) / tiles, 64, (g.K + 15) / 16}));
-        if (g.splitk > 8 && tiles * 8 >= 296) g.splitk = 8;
+        g.splitk = split_for(g.M, g.N, g.K, target);
         g.work = work;
     }
     CK(launch_gemm(g, st));
@@ -235,8 +239,18 @@ bool davidson_solve(dvr3d_ctx *ctx, const H3Op &op, const Contracted &C, const d
         CK(cudaMemcpyAsync(ones, o.data(), sizeof(double) * bs, cudaMemcpyHostToDevice, st));
         CK(cudaStreamSynchronize(st));
     }
-    double *work = A("dv_work", (size_t)std::max<long long>(std::min<long long>(64LL * mmax * mmax, 1LL << 22),
-                                                          16LL * N * bs));
+    // partial sums of the split products: H3 V and the projections by any block of columns, V^T HV
+    // at any basis size (below about 2300 rows H3 V splits more than sixteen ways)
+    size_t wk = 0;
+    std::vector<int> widths{bs};  // a split depends on the width only through its 64-column tiles
+    for (int c = 64; c < bs; c += 64) widths.push_back(c);
+    for (int c : widths) wk = std::max(wk, gemm_splitk_work(N, c, split_for(N, c, N, 600)));
+    for (int q = 1; q <= mmax; ++q) {
+        wk = std::max(wk, gemm_splitk_work(q, q, split_for(q, q, N, 600)));
+        for (int c : widths) wk = std::max(wk, gemm_splitk_work(q, c, split_for(q, c, N, 600)));
+    }
+    wk = std::max(wk, gemm_splitk_work(64, 64, 64));  // Cholesky-QR of 64 columns
+    double *work = A("dv_work", wk);
     int *err = ctx->arena.get_t<int>("dv_err", 3);
     CK(cudaMemsetAsync(err, 0, 3 * sizeof(int), st));
     // Rayleigh-Ritz eigensolver of the small path: the batched solver's kernels on one block
