@@ -345,8 +345,6 @@ int dvr3d_b200_diag_batched(dvr3d_ctx *ctx, int nblk, const int *n_host, const l
         for (int b = 0; b < nblk; ++b)
             cudaMemcpyAsync(ac + asz[b], a_dev + aoff[b], sizeof(double) * n[b] * n[b], cudaMemcpyDeviceToDevice, st);
         // the reference reads the lower triangle only: mirror it into full storage
-        std::vector<int> dummy;
-        (void)dummy;
         dvr3d::BatchDesc bdc{nblk, bd.n, up("dg_asz", asz), bd.voff};
         dvr3d::launch_symmetrize_lower(bdc, ac, nmax, st);
         dvr3d::launch_tridiag_batched(bdc, ac, d, e, tau, nmax, st);
@@ -356,17 +354,8 @@ int dvr3d_b200_diag_batched(dvr3d_ctx *ctx, int nblk, const int *n_host, const l
         int *err = ctx->arena.get_t<int>("err", 1);
         int err_host = 0;
         if (vecs) {
-            std::vector<int> zld(n);
-            std::vector<long long> woff(nblk);
-            long long wt = 0;
-            for (int b = 0; b < nblk; ++b) {
-                woff[b] = wt;
-                wt += 5LL * n[b] * std::min(128, n[b]) + (long long)n[b] * n[b];
-            }
-            double *work = ctx->arena.get_t<double>("dg_work", wt);
             cudaMemsetAsync(err, 0, sizeof(int), st);
-            dvr3d::launch_eigvecs_batched(bdc, ac, d, e, tau, w, bd.n, up("dg_zoff", aoff), up("dg_zld", n), a_dev,
-                                          work, up("dg_woff", woff), nmax, err, st);
+            dvr3d::launch_eigvecs_batched(bdc, ac, d, e, tau, w, bd.n, bd.aoff, bd.n, a_dev, nmax, err, st);
             cudaMemcpyAsync(&err_host, err, sizeof(int), cudaMemcpyDeviceToHost, st);
         }
         cudaError_t ce = cudaStreamSynchronize(st);

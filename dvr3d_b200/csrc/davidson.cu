@@ -27,7 +27,6 @@
 #include "gemm64.cuh"
 #include "learned_precond.cuh"
 #include "pipeline.cuh"
-#include "small_syev.cuh"
 #include "tc_gemm.cuh"
 
 #define CK(x)                                          \
@@ -39,6 +38,9 @@
 namespace dvr3d {
 
 namespace {
+
+constexpr int kBatchedRR = 160;  // Rayleigh-Ritz matrices up to this order go to the batched eigensolver
+
 
 // R[:, j] = HX[:, j] - w_j X[:, j], rn[j] = ||R[:, j]||; one CTA per column
 __global__ void residual_kernel(const double *X, const double *HX, long long ld, const double *w, int N, double *R,
@@ -221,7 +223,7 @@ bool davidson_solve(dvr3d_ctx *ctx, const H3Op &op, const Contracted &C, const d
     bs += (bs & 1);
     const int keep = 2 * bs, mmax = 3 * bs;
     if (mmax >= N) return false;
-    const bool big_rr = mmax > kSmallSyevMax;  // Rayleigh-Ritz on the dense eigensolver
+    const bool big_rr = mmax > kBatchedRR;  // Rayleigh-Ritz on the dense eigensolver
     const double tolE = (opt.tol_cm > 0.0 ? opt.tol_cm : 1.0e-4) / 2.19474624e5;
     const int max_iter = opt.max_iter > 0 ? opt.max_iter : 300;
     const long long ld = rup(N, 8);
@@ -314,7 +316,7 @@ bool davidson_solve(dvr3d_ctx *ctx, const H3Op &op, const Contracted &C, const d
         launch_symmetrize_lower(bd, rr_a, m, st);
         launch_tridiag_batched(bd, rr_a, rr_d, rr_e, rr_tau, m, st);
         launch_eigvals_batched(bd, rr_d, rr_e, w, rr_int + 3, 0, 0.0, st);
-        launch_eigvecs_batched_fast(bd, rr_a, rr_d, rr_e, rr_tau, w, rr_int + 1, rr_zero, rr_int + 2, Z, m, err, st);
+        launch_eigvecs_batched(bd, rr_a, rr_d, rr_e, rr_tau, w, rr_int + 1, rr_zero, rr_int + 2, Z, m, err, st);
         CK(cudaGetLastError());
     };
     // HV[:, c0:c0+nc] = H3 V[:, c0:c0+nc]: BF16x3 tensor-core GEMM (split form, phase 1), the

@@ -5,6 +5,7 @@
 #include <cmath>
 
 #include "common.cuh"
+#include "dmma.cuh"
 #include "eig_batched.cuh"
 #include "tridiag_dev.cuh"
 
@@ -153,439 +154,515 @@ __global__ void __launch_bounds__(kTriMaxThreads) tridiag_kernel(BatchDesc bd, d
     }
 }
 
-constexpr int kEvThreads = 256;
+// ------------------------------------------------------------------ eigenvalues
+constexpr int kEvThreads = 512;
 
-__global__ void __launch_bounds__(kEvThreads) eigvals_kernel(BatchDesc bd, const double *dg,
-                                                              const double *eo, double *wo,
-                                                              int *cnt, int mode, double cut) {
+// Sturm-count multisection. Every CTA first counts at 512 equidistant points, which brackets each
+// eigenvalue to 1/513 of the Gershgorin interval in one pass; then groups of L lanes narrow one
+// eigenvalue each, L + 1 times a pass, L the largest power of two that keeps the CTA's threads busy.
+// gridDim.y CTAs share a block's eigenvalues. Bound by the FP64 issue of the counts (three
+// operations a row): 64 blocks of order 465, 62 eigenvalues each: 0.21 ms (one thread an eigenvalue
+// with a division a row: 2.2 ms).
+__global__ void __launch_bounds__(kEvThreads) eigvals_kernel(BatchDesc bd, const double *dg, const double *eo, double *wo,
+                                                             int *cnt, int mode, double cut) {
     const int b = blockIdx.x;
     if (b >= bd.nblk) return;
     const int n = bd.n[b];
     const double *d = dg + bd.voff[b], *e = eo + bd.voff[b];
     double *w = wo + bd.voff[b];
     extern __shared__ double sm[];
-    double *sd = sm, *e2 = sm + n;
-    __shared__ double red[32];
+    double *sd = sm, *ne2 = sm + n;
+    __shared__ double s_min[kEvThreads], s_max[kEvThreads];
+    __shared__ int s_cnt[kEvThreads];
     __shared__ int s_count;
-    __shared__ double s_lo, s_hi, s_piv;
-    const int tid = threadIdx.x;
-    double lo = DBL_MAX, hi = -DBL_MAX, emx = 0.0;
+    const int tid = threadIdx.x, lane = tid & 31;
+    double lo = DBL_MAX, hi = -DBL_MAX;
     for (int i = tid; i < n; i += blockDim.x) {
         const double di = d[i];
         const double em = (i > 0) ? fabs(e[i - 1]) : 0.0, ep = (i < n - 1) ? fabs(e[i]) : 0.0;
-        sd[i] = di;
-        if (i < n - 1) e2[i] = e[i] * e[i];
         lo = fmin(lo, di - em - ep);
         hi = fmax(hi, di + em + ep);
-        emx = fmax(emx, (i < n - 1) ? e[i] * e[i] : 0.0);
     }
-    // block min / max via the sum helper on negated / shifted values is awkward: use shared
-    __shared__ double s_min[kEvThreads], s_max[kEvThreads], s_e[kEvThreads];
     s_min[tid] = lo;
     s_max[tid] = hi;
-    s_e[tid] = emx;
     __syncthreads();
     for (int s = blockDim.x / 2; s > 0; s >>= 1) {
         if (tid < s) {
             s_min[tid] = fmin(s_min[tid], s_min[tid + s]);
             s_max[tid] = fmax(s_max[tid], s_max[tid + s]);
-            s_e[tid] = fmax(s_e[tid], s_e[tid + s]);
         }
         __syncthreads();
     }
-    if (tid == 0) {
-        const double tnorm = fmax(fabs(s_min[0]), fabs(s_max[0]));
-        s_piv = DBL_MIN * fmax(1.0, s_e[0]);
-        s_lo = s_min[0] - 2.0 * DBL_EPSILON * tnorm * n - 2.0 * s_piv;
-        s_hi = s_max[0] + 2.0 * DBL_EPSILON * tnorm * n + 2.0 * s_piv;
+    // the matrix and its bounds in units of 1 / scale
+    const double tnorm = fmax(fabs(s_min[0]), fabs(s_max[0]));
+    const double scale = sturm_scale(tnorm), unit = 1.0 / scale;
+    const double margin = 2.0 * DBL_EPSILON * (tnorm * scale) * n + 2.0 * DBL_MIN;
+    const double glo = s_min[0] * scale - margin, ghi = s_max[0] * scale + margin;
+    for (int i = tid; i < n; i += blockDim.x) {
+        sd[i] = d[i] * scale;
+        if (i < n - 1) ne2[i] = sturm_off(e[i], scale);
     }
     __syncthreads();
-    (void)red;
-    int m = n;
-    if (mode != 0) {
-        if (tid == 0) {
-            double x = cut;
-            if (mode == 2) x = nextafter(cut, DBL_MAX);  // count of eigenvalues <= cut
-            s_count = (x <= s_lo) ? 0 : (x >= s_hi ? n : sturm_count(sd, e2, n, x, s_piv));
-        }
-        __syncthreads();
-        m = s_count;
+    const double h = (ghi - glo) / (double)(kEvThreads + 1);
+    s_cnt[tid] = sturm_count(sd, ne2, n, glo + h * (double)(tid + 1));
+    if (mode != 0 && tid == 0) {
+        double x = cut;
+        if (mode == 2) x = nextafter(cut, DBL_MAX);  // count of eigenvalues <= cut
+        x *= scale;
+        s_count = (x <= glo) ? 0 : (x >= ghi ? n : sturm_count(sd, ne2, n, x));
     }
-    if (tid == 0) cnt[b] = m;
-    for (int j = tid; j < m; j += blockDim.x) w[j] = bisect_one(sd, e2, n, j, s_lo, s_hi, s_piv);
+    __syncthreads();
+    const int m = (mode != 0) ? s_count : n;
+    const int P = gridDim.y, jb = (int)((long long)m * blockIdx.y / P), je = (int)((long long)m * (blockIdx.y + 1) / P);
+    if (tid == 0 && blockIdx.y == 0) cnt[b] = m;
+    int L = 1;
+    while (L < 32 && (je - jb) * L * 2 <= kEvThreads) L *= 2;
+    const int per = kEvThreads / L, sub = tid % L, g0 = lane - sub;  // eigenvalues at a time; lane in the group; its first
+    const unsigned gmask = (L == 32 ? 0xffffffffu : ((1u << L) - 1u)) << g0;
+    for (int j0 = jb; j0 < je; j0 += per) {
+        const int j = j0 + tid / L;
+        const bool mine = j < je;
+        double a = glo, z = ghi;
+        if (mine) {  // first point with more than j eigenvalues below it
+            int p = 0, q = kEvThreads;
+            while (p < q) {
+                const int mid = (p + q) >> 1;
+                if (s_cnt[mid] > j) q = mid;
+                else p = mid + 1;
+            }
+            if (p > 0) a = glo + h * (double)p;
+            if (p < kEvThreads) z = glo + h * (double)(p + 1);
+        }
+        bool run = mine;
+        for (int pass = 0; pass < 200; ++pass) {
+            if (run && z - a <= 2.0 * DBL_EPSILON * fmax(fabs(a), fabs(z))) run = false;
+            if (!__any_sync(0xffffffffu, run)) break;
+            const double x = (L == 1) ? 0.5 * (a + z) : a + (z - a) * ((double)(sub + 1) / (double)(L + 1));
+            const bool above = sturm_count(sd, ne2, n, x) > j;
+            const unsigned bal = __ballot_sync(0xffffffffu, above) & gmask;
+            const int f = bal ? __ffs(bal) - 1 - g0 : L;  // first lane above
+            const double xl = __shfl_sync(0xffffffffu, x, g0 + (f > 0 ? f - 1 : 0));
+            const double xh = __shfl_sync(0xffffffffu, x, g0 + (f < L ? f : L - 1));
+            const double na = (f == 0) ? a : xl, nz = (f == L) ? z : xh;
+            if (run) {
+                if (!(nz - na < z - a)) run = false;  // interval at rounding level
+                a = na;
+                z = nz;
+            }
+        }
+        if (mine && sub == 0) w[j] = 0.5 * (a + z) * unit;
+    }
 }
 
 // ------------------------------------------------------------------ inverse iteration
-constexpr int kVecThreads = 128;
-
-__global__ void __launch_bounds__(kVecThreads) eigvecs_kernel(BatchDesc bd, const double *A,
-                                                               const double *dg, const double *eo,
-                                                               const double *tauo, const double *wo,
-                                                               const int *sel, const long long *zoff,
-                                                               const int *zld, double *Z, double *work,
-                                                               const long long *workoff, int *err) {
-    const int b = blockIdx.x;
-    if (b >= bd.nblk) return;
-    const int n = bd.n[b];
-    const int m = sel[b];
-    if (m <= 0) return;
-    const double *a = A + bd.aoff[b];
-    const double *d = dg + bd.voff[b], *e = eo + bd.voff[b], *tau = tauo + bd.voff[b];
-    const double *w = wo + bd.voff[b];
-    double *z = Z + zoff[b];
-    const int ldz = zld[b];
-    double *wk = work + workoff[b];
-    extern __shared__ double sm[];
-    int *cstart = reinterpret_cast<int *>(sm);  // cluster starts (m+1 ints)
-    __shared__ int s_ncl;
-    __shared__ double s_onenrm;
-    const int tid = threadIdx.x;
-    // clusters: consecutive eigenvalues closer than 1e-6 ||T||_1 are orthogonalised
-    if (tid == 0) {
-        double on = 0.0;
-        for (int i = 0; i < n; ++i) {
-            const double r = fabs(d[i]) + (i > 0 ? fabs(e[i - 1]) : 0.0) + (i < n - 1 ? fabs(e[i]) : 0.0);
-            on = fmax(on, r);
-        }
-        s_onenrm = fmax(on, DBL_MIN);
-        const double ortol = 1.0e-6 * s_onenrm;
-        int nc = 0;
-        cstart[nc++] = 0;
-        for (int j = 1; j < m; ++j)
-            if (w[j] - w[j - 1] > ortol) cstart[nc++] = j;
-        cstart[nc] = m;
-        s_ncl = nc;
-    }
-    __syncthreads();
-    const int ncl = s_ncl;
-    const int T = min((int)blockDim.x, m);   // thread slots holding LU factors
-    double *fac = wk;                        // 5 * n * T
-    double *X = wk + (size_t)5 * n * T;      // n * m, interleaved by eigenvalue
-    if (tid < T)
-        for (int c = tid; c < ncl; c += T)
-            invit_cluster(d, e, n, w, cstart[c], cstart[c + 1], s_onenrm, fac, T, tid, X, m, err);
-    __syncthreads();
-    const int TT = blockDim.x;
-    // copy to Z (column per eigenvalue) -- coalesced over rows
-    for (int idx = tid; idx < n * m; idx += TT) {
-        const int jcol = idx / n, i = idx - jcol * n;
-        z[(size_t)jcol * ldz + i] = X[(size_t)i * m + jcol];
-    }
-    __syncthreads();
-    // back-transform: z <- H_0 H_1 ... H_{n-3} z  (apply H_{n-3} first)
-    double *vs = sm;  // reuse shared memory for the reflector
-    const int lane = tid & 31, wid = tid >> 5, nw = TT >> 5;
-    for (int k = n - 3; k >= 0; --k) {
-        const double tk = tau[k];
-        __syncthreads();
-        if (tk == 0.0) continue;
-        for (int i = k + 1 + tid; i < n; i += TT) vs[i] = (i == k + 1) ? 1.0 : a[(size_t)k * n + i];
-        __syncthreads();
-        for (int jcol = wid; jcol < m; jcol += nw) {
-            double *zc = z + (size_t)jcol * ldz;
-            double s = 0.0;
-            for (int i = k + 1 + lane; i < n; i += 32) s += vs[i] * zc[i];
-            s = warp_sum(s) * tk;
-            for (int i = k + 1 + lane; i < n; i += 32) zc[i] -= s * vs[i];
-        }
-    }
-    (void)err;
-}
-
-// ------------------------------------------------------------------ eigenvectors, fast form
-// Same method as eigvecs_kernel (dstein-style inverse iteration, Gram-Schmidt inside clusters
-// closer than 1e-6 ||T||, back-transformation by the block's reflectors), organised for speed:
-//   * one warp per cluster, the LU factors of T - lambda I and the iterate in that warp's
-//     slice of shared memory (lane 0 runs the recurrences, the warp the vector operations);
-//   * the back-transformation in panels of 16 reflectors (compact WY, I - V Tm V^T): per
-//     panel V and Tm in shared memory, one thread per eigenvector column computing
-//     W = V^T z, W2 = Tm W and z -= V W2 in registers.
-constexpr int kFastPanel = 16;
-
-// The first vector of eigvecs_fast_kernel that failed its growth test since the last clear:
-// {failed, block, eigenvalue index, block order}, for the host's error message.
+// The first vector that failed its growth test since the last clear: {failed, block, eigenvalue
+// index, block order}, for the host's error message.
 __device__ int g_invit_fail[4];
 
-__global__ void eigvecs_fast_kernel(BatchDesc bd, const double *A, const double *dg, const double *eo,
-                                    const double *tauo, const double *wo, const int *sel, const long long *zoff,
-                                    const int *zld, double *Z, int *err) {
-    // gridDim.y CTAs share a block: CTA y takes the eigenvalue clusters c = y (mod gridDim.y)
-    // and back-transforms their columns
+// Eigenvectors of the tridiagonal matrices for the selected eigenvalues, as dstein: LU factors of
+// T - lambda I with partial pivoting, up to four solves, modified Gram-Schmidt inside clusters of
+// eigenvalues closer than 1e-6 ||T||. One warp per cluster with the factors and the iterate in its
+// slice of shared memory; lane 0 runs the recurrences eight rows at a time, operands first, so that
+// a row costs its dependent operations only. gridDim.y CTAs share a block's clusters. Bound by that
+// chain: 3960 vectors of 64 blocks of order 465 take 1.0 ms.
+__global__ void invit_batched_kernel(BatchDesc bd, const double *dg, const double *eo, const double *wo, const int *sel,
+                                     const long long *zoff, const int *zld, double *Z, int *err) {
     const int b = blockIdx.x, part = blockIdx.y, nparts = gridDim.y;
     if (b >= bd.nblk) return;
     const int n = bd.n[b];
     const int m = sel[b];
     if (m <= 0) return;
-    const double *a = A + bd.aoff[b];
-    const double *d = dg + bd.voff[b], *e = eo + bd.voff[b], *tau = tauo + bd.voff[b];
     const double *w = wo + bd.voff[b];
     double *z = Z + zoff[b];
     const int ldz = zld[b];
     extern __shared__ double sm[];
-    __shared__ int cstart[1025];
-    __shared__ int mycols[1024];  // columns of this CTA's clusters
-    __shared__ int s_ncl, s_nmine;
-    __shared__ double s_onenrm;
+    __shared__ int cstart[1026];
+    __shared__ int s_ncl;
+    __shared__ double red[32];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarp = blockDim.x >> 5;
-    if (tid == 0) {
-        double on = 0.0;
-        for (int i = 0; i < n; ++i) {
-            const double r = fabs(d[i]) + (i > 0 ? fabs(e[i - 1]) : 0.0) + (i < n - 1 ? fabs(e[i]) : 0.0);
-            on = fmax(on, r);
-        }
-        s_onenrm = fmax(on, DBL_MIN);
-        const double ortol = 1.0e-6 * s_onenrm;
+    const int np = (n + 8) & ~7;  // the eight-row loops run into the padding
+    double *d = sm, *e = sm + np;
+    double on = 0.0;
+    for (int i = tid; i < np; i += blockDim.x) {
+        const double di = (i < n) ? dg[bd.voff[b] + i] : 0.0, ei = (i < n - 1) ? eo[bd.voff[b] + i] : 0.0;
+        const double em = (i > 0 && i < n) ? fabs(eo[bd.voff[b] + i - 1]) : 0.0;
+        d[i] = di;
+        e[i] = ei;
+        on = fmax(on, fabs(di) + em + fabs(ei));
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) on = fmax(on, __shfl_xor_sync(0xffffffffu, on, o));
+    if (lane == 0) red[warp] = on;
+    __syncthreads();
+    on = red[0];
+    for (int q = 1; q < nwarp; ++q) on = fmax(on, red[q]);
+    const double onenrm = fmax(on, DBL_MIN);
+    if (warp == 0) {  // cluster starts
+        const double ortol = 1.0e-6 * onenrm;
         int nc = 0;
-        cstart[nc++] = 0;
-        for (int j = 1; j < m; ++j)
-            if (w[j] - w[j - 1] > ortol) cstart[nc++] = j;
-        cstart[nc] = m;
-        s_ncl = nc;
-        int nm = 0;
-        for (int c = part; c < nc; c += nparts)
-            for (int j = cstart[c]; j < cstart[c + 1]; ++j) mycols[nm++] = j;
-        s_nmine = nm;
+        for (int j0 = 0; j0 < m; j0 += 32) {
+            const int j = j0 + lane;
+            const bool st = j < m && (j == 0 || w[j] - w[j - 1] > ortol);
+            const unsigned bal = __ballot_sync(0xffffffffu, st);
+            if (st) cstart[nc + __popc(bal & ((1u << lane) - 1u))] = j;
+            nc += __popc(bal);
+        }
+        if (lane == 0) {
+            cstart[nc] = m;
+            s_ncl = nc;
+        }
     }
     __syncthreads();
-    // ---- inverse iteration, one warp per cluster
-    {
-        const size_t slice = (size_t)5 * n + (n + 7) / 8;  // doubles per warp
-        double *D = sm + warp * slice, *E1 = D + n, *E2 = E1 + n, *Lm = E2 + n, *x = Lm + n;
-        unsigned char *P = reinterpret_cast<unsigned char *>(x + n);
-        const double onenrm = s_onenrm;
-        const double eps = DBL_EPSILON, tiny = eps * onenrm, pertol = 10.0 * eps * onenrm;
-        for (int c = part + nparts * warp; c < s_ncl; c += nparts * nwarp) {
-            const int j0 = cstart[c], j1 = cstart[c + 1];
-            double lamprev = 0.0;
-            for (int j = j0; j < j1; ++j) {
-                double lam = w[j];
-                if (j > j0 && lam - lamprev < pertol) lam = lamprev + pertol;
-                lamprev = lam;
+    const size_t slice = (size_t)5 * np + np / 8;  // doubles per warp
+    double *D = sm + 2 * np + warp * slice, *E1 = D + np, *E2 = E1 + np, *Lm = E2 + np, *x = Lm + np;
+    unsigned char *P = reinterpret_cast<unsigned char *>(x + np);
+    const double eps = DBL_EPSILON, tiny = eps * onenrm, pertol = 10.0 * eps * onenrm;
+    const double grow_lim = invit_growth_limit(n);
+    for (int c = part + nparts * warp; c < s_ncl; c += nparts * nwarp) {
+        const int j0 = cstart[c], j1 = cstart[c + 1];
+        double lamprev = 0.0;
+        for (int j = j0; j < j1; ++j) {
+            double lam = w[j];
+            if (j > j0 && lam - lamprev < pertol) lam = lamprev + pertol;
+            lamprev = lam;
+            if (lane == 0) {
+                double av = d[0] - lam, bv = e[0];
+                for (int i = 0; i < n - 1; i += 8) {
+                    double cc[9], an[8];
+#pragma unroll
+                    for (int u = 0; u < 8; ++u) {
+                        cc[u] = e[i + u];
+                        an[u] = d[min(i + u + 1, np - 1)] - lam;
+                    }
+                    cc[8] = e[min(i + 8, np - 1)];
+#pragma unroll
+                    for (int u = 0; u < 8; ++u) {
+                        if (i + u < n - 1) {
+                            const bool keep = fabs(av) >= fabs(cc[u]);
+                            if (keep && av == 0.0) av = tiny;
+                            const double piv = keep ? av : cc[u], mlt = (keep ? cc[u] : av) / piv;
+                            const double bn = (i + u + 2 < n) ? cc[u + 1] : 0.0;
+                            P[i + u] = keep ? 0 : 1;
+                            Lm[i + u] = mlt;
+                            D[i + u] = piv;
+                            E1[i + u] = keep ? bv : an[u];
+                            E2[i + u] = keep ? 0.0 : bn;
+                            av = keep ? an[u] - mlt * bv : bv - mlt * an[u];
+                            bv = keep ? bn : -mlt * bn;
+                        }
+                    }
+                }
+                if (fabs(av) < tiny) av = (av < 0.0) ? -tiny : tiny;
+                D[n - 1] = av;
+                // no superdiagonals in the last row of U; the back substitution reads them
+                // (times zero), so stale shared memory must not leave a NaN there
+                E1[n - 1] = 0.0;
+                E2[n - 1] = 0.0;
+            }
+            __syncwarp();
+            for (int i = lane; i < n - 1; i += 32)
+                if (fabs(D[i]) < tiny) D[i] = (D[i] < 0.0) ? -tiny : tiny;
+            __syncwarp();
+            // the solves below multiply by the pivots' reciprocals (one division per pivot
+            // here instead of one per pivot and iteration on the sequential path)
+            const double dlast = D[n - 1];
+            __syncwarp();
+            for (int i = lane; i < n; i += 32) D[i] = 1.0 / D[i];
+            for (int i = lane; i < n; i += 32) {
+                const unsigned h = hash32((unsigned)(i * 2654435761u) ^ (unsigned)(j * 40503u + 17u));
+                x[i] = ((double)(h & 0xffffff) / 8388608.0) - 1.0;
+            }
+            __syncwarp();
+            int grown = 0;
+            for (int it = 0; it < kInvitPasses; ++it) {
+                double s1 = 0.0;
+                for (int i = lane; i < n; i += 32) s1 += fabs(x[i]);
+                s1 = warp_sum(s1);
+                const double sc = (double)n * onenrm * fmax(eps, fabs(dlast)) / fmax(s1, DBL_MIN);
+                for (int i = lane; i < n; i += 32) x[i] *= sc;
+                __syncwarp();
                 if (lane == 0) {
-                    double av = d[0] - lam, bv = (n > 1) ? e[0] : 0.0;
-                    for (int i = 0; i < n - 1; ++i) {
-                        const double cc = e[i];
-                        const double an = d[i + 1] - lam, bn = (i + 2 < n) ? e[i + 1] : 0.0;
-                        if (fabs(av) >= fabs(cc)) {
-                            if (av == 0.0) av = tiny;
-                            const double mlt = cc / av;
-                            P[i] = 0;
-                            Lm[i] = mlt;
-                            D[i] = av;
-                            E1[i] = bv;
-                            E2[i] = 0.0;
-                            av = an - mlt * bv;
-                            bv = bn;
-                        } else {
-                            const double mlt = av / cc;
-                            P[i] = 1;
-                            Lm[i] = mlt;
-                            D[i] = cc;
-                            E1[i] = an;
-                            E2[i] = bn;
-                            av = bv - mlt * an;
-                            bv = -mlt * bn;
+                    double y = x[0];
+                    for (int i = 0; i < n - 1; i += 8) {
+                        double xn[8], l[8];
+                        const unsigned long long pm = *reinterpret_cast<const unsigned long long *>(P + i);
+#pragma unroll
+                        for (int u = 0; u < 8; ++u) {
+                            xn[u] = x[min(i + u + 1, np - 1)];
+                            l[u] = Lm[i + u];
                         }
-                    }
-                    if (fabs(av) < tiny) av = (av < 0.0) ? -tiny : tiny;
-                    D[n - 1] = av;
-                    // no superdiagonals in the last row of U; the back substitution reads them
-                    // (times zero), so stale shared memory must not leave a NaN there
-                    E1[n - 1] = 0.0;
-                    E2[n - 1] = 0.0;
-                }
-                __syncwarp();
-                for (int i = lane; i < n - 1; i += 32)
-                    if (fabs(D[i]) < tiny) D[i] = (D[i] < 0.0) ? -tiny : tiny;
-                __syncwarp();
-                // the solves below multiply by the pivots' reciprocals (one division per pivot
-                // here instead of one per pivot and iteration on the sequential path)
-                const double dlast = D[n - 1];
-                __syncwarp();
-                for (int i = lane; i < n; i += 32) D[i] = 1.0 / D[i];
-                for (int i = lane; i < n; i += 32) {
-                    const unsigned h = hash32((unsigned)(i * 2654435761u) ^ (unsigned)(j * 40503u + 17u));
-                    x[i] = ((double)(h & 0xffffff) / 8388608.0) - 1.0;
-                }
-                __syncwarp();
-                const double grow_lim = invit_growth_limit(n);
-                int grown = 0;
-                for (int it = 0; it < kInvitPasses; ++it) {
-                    double s1 = 0.0;
-                    for (int i = lane; i < n; i += 32) s1 += fabs(x[i]);
-                    s1 = warp_sum(s1);
-                    const double sc = (double)n * onenrm * fmax(eps, fabs(dlast)) / fmax(s1, DBL_MIN);
-                    for (int i = lane; i < n; i += 32) x[i] *= sc;
-                    __syncwarp();
-                    if (lane == 0) {
-                        for (int i = 0; i < n - 1; ++i) {
-                            double yi = x[i], yn = x[i + 1];
-                            if (P[i]) {
-                                const double tmp = yi;
-                                yi = yn;
-                                yn = tmp;
-                                x[i] = yi;
+#pragma unroll
+                        for (int u = 0; u < 8; ++u) {
+                            if (i + u < n - 1) {
+                                const bool sw = (pm >> (8 * u)) & 1ull;
+                                const double yi = sw ? xn[u] : y, yn = sw ? y : xn[u];
+                                x[i + u] = yi;
+                                y = yn - l[u] * yi;
                             }
-                            x[i + 1] = yn - Lm[i] * yi;
-                        }
-                        double x1 = 0.0, x2 = 0.0;
-                        for (int i = n - 1; i >= 0; --i) {
-                            const double xi = (x[i] - E1[i] * x1 - E2[i] * x2) * D[i];
-                            x[i] = xi;
-                            x2 = x1;
-                            x1 = xi;
                         }
                     }
-                    __syncwarp();
-                    for (int jj = j0; jj < j; ++jj) {
-                        const double *zc = z + (size_t)jj * ldz;
-                        double dot = 0.0;
-                        for (int i = lane; i < n; i += 32) dot += x[i] * zc[i];
-                        dot = warp_sum(dot);
-                        for (int i = lane; i < n; i += 32) x[i] -= dot * zc[i];
-                    }
-                    double nrm = 0.0, xinf = 0.0;
-                    for (int i = lane; i < n; i += 32) {
-                        nrm += x[i] * x[i];
-                        xinf = fmax(xinf, fabs(x[i]));
-                    }
-                    nrm = sqrt(warp_sum(nrm));
+                    x[n - 1] = y;
+                    double x1 = 0.0, x2 = 0.0;
+                    for (int i = ((n - 1) / 8) * 8; i >= 0; i -= 8) {
+                        double xx[8], r1[8], r2[8], dd[8];
 #pragma unroll
-                    for (int o = 16; o > 0; o >>= 1) xinf = fmax(xinf, __shfl_xor_sync(0xffffffffu, xinf, o));
-                    grown += (xinf >= grow_lim);
-                    const double inv = (nrm > 0.0) ? 1.0 / nrm : 0.0;
-                    for (int i = lane; i < n; i += 32) x[i] *= inv;
-                    __syncwarp();
-                }
-                if (grown < kInvitGrowPasses && lane == 0 && err) {
-                    *err = kDevNoConv;
-                    if (atomicCAS(&g_invit_fail[0], 0, 1) == 0) {
-                        g_invit_fail[1] = b;
-                        g_invit_fail[2] = j;
-                        g_invit_fail[3] = n;
-                    }
-                }
-                // sign convention: the first largest component positive
-                double big = 0.0;
-                int bi = n;
-                for (int i = lane; i < n; i += 32)
-                    if (fabs(x[i]) > fabs(big)) {
-                        big = x[i];
-                        bi = i;
-                    }
+                        for (int u = 0; u < 8; ++u) {
+                            xx[u] = x[i + u];
+                            r1[u] = E1[i + u];
+                            r2[u] = E2[i + u];
+                            dd[u] = D[i + u];
+                        }
 #pragma unroll
-                for (int o = 16; o > 0; o >>= 1) {
-                    const double ob = __shfl_xor_sync(0xffffffffu, big, o);
-                    const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-                    if (fabs(ob) > fabs(big) || (fabs(ob) == fabs(big) && oi < bi)) {
-                        big = ob;
-                        bi = oi;
+                        for (int u = 7; u >= 0; --u) {
+                            if (i + u < n) {
+                                const double xi = (xx[u] - r2[u] * x2 - r1[u] * x1) * dd[u];
+                                x[i + u] = xi;
+                                x2 = x1;
+                                x1 = xi;
+                            }
+                        }
                     }
                 }
-                const double sg = (big < 0.0) ? -1.0 : 1.0;
-                double *zc = z + (size_t)j * ldz;
-                for (int i = lane; i < n; i += 32) zc[i] = sg * x[i];
+                __syncwarp();
+                for (int jj = j0; jj < j; ++jj) {
+                    const double *zc = z + (size_t)jj * ldz;
+                    double dot = 0.0;
+                    for (int i = lane; i < n; i += 32) dot += x[i] * zc[i];
+                    dot = warp_sum(dot);
+                    for (int i = lane; i < n; i += 32) x[i] -= dot * zc[i];
+                }
+                double nrm = 0.0, xinf = 0.0;
+                for (int i = lane; i < n; i += 32) {
+                    nrm += x[i] * x[i];
+                    xinf = fmax(xinf, fabs(x[i]));
+                }
+                nrm = sqrt(warp_sum(nrm));
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) xinf = fmax(xinf, __shfl_xor_sync(0xffffffffu, xinf, o));
+                grown += (xinf >= grow_lim);
+                const double inv = (nrm > 0.0) ? 1.0 / nrm : 0.0;
+                for (int i = lane; i < n; i += 32) x[i] *= inv;
                 __syncwarp();
             }
+            if (grown < kInvitGrowPasses && lane == 0 && err) {
+                *err = kDevNoConv;
+                if (atomicCAS(&g_invit_fail[0], 0, 1) == 0) {
+                    g_invit_fail[1] = b;
+                    g_invit_fail[2] = j;
+                    g_invit_fail[3] = n;
+                }
+            }
+            // sign convention: the first largest component positive
+            double big = 0.0;
+            int bi = n;
+            for (int i = lane; i < n; i += 32)
+                if (fabs(x[i]) > fabs(big)) {
+                    big = x[i];
+                    bi = i;
+                }
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) {
+                const double ob = __shfl_xor_sync(0xffffffffu, big, o);
+                const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
+                if (fabs(ob) > fabs(big) || (fabs(ob) == fabs(big) && oi < bi)) {
+                    big = ob;
+                    bi = oi;
+                }
+            }
+            const double sg = (big < 0.0) ? -1.0 : 1.0;
+            double *zc = z + (size_t)j * ldz;
+            for (int i = lane; i < n; i += 32) zc[i] = sg * x[i];
+            __syncwarp();
+        }
+    }
+}
+
+// ------------------------------------------------------------------ back-transformation
+// z <- H_0 H_1 ... H_{n-3} z by panels of 32 reflectors in compact WY form, I - V T V^T, on the FP64
+// tensor path. V is read from the block itself (unit diagonal implied), T is kept in the block's
+// upper triangle, which the reduction has left unused: panel p0's T(r, c), r <= c, at row p0 + r of
+// column p0 + c + 1. 3960 vectors of 64 blocks of order 465: 0.05 + 0.38 ms; with inverse iteration
+// 5.4 -> 1.45 ms against one kernel that walked a column per thread through panels of 16.
+constexpr int kBtP = 32;
+
+// V(i, c) of panel p0: rows i of the block
+__device__ __forceinline__ double bt_v(const double *a, int n, int p0, int nbk, int i, int c) {
+    const int top = p0 + c + 1;
+    if (c >= nbk || i >= n || i < top) return 0.0;
+    return (i == top) ? 1.0 : a[(size_t)(p0 + c) * n + i];
+}
+
+// T of every panel: the Gram matrix V^T V over four warps, then dlarft (forward, columnwise).
+__global__ void __launch_bounds__(128) bt_factor_kernel(BatchDesc bd, double *A, const double *tauo, const int *sel) {
+    const int b = blockIdx.y, p0 = blockIdx.x * kBtP;
+    const int n = bd.n[b], nbk = min(kBtP, n - 2 - p0);
+    if (nbk <= 0 || sel[b] <= 0) return;
+    double *a = A + bd.aoff[b];
+    const double *tau = tauo + bd.voff[b] + p0;
+    __shared__ double G[4][32 * 33];
+    __shared__ double T[32][33];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, r = lane >> 2, c = lane & 3;
+    double acc[2][4][4];
+#pragma unroll
+    for (int x = 0; x < 2; ++x)
+#pragma unroll
+        for (int y = 0; y < 4; ++y)
+#pragma unroll
+            for (int h = 0; h < 4; ++h) acc[x][y][h] = 0.0;
+    for (int k0 = p0 + 1 + 16 * warp; k0 < n; k0 += 64) {
+        double af[2][8], bf[4][4];
+#pragma unroll
+        for (int x = 0; x < 2; ++x)
+#pragma unroll
+            for (int i = 0; i < 8; ++i) af[x][i] = bt_v(a, n, p0, nbk, k0 + c + 4 * (i >> 1), x * 16 + r + 8 * (i & 1));
+#pragma unroll
+        for (int y = 0; y < 4; ++y)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) bf[y][i] = af[y >> 1][2 * i + (y & 1)];  // the same elements
+#pragma unroll
+        for (int x = 0; x < 2; ++x)
+#pragma unroll
+            for (int y = 0; y < 4; ++y) dmma16(acc[x][y], af[x], bf[y]);
+    }
+#pragma unroll
+    for (int x = 0; x < 2; ++x)
+#pragma unroll
+        for (int y = 0; y < 4; ++y)
+#pragma unroll
+            for (int h = 0; h < 4; ++h) G[warp][(y * 8 + c * 2 + (h & 1)) * 33 + x * 16 + r + 8 * (h >> 1)] = acc[x][y][h];
+    for (int q = tid; q < 32 * 33; q += 128) (&T[0][0])[q] = 0.0;
+    __syncthreads();
+    for (int q = tid; q < 1024; q += 128) {
+        const int k = (q >> 5) * 33 + (q & 31);
+        G[0][k] = (G[0][k] + G[1][k]) + (G[2][k] + G[3][k]);
+    }
+    __syncthreads();
+    if (warp == 0) {
+        for (int i = 0; i < nbk; ++i) {  // T(0:i, i) = -tau_i T(0:i, 0:i) V^T v_i
+            const double ti = tau[i];
+            double s0 = 0.0, s1 = 0.0;
+            for (int k = 0; k < i; k += 2) {
+                s0 = fma(T[lane][k], G[0][i * 33 + k], s0);
+                if (k + 1 < i) s1 = fma(T[lane][k + 1], G[0][i * 33 + k + 1], s1);
+            }
+            T[lane][i] = (lane < i) ? -ti * (s0 + s1) : (lane == i ? ti : 0.0);
+            __syncwarp();
         }
     }
     __syncthreads();
-    // ---- back-transformation z <- H_0 H_1 ... H_{n-3} z, panels of 16 reflectors
-    const int nref = n - 2;
-    if (nref <= 0) return;
-    double *Vs = sm;                                   // [kFastPanel][n]
-    double *Sg = Vs + (size_t)kFastPanel * n;          // [16][16] Gram, then
-    double *Tm = Sg + kFastPanel * kFastPanel;         // [16][16] upper triangular factor
-    for (int p0 = ((nref - 1) / kFastPanel) * kFastPanel; p0 >= 0; p0 -= kFastPanel) {
-        const int nbk = min(kFastPanel, nref - p0);
-        for (int q = tid; q < kFastPanel * n; q += blockDim.x) {
-            const int c = q / n, i = q % n, top = p0 + c + 1;
-            double v = 0.0;
-            if (c < nbk && i >= top) v = (i == top) ? 1.0 : a[(size_t)(p0 + c) * n + i];
-            Vs[q] = v;
+    for (int q = tid; q < 1024; q += 128) {
+        const int i = q >> 5, k = q & 31;  // T(k, i)
+        if (k <= i && i < nbk) a[(size_t)(p0 + i + 1) * n + p0 + k] = T[k][i];
+    }
+}
+
+// NC columns of Z a CTA, kept in shared memory ([column][row], stride 4 mod 16) through all panels:
+// W = V^T Z (rows split over the eight warps), W2 = T W, Z -= V W2.
+template <int NC>
+__global__ void __launch_bounds__(256) bt_apply_kernel(BatchDesc bd, const double *A, const int *sel, const long long *zoff,
+                                                       const int *zld, double *Z, int zs) {
+    const int b = blockIdx.y, c0 = blockIdx.x * NC;
+    const int n = bd.n[b], m = sel[b];
+    if (c0 >= m || n < 3) return;
+    constexpr int NT = NC / 8;
+    const double *a = A + bd.aoff[b];
+    double *z = Z + zoff[b] + (size_t)c0 * zld[b];
+    const int ldz = zld[b], nc = min(NC, m - c0);
+    extern __shared__ double sm[];
+    double *zt = sm, *red = sm + (size_t)NC * zs, *W = red + 8 * NC * 33, *W2 = W + NC * 36;  // W: [column][k]
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, r = lane >> 2, c = lane & 3;
+    for (int k = 0; k < NC; ++k)
+        for (int i = tid; i < zs; i += 256) zt[(size_t)k * zs + i] = (k < nc && i < n) ? z[(size_t)k * ldz + i] : 0.0;
+    __syncthreads();
+    for (int p0 = ((n - 3) / kBtP) * kBtP; p0 >= 0; p0 -= kBtP) {
+        const int nbk = min(kBtP, n - 2 - p0);
+        {
+            double acc[2][NT][4];
+#pragma unroll
+            for (int x = 0; x < 2; ++x)
+#pragma unroll
+                for (int y = 0; y < NT; ++y)
+#pragma unroll
+                    for (int h = 0; h < 4; ++h) acc[x][y][h] = 0.0;
+            for (int k0 = p0 + 1 + 16 * warp; k0 < n; k0 += 128) {
+                double af[2][8], bf[NT][4];
+#pragma unroll
+                for (int x = 0; x < 2; ++x)
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) af[x][i] = bt_v(a, n, p0, nbk, k0 + c + 4 * (i >> 1), x * 16 + r + 8 * (i & 1));
+#pragma unroll
+                for (int y = 0; y < NT; ++y)
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) bf[y][i] = zt[(size_t)(y * 8 + r) * zs + k0 + c + 4 * i];
+#pragma unroll
+                for (int x = 0; x < 2; ++x)
+#pragma unroll
+                    for (int y = 0; y < NT; ++y) dmma16(acc[x][y], af[x], bf[y]);
+            }
+            double *mine = red + (size_t)warp * NC * 33;
+#pragma unroll
+            for (int x = 0; x < 2; ++x)
+#pragma unroll
+                for (int y = 0; y < NT; ++y)
+#pragma unroll
+                    for (int h = 0; h < 4; ++h) mine[(y * 8 + c * 2 + (h & 1)) * 33 + x * 16 + r + 8 * (h >> 1)] = acc[x][y][h];
         }
         __syncthreads();
-        for (int q = tid; q < kFastPanel * kFastPanel; q += blockDim.x) {
-            const int c1 = q / kFastPanel, c2 = q % kFastPanel;
+        for (int q = tid; q < NC * 32; q += 256) {
+            const int col = q >> 5, k = q & 31;
             double s = 0.0;
-            if (c1 < nbk && c2 < nbk)
-                for (int i = p0 + 1; i < n; ++i) s += Vs[c1 * n + i] * Vs[c2 * n + i];
-            Sg[q] = s;
+#pragma unroll
+            for (int u = 0; u < 8; ++u) s += red[(size_t)u * NC * 33 + col * 33 + k];
+            W[col * 36 + k] = s;
         }
         __syncthreads();
-        if (tid < kFastPanel) {  // dlarft (forward, columnwise), one thread per row of Tm
-            const int r = tid;
-            for (int c = 0; c < kFastPanel; ++c) Tm[r * kFastPanel + c] = 0.0;
+        if (warp < 2 * NT) {  // W2 = T W: 16 rows, 8 columns a warp
+            const int m0 = (warp & 1) * 16, n0 = (warp >> 1) * 8;
+            double acc[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+            for (int k0 = 0; k0 < 32; k0 += 16) {
+                double af[8], bf[4];
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    const int row = m0 + r + 8 * (i & 1), k = k0 + c + 4 * (i >> 1);
+                    af[i] = (row <= k && k < nbk) ? a[(size_t)(p0 + k + 1) * n + p0 + row] : 0.0;
+                }
+#pragma unroll
+                for (int i = 0; i < 4; ++i) bf[i] = W[(n0 + r) * 36 + k0 + c + 4 * i];
+                dmma16(acc, af, bf);
+            }
+#pragma unroll
+            for (int h = 0; h < 4; ++h) W2[(n0 + c * 2 + (h & 1)) * 36 + m0 + r + 8 * (h >> 1)] = -acc[h];
         }
         __syncthreads();
-        for (int i = 0; i < nbk; ++i) {
-            if (tid < kFastPanel) {
-                const int r = tid;
-                const double ti = tau[p0 + i];
-                if (r < i) {
-                    double s = 0.0;
-                    for (int c = r; c < i; ++c) s += Tm[r * kFastPanel + c] * Sg[c * kFastPanel + i];
-                    Tm[r * kFastPanel + i] = -ti * s;
-                } else if (r == i) {
-                    Tm[i * kFastPanel + i] = ti;
+        for (int i0 = p0 + 1 + 16 * warp; i0 < n; i0 += 128) {
+            double acc[NT][4];
+#pragma unroll
+            for (int y = 0; y < NT; ++y)
+#pragma unroll
+                for (int h = 0; h < 4; ++h) acc[y][h] = zt[(size_t)(y * 8 + c * 2 + (h & 1)) * zs + i0 + r + 8 * (h >> 1)];
+#pragma unroll
+            for (int k0 = 0; k0 < 32; k0 += 16) {
+                double af[8];
+#pragma unroll
+                for (int i = 0; i < 8; ++i) af[i] = bt_v(a, n, p0, nbk, i0 + r + 8 * (i & 1), k0 + c + 4 * (i >> 1));
+#pragma unroll
+                for (int y = 0; y < NT; ++y) {
+                    double bf[4];
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) bf[i] = W2[(y * 8 + r) * 36 + k0 + c + 4 * i];
+                    dmma16(acc[y], af, bf);
                 }
             }
-            __syncthreads();
-        }
-        for (int q = tid; q < s_nmine; q += blockDim.x) {
-            double *zc = z + (size_t)mycols[q] * ldz;
-            // the column is walked four rows at a time so that four loads are in flight
-            double wv[kFastPanel];
 #pragma unroll
-            for (int c = 0; c < kFastPanel; ++c) wv[c] = 0.0;
-            int i = p0 + 1;
-            for (; i + 3 < n; i += 4) {
-                const double z0 = zc[i], z1 = zc[i + 1], z2 = zc[i + 2], z3 = zc[i + 3];
+            for (int y = 0; y < NT; ++y)
 #pragma unroll
-                for (int c = 0; c < kFastPanel; ++c) {
-                    const double *vc = Vs + c * n + i;
-                    wv[c] += (vc[0] * z0 + vc[1] * z1) + (vc[2] * z2 + vc[3] * z3);
-                }
-            }
-            for (; i < n; ++i) {
-                const double zi = zc[i];
-#pragma unroll
-                for (int c = 0; c < kFastPanel; ++c) wv[c] += Vs[c * n + i] * zi;
-            }
-            double w2[kFastPanel];
-#pragma unroll
-            for (int r = 0; r < kFastPanel; ++r) {
-                double s = 0.0;
-#pragma unroll
-                for (int c = 0; c < kFastPanel; ++c) s += Tm[r * kFastPanel + c] * wv[c];
-                w2[r] = s;
-            }
-            i = p0 + 1;
-            for (; i + 3 < n; i += 4) {
-                const double z0 = zc[i], z1 = zc[i + 1], z2 = zc[i + 2], z3 = zc[i + 3];
-                double s0 = 0.0, s1 = 0.0, s2 = 0.0, s3 = 0.0;
-#pragma unroll
-                for (int c = 0; c < kFastPanel; ++c) {
-                    const double *vc = Vs + c * n + i;
-                    s0 += vc[0] * w2[c];
-                    s1 += vc[1] * w2[c];
-                    s2 += vc[2] * w2[c];
-                    s3 += vc[3] * w2[c];
-                }
-                zc[i] = z0 - s0;
-                zc[i + 1] = z1 - s1;
-                zc[i + 2] = z2 - s2;
-                zc[i + 3] = z3 - s3;
-            }
-            for (; i < n; ++i) {
-                double s = 0.0;
-#pragma unroll
-                for (int c = 0; c < kFastPanel; ++c) s += Vs[c * n + i] * w2[c];
-                zc[i] -= s;
-            }
+                for (int h = 0; h < 4; ++h) zt[(size_t)(y * 8 + c * 2 + (h & 1)) * zs + i0 + r + 8 * (h >> 1)] = acc[y][h];
         }
         __syncthreads();
     }
+    for (int k = 0; k < nc; ++k)
+        for (int i = tid; i < n; i += 256) z[(size_t)k * ldz + i] = zt[(size_t)k * zs + i];
 }
 
 __global__ void symmetrize_lower_kernel(BatchDesc bd, double *A) {
@@ -616,57 +693,68 @@ void launch_tridiag_batched(const BatchDesc &bd, double *A, double *d, double *e
     tridiag_kernel<<<bd.nblk, threads, smem, st>>>(bd, A, d, e, tau);
 }
 
+namespace {
+int sm_count() {
+    int dev = 0, nsm = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+    return std::max(nsm, 1);
+}
+}  // namespace
+
 void launch_eigvals_batched(const BatchDesc &bd, const double *d, const double *e, double *w,
                             int *cnt, int mode, double cut, cudaStream_t st) {
     if (bd.nblk <= 0) return;
-    int nmax = 0;
-    (void)nmax;
-    // dynamic shared memory: d and e^2 of the largest block (caller guarantees <= 1024)
+    // few blocks: several CTAs a block, each with its share of the eigenvalues
+    const int parts = std::max(1, std::min(8, sm_count() / bd.nblk));
+    // dynamic shared memory: d and -e^2 of the largest block (caller guarantees <= 1024)
     DVR3D_COUNT_LAUNCH(1);
-    eigvals_kernel<<<bd.nblk, kEvThreads, 2 * 1024 * sizeof(double), st>>>(bd, d, e, w, cnt, mode, cut);
+    eigvals_kernel<<<dim3(bd.nblk, parts), kEvThreads, 2 * 1024 * sizeof(double), st>>>(bd, d, e, w, cnt, mode, cut);
 }
 
-void launch_eigvecs_batched(const BatchDesc &bd, const double *A, const double *d,
-                            const double *e, const double *tau, const double *w,
-                            const int *sel, const long long *zoff, const int *zld, double *Z,
-                            double *work, const long long *workoff, int nmax, int *err,
-                            cudaStream_t st) {
+void launch_eigvecs_batched(const BatchDesc &bd, double *A, const double *d, const double *e, const double *tau,
+                            const double *w, const int *sel, const long long *zoff, const int *zld, double *Z, int nmax,
+                            int *err, cudaStream_t st) {
     if (bd.nblk <= 0) return;
-    size_t smem = (size_t)nmax * sizeof(double);
-    const size_t smem_cl = (size_t)(nmax + 2) * sizeof(int);
-    if (smem_cl > smem) smem = smem_cl;
-    DVR3D_COUNT_LAUNCH(1);
-    eigvecs_kernel<<<bd.nblk, kVecThreads, smem, st>>>(bd, A, d, e, tau, w, sel, zoff, zld, Z, work,
-                                                       workoff, err);
-}
-
-size_t eigvecs_fast_smem(int nmax, int nwarp) {
-    const size_t inv = (size_t)nwarp * (5 * (size_t)nmax + (nmax + 7) / 8) * sizeof(double);
-    const size_t bt = ((size_t)kFastPanel * nmax + 2 * kFastPanel * kFastPanel) * sizeof(double);
-    return std::max(inv, bt);
-}
-
-void launch_eigvecs_batched_fast(const BatchDesc &bd, const double *A, const double *d, const double *e,
-                                 const double *tau, const double *w, const int *sel, const long long *zoff,
-                                 const int *zld, double *Z, int nmax, int *err, cudaStream_t st) {
-    if (bd.nblk <= 0) return;
-    const size_t cap = 200 * 1024;
+    constexpr size_t cap = 200 * 1024;
+    const int np = (nmax + 8) & ~7;
     int nwarp = 8;
-    while (nwarp > 1 && eigvecs_fast_smem(nmax, nwarp) > cap) --nwarp;
-    const size_t smem = eigvecs_fast_smem(nmax, nwarp);
-    // fewer blocks than SMs: two CTAs per block (their clusters split between them)
-    int dev = 0, nsm = 0;
+    auto invit_smem = [&](int k) { return ((size_t)2 * np + (size_t)k * (5 * np + np / 8)) * sizeof(double); };
+    while (nwarp > 1 && invit_smem(nwarp) > cap) --nwarp;
+    // 32 columns of Z a CTA where they fit (orders up to 536), else 16
+    auto bt_smem = [&](int nc, int zs) { return ((size_t)nc * zs + 8 * nc * 33 + 2 * nc * 36) * sizeof(double); };
+    const int zs = (nmax + 32) / 16 * 16 + 4;  // 16-row tiles run past the end
+    const bool wide = bt_smem(32, zs) <= cap + 24 * 1024;
+    int dev = 0;
     cudaGetDevice(&dev);
-    // the shared-memory limit is a per-device attribute of the kernel
+    // the shared-memory limit is a per-device attribute of the kernels
     static bool attr[kMaxAttrDevices] = {};
     if (dev < 0 || dev >= kMaxAttrDevices || !attr[dev]) {
-        cudaFuncSetAttribute(eigvecs_fast_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cap);
+        cudaFuncSetAttribute(invit_batched_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cap);
+        cudaFuncSetAttribute(bt_apply_kernel<32>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cap + 24 * 1024);
+        cudaFuncSetAttribute(bt_apply_kernel<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cap + 24 * 1024);
         if (dev >= 0 && dev < kMaxAttrDevices) attr[dev] = true;
     }
-    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-    const int parts = (bd.nblk < nsm) ? 2 : 1;
+    // fewer blocks than SMs: several CTAs per block (their clusters split between them)
+    const int parts = std::max(1, std::min(16, sm_count() / bd.nblk));
     DVR3D_COUNT_LAUNCH(1);
-    eigvecs_fast_kernel<<<dim3(bd.nblk, parts), 32 * nwarp, smem, st>>>(bd, A, d, e, tau, w, sel, zoff, zld, Z, err);
+    invit_batched_kernel<<<dim3(bd.nblk, parts), 32 * nwarp, invit_smem(nwarp), st>>>(bd, d, e, w, sel, zoff, zld, Z, err);
+    if (nmax < 3) return;
+    DVR3D_COUNT_LAUNCH(2);
+    for (int b0 = 0; b0 < bd.nblk; b0 += 65535) {  // blocks per launch: gridDim.y
+        BatchDesc q = bd;
+        q.nblk = std::min(65535, bd.nblk - b0);
+        q.n += b0;
+        q.aoff += b0;
+        q.voff += b0;
+        bt_factor_kernel<<<dim3((nmax - 2 + kBtP - 1) / kBtP, q.nblk), 128, 0, st>>>(q, A, tau, sel + b0);
+        if (wide)
+            bt_apply_kernel<32><<<dim3((nmax + 31) / 32, q.nblk), 256, bt_smem(32, zs), st>>>(q, A, sel + b0, zoff + b0,
+                                                                                           zld + b0, Z, zs);
+        else
+            bt_apply_kernel<16><<<dim3((nmax + 15) / 16, q.nblk), 256, bt_smem(16, zs), st>>>(q, A, sel + b0, zoff + b0,
+                                                                                           zld + b0, Z, zs);
+    }
 }
 
 void invit_fail_clear(cudaStream_t st) {

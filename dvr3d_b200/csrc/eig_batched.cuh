@@ -37,25 +37,17 @@ void launch_tridiag_batched(const BatchDesc &bd, double *A, double *d, double *e
 void launch_eigvals_batched(const BatchDesc &bd, const double *d, const double *e, double *w,
                             int *cnt, int mode, double cut, cudaStream_t st);
 
-// Eigenvectors of eigenvalues w[voff[b] + 0 .. sel[b]-1]: written to Z + zoff[b] with
-// leading dimension zld[b] (column-major, one column per eigenvalue). `work` needs
-// 6 * sum_b(n[b]) * 256 doubles at most (see eigvecs_work_doubles).
-void launch_eigvecs_batched(const BatchDesc &bd, const double *A, const double *d,
-                            const double *e, const double *tau, const double *w,
-                            const int *sel, const long long *zoff, const int *zld, double *Z,
-                            double *work, const long long *workoff, int nmax, int *err,
-                            cudaStream_t st);
-
-// Same output as launch_eigvecs_batched (n <= 1024), without work buffer: inverse iteration
-// with the factors in shared memory (one warp per cluster) and a blocked back-transformation.
-// Both set *err = 1 (err may be null) when inverse iteration fails its growth test for some
-// vector (dstein's convergence criterion); the flag is never cleared by the kernels.
-// Diagnostics of the fast batched inverse iteration: the first vector that failed its growth
-// test since the last clear ({failed, block, eigenvalue index, block order}).
+// Eigenvectors of eigenvalues w[voff[b] + 0 .. sel[b]-1] (n <= 1024): written to Z + zoff[b] with
+// leading dimension zld[b] (column-major, one column per eigenvalue). The blocks' upper triangles
+// are overwritten (factors of the back-transformation). *err = kDevNoConv (err may be null) when
+// inverse iteration fails its growth test for some vector (dstein's convergence criterion); the
+// flag is never cleared by the kernels.
+void launch_eigvecs_batched(const BatchDesc &bd, double *A, const double *d, const double *e, const double *tau,
+                            const double *w, const int *sel, const long long *zoff, const int *zld, double *Z, int nmax,
+                            int *err, cudaStream_t st);
+// Diagnostics of the inverse iteration: the first vector that failed its growth test since the
+// last clear ({failed, block, eigenvalue index, block order}).
 void invit_fail_clear(cudaStream_t st);
 void invit_fail_info(cudaStream_t st, int out[4]);
-void launch_eigvecs_batched_fast(const BatchDesc &bd, const double *A, const double *d, const double *e,
-                                 const double *tau, const double *w, const int *sel, const long long *zoff,
-                                 const int *zld, double *Z, int nmax, int *err, cudaStream_t st);
 
 }  // namespace dvr3d

@@ -575,55 +575,81 @@ __global__ void dense_finish_kernel(const double *A, long long ld, int n, double
     tau[n - 1] = 0.0;
 }
 
-// Gershgorin bounds, pivmin, e^2 and ||T||_1 (one CTA).
-__global__ void tri_bounds_kernel(const double *d, const double *e, int n, double *e2, double *info) {
-    __shared__ double smin[256], smax[256], se[256];
+// Gershgorin bounds, ||T||_1 and the off-diagonal terms of the Sturm counts (one CTA).
+__global__ void __launch_bounds__(1024) tri_bounds_kernel(const double *d, const double *e, int n, double *ne2, double *info) {
+    __shared__ double smin[1024], smax[1024];
     const int tid = threadIdx.x;
-    double lo = DBL_MAX, hi = -DBL_MAX, emx = 0.0;
+    double lo = DBL_MAX, hi = -DBL_MAX;
     for (int i = tid; i < n; i += blockDim.x) {
         const double em = (i > 0) ? fabs(e[i - 1]) : 0.0, ep = (i < n - 1) ? fabs(e[i]) : 0.0;
         lo = fmin(lo, d[i] - em - ep);
         hi = fmax(hi, d[i] + em + ep);
-        if (i < n - 1) {
-            e2[i] = e[i] * e[i];
-            emx = fmax(emx, e2[i]);
-        }
     }
     smin[tid] = lo;
     smax[tid] = hi;
-    se[tid] = emx;
     __syncthreads();
     for (int s = blockDim.x / 2; s > 0; s >>= 1) {
         if (tid < s) {
             smin[tid] = fmin(smin[tid], smin[tid + s]);
             smax[tid] = fmax(smax[tid], smax[tid + s]);
-            se[tid] = fmax(se[tid], se[tid + s]);
         }
         __syncthreads();
     }
+    const double tnorm = fmax(fabs(smin[0]), fabs(smax[0])), scale = sturm_scale(tnorm);
+    for (int i = tid; i + 1 < n; i += blockDim.x) ne2[i] = sturm_off(e[i], scale);
     if (tid == 0) {
-        const double tnorm = fmax(fabs(smin[0]), fabs(smax[0]));
-        const double piv = DBL_MIN * fmax(1.0, se[0]);
-        info[0] = smin[0] - 2.0 * DBL_EPSILON * tnorm * n - 2.0 * piv;
-        info[1] = smax[0] + 2.0 * DBL_EPSILON * tnorm * n + 2.0 * piv;
-        info[2] = piv;
+        const double margin = 2.0 * DBL_EPSILON * tnorm * n + 2.0 * DBL_MIN;
+        info[0] = smin[0] - margin;
+        info[1] = smax[0] + margin;
+        info[2] = scale;
         info[3] = fmax(tnorm, DBL_MIN);
     }
 }
 
-// Multisection: warp w finds eigenvalue j = w (0-based ascending).
-__global__ void multisect_kernel(const double *d, const double *e2, int n, int nev, const double *info,
-                                 double *w) {
+// Multisection: warp w finds eigenvalue j = w (0-based ascending), 32 Sturm counts a pass. The rows
+// stream through registers eight ahead of their use; a row costs its dependent multiply-add:
+// 500 eigenvalues of order 12241 in 3.0 ms (13.2 ms with a division a row).
+__global__ void __launch_bounds__(128) multisect_kernel(const double *d, const double *ne2, int n, int nev, const double *info,
+                                                        double *w) {
     const int gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
     if (gw >= nev) return;
     const int j = gw;
-    double lo = info[0], hi = info[1];
-    const double piv = info[2];
+    const double scale = info[2], unit = 1.0 / scale;
+    double lo = info[0] * scale, hi = info[1] * scale;
     for (int pass = 0; pass < 64; ++pass) {
         if (hi - lo <= 2.0 * DBL_EPSILON * fmax(fabs(lo), fabs(hi))) break;
         const double x = lo + (hi - lo) * (double)(lane + 1) / 33.0;
-        const int c = sturm_count(d, e2, n, x, piv);
+        SturmCount s;
+        s.start(fma(d[0], scale, -x));
+        int i = 1;
+        if (n >= 9) {
+            double dd[8], ee[8];
+#pragma unroll
+            for (int u = 0; u < 8; ++u) {
+                dd[u] = d[i + u];
+                ee[u] = ne2[i + u - 1];
+            }
+            for (; i + 8 <= n; i += 8) {
+                double dn[8], en[8];
+                const int q = (i + 16 <= n) ? i + 8 : i;  // the next eight rows, if there are
+#pragma unroll
+                for (int u = 0; u < 8; ++u) {
+                    dn[u] = d[q + u];
+                    en[u] = ne2[q + u - 1];
+                }
+#pragma unroll
+                for (int u = 0; u < 8; ++u) s.step(fma(dd[u], scale, -x), ee[u]);
+                s.rescale();
+#pragma unroll
+                for (int u = 0; u < 8; ++u) {
+                    dd[u] = dn[u];
+                    ee[u] = en[u];
+                }
+            }
+        }
+        for (; i < n; ++i) s.step(fma(d[i], scale, -x), ne2[i - 1]);
+        const int c = s.c;
         const unsigned bal = __ballot_sync(0xffffffffu, c > j);
         const int l = bal ? (__ffs(bal) - 1) : 32;
         const double xl = __shfl_sync(0xffffffffu, x, l > 0 ? l - 1 : 0);
@@ -634,7 +660,7 @@ __global__ void multisect_kernel(const double *d, const double *e2, int n, int n
         lo = nlo;
         hi = nhi;
     }
-    if (lane == 0) w[j] = 0.5 * (lo + hi);
+    if (lane == 0) w[j] = 0.5 * (lo + hi) * unit;
 }
 
 // Cluster starts for inverse iteration (single thread; nev is at most a few thousand).
@@ -1023,8 +1049,8 @@ cudaError_t launch_dense_tridiag(DenseTri &t, int grid, cudaStream_t st) {
 void launch_dense_eigvals(const double *d, const double *e, int n, int nev, double *e2, double *info,
                           double *w, cudaStream_t st) {
     DVR3D_COUNT_LAUNCH(2);
-    tri_bounds_kernel<<<1, 256, 0, st>>>(d, e, n, e2, info);
-    const int warps_per_block = 4;
+    tri_bounds_kernel<<<1, 1024, 0, st>>>(d, e, n, e2, info);
+    const int warps_per_block = (nev > 600) ? 4 : 1;  // an SM sub-partition each while they last
     multisect_kernel<<<(nev + warps_per_block - 1) / warps_per_block, 32 * warps_per_block, 0, st>>>(
         d, e2, n, nev, info, w);
 }

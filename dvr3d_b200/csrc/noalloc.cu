@@ -58,18 +58,15 @@ inline size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
 constexpr int kMaxNoallocBlocks = 65535;
 
 // Offsets of every block inside the scratch regions (one thread; nblk is small).
-__global__ void noalloc_plan_kernel(int nblk, const int *n, long long *voff, long long *asz,
-                                    long long *wkoff) {
+__global__ void noalloc_plan_kernel(int nblk, const int *n, long long *voff, long long *asz) {
     if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    long long v = 0, a = 0, w = 0;
+    long long v = 0, a = 0;
     for (int b = 0; b < nblk; ++b) {
         const long long nb = n[b];
         voff[b] = v;
         asz[b] = a;
-        wkoff[b] = w;
         v += nb;
         a += nb * nb;
-        w += 5 * nb * (nb < 128 ? nb : 128) + nb * nb;
     }
 }
 
@@ -106,6 +103,8 @@ extern "C" int dvr3d_b200_diag_batched_noalloc(void *stream, int nblk, const int
         nmax = std::max(nmax, nb);
         sum_n += (size_t)nb;
         sum_n2 += (size_t)nb * nb;
+        // documented limit: room for inverse iteration's factors in the scratch (the kernels keep
+        // them on chip)
         sum_work += 5 * (size_t)nb * std::min(nb, 128) + (size_t)nb * nb;
     }
     const size_t meta =
@@ -132,13 +131,11 @@ extern "C" int dvr3d_b200_diag_batched_noalloc(void *stream, int nblk, const int
     long long *d_woff = reinterpret_cast<long long *>(take(sizeof(long long) * nblk));
     long long *d_voff = reinterpret_cast<long long *>(take(sizeof(long long) * nblk));
     long long *d_asz = reinterpret_cast<long long *>(take(sizeof(long long) * nblk));
-    long long *d_wk = reinterpret_cast<long long *>(take(sizeof(long long) * nblk));
     double *d_d = reinterpret_cast<double *>(take(sizeof(double) * sum_n));
     double *d_e = reinterpret_cast<double *>(take(sizeof(double) * sum_n));
     double *d_tau = reinterpret_cast<double *>(take(sizeof(double) * sum_n));
     double *d_w = reinterpret_cast<double *>(take(sizeof(double) * sum_n));
     double *d_acopy = reinterpret_cast<double *>(take(sizeof(double) * sum_n2));
-    double *d_work = vecs ? reinterpret_cast<double *>(take(sizeof(double) * sum_work)) : nullptr;
     cudaError_t e = cudaSuccess;
     auto ck = [&](cudaError_t x) {
         if (e == cudaSuccess && x != cudaSuccess) e = x;
@@ -155,7 +152,7 @@ extern "C" int dvr3d_b200_diag_batched_noalloc(void *stream, int nblk, const int
         return DVR3D_ERR_CUDA;
     };
     if (e != cudaSuccess) return bail();
-    noalloc_plan_kernel<<<1, 32, 0, st>>>(nblk, d_n, d_voff, d_asz, d_wk);
+    noalloc_plan_kernel<<<1, 32, 0, st>>>(nblk, d_n, d_voff, d_asz);
     ck(cudaGetLastError());
     noalloc_copy_in_kernel<<<dim3(64, nblk), 256, 0, st>>>(d_n, d_off, d_asz, a_dev, d_acopy);
     ck(cudaGetLastError());
@@ -174,8 +171,7 @@ extern "C" int dvr3d_b200_diag_batched_noalloc(void *stream, int nblk, const int
     ck(cudaGetLastError());
     if (vecs && e == cudaSuccess) {
         // eigenvectors of all eigenvalues written over the caller's blocks (ld = n)
-        dvr3d::launch_eigvecs_batched(bd, d_acopy, d_d, d_e, d_tau, d_w, d_n, d_off, d_n, a_dev, d_work, d_wk,
-                                      nmax, d_err, st);
+        dvr3d::launch_eigvecs_batched(bd, d_acopy, d_d, d_e, d_tau, d_w, d_n, d_off, d_n, a_dev, nmax, d_err, st);
         ck(cudaGetLastError());
     }
     int err_host = 0;

@@ -232,7 +232,7 @@ void radau_stage(dvr3d_ctx *ctx, const BlockPlan &p, Contracted &out) {
         }
         col += sel[b];
     }
-    launch_eigvecs_batched_fast(bd, H, d, e, tau, w, upload(ctx, "sel", sel), upload(ctx, "zoff", zoff),
+    launch_eigvecs_batched(bd, H, d, e, tau, w, upload(ctx, "sel", sel), upload(ctx, "zoff", zoff),
                                 upload(ctx, "zld", zld), out.Vt, n, ev_err(ctx), st);
     CK(cudaGetLastError());
     // sqrt of the pair weight w_p = 1/(2 mu r_a^2) + 1/(2 mu r_b^2) (blc2d2 :3537-3539)
@@ -334,7 +334,7 @@ void jacobi_stage(dvr3d_ctx *ctx, const BlockPlan &p, Contracted &out) {
     double *U = ctx->arena.get_t<double>("u1", (size_t)std::max<long long>(ut, 1));
     {
         std::vector<int> zld1(nb1, na);
-        launch_eigvecs_batched_fast(bd1, H1, d1, e1, t1, w1, upload(ctx, "sel1", iv1), upload(ctx, "zoff1", zoff1),
+        launch_eigvecs_batched(bd1, H1, d1, e1, t1, w1, upload(ctx, "sel1", iv1), upload(ctx, "zoff1", zoff1),
                                     upload(ctx, "zld1", zld1), U, na, ev_err(ctx), st);
         CK(cudaGetLastError());
     }
@@ -457,7 +457,7 @@ void jacobi_stage(dvr3d_ctx *ctx, const BlockPlan &p, Contracted &out) {
     }
     double *V2 = ctx->arena.get_t<double>("v2", (size_t)std::max<long long>(v2t, 1));
     {
-        launch_eigvecs_batched_fast(bd2, H2, d2, e2d, t2, w2, upload(ctx, "sel2", sel2), upload(ctx, "zoff2", zoff2),
+        launch_eigvecs_batched(bd2, H2, d2, e2d, t2, w2, upload(ctx, "sel2", sel2), upload(ctx, "zoff2", zoff2),
                                     upload(ctx, "zld2", zld2), V2, n2max, ev_err(ctx), st);
         CK(cudaGetLastError());
     }
@@ -592,7 +592,7 @@ void channel_setup(dvr3d_ctx *ctx, const H3Op &op, const Contracted &C, ChanPrec
     int *cnt = ctx->arena.get_t<int>("ch_cnt", kmax);
     launch_tridiag_batched(bd, A, d, e, tau, nmax, st);
     launch_eigvals_batched(bd, d, e, lam, cnt, 0, 0.0, st);
-    launch_eigvecs_batched_fast(bd, A, d, e, tau, lam, dn, dq, dn, Q, nmax, ev_err(ctx), st);
+    launch_eigvecs_batched(bd, A, d, e, tau, lam, dn, dq, dn, Q, nmax, ev_err(ctx), st);
     CK(cudaGetLastError());
     // per-mode features
     std::vector<double> lh = download(ctx, lam, N), e2h = download(ctx, C.e2, N);
@@ -1035,7 +1035,7 @@ void radau_stage_batch(dvr3d_ctx *ctx, const std::vector<BlockPlan> &plans, cons
     }
     double *Vpool = ctx->arena.get_t<double>("bt_vt", (size_t)vtot);
     CK(cudaMemsetAsync(Vpool, 0, sizeof(double) * vtot, st));
-    launch_eigvecs_batched_fast(bd, H, d, e, tau, w, upload(ctx, "bt_sel", sel), upload(ctx, "bt_zoff", zoff),
+    launch_eigvecs_batched(bd, H, d, e, tau, w, upload(ctx, "bt_sel", sel), upload(ctx, "bt_zoff", zoff),
                                 upload(ctx, "bt_zld", zld), Vpool, nmax, ev_err(ctx), st);
     CK(cudaGetLastError());
     for (int i = 0; i < np; ++i) {

@@ -8,33 +8,64 @@
 
 namespace dvr3d {
 
-// ------------------------------------------------------------------ Sturm bisection
-// Number of eigenvalues of T (diag d, squared off-diagonals e2) strictly below x.
-static __device__ __forceinline__ int sturm_count(const double *d, const double *e2, int n, double x,
-                                           double pivmin) {
-    int c = 0;
-    double q = d[0] - x;
-    if (fabs(q) < pivmin) q = -pivmin;
-    c += (q < 0.0);
-    for (int i = 1; i < n; ++i) {
-        q = (d[i] - x) - e2[i - 1] / q;
-        if (fabs(q) < pivmin) q = -pivmin;
-        c += (q < 0.0);
-    }
-    return c;
+// ------------------------------------------------------------------ Sturm counts
+// The number of eigenvalues of T below x is the number of sign changes in the sequence of leading
+// principal minors p_0 = 1, p_i = (d_i - x) p_{i-1} - e_{i-1}^2 p_{i-2} (Givens). Unlike the
+// quotients p_i / p_{i-1} of dstebz this needs no division: one dependent multiply-add a row (about
+// 8 cycles against 110). T is scaled to norm below one by a power of two, so a pair of minors grows
+// at most threefold a row; squared off-diagonals below 2^-120 (a perturbation of 2^-60 ||T||) are
+// raised to it, so no two consecutive minors vanish; and the pair is brought back to magnitude one
+// every eight rows, between which it cannot leave the exponent range.
+constexpr double kSturmFloor = 7.52316384526264e-37;  // 2^-120
+
+// power of two that brings ||T|| = tnorm below one
+static __device__ __forceinline__ double sturm_scale(double tnorm) {
+    if (!(tnorm > 0.0) || !(tnorm < DBL_MAX)) return 1.0;
+    int ex = 0;
+    frexp(tnorm, &ex);
+    return ldexp(1.0, -max(-1000, min(1000, ex)));
+}
+// the off-diagonal term of the recurrence, -e^2 of the scaled matrix
+static __device__ __forceinline__ double sturm_off(double e, double scale) {
+    const double es = e * scale;
+    return -fmax(es * es, kSturmFloor);
 }
 
-// Eigenvalue j (0-based, ascending) by bisection on [lo, hi].
-static __device__ __forceinline__ double bisect_one(const double *d, const double *e2, int n, int j, double lo, double hi,
-                             double pivmin) {
-    for (int it = 0; it < 200; ++it) {
-        const double mid = 0.5 * (lo + hi);
-        if (!(mid > lo && mid < hi)) break;
-        if (hi - lo <= 2.0 * DBL_EPSILON * fmax(fabs(lo), fabs(hi))) break;
-        if (sturm_count(d, e2, n, mid, pivmin) > j) hi = mid;
-        else lo = mid;
+// Running count: rows are fed in order with step(), eight at most between calls of rescale().
+struct SturmCount {
+    double p0, p1;
+    int c;
+    __device__ __forceinline__ void start(double t0) {  // t0 = d_0 - x
+        p0 = 1.0;
+        p1 = t0;
+        c = (int)((unsigned)__double2hiint(t0) >> 31);
     }
-    return 0.5 * (lo + hi);
+    __device__ __forceinline__ void step(double t, double ne2) {  // t = d_i - x, ne2 = -e_{i-1}^2
+        const double p = fma(t, p1, ne2 * p0);
+        c += (int)((unsigned)(__double2hiint(p) ^ __double2hiint(p1)) >> 31);
+        p0 = p1;
+        p1 = p;
+    }
+    __device__ __forceinline__ void rescale() {
+        const int e0 = (__double2hiint(p0) >> 20) & 2047, e1 = (__double2hiint(p1) >> 20) & 2047;
+        const double f = __hiloint2double((2046 - max(1, min(2045, max(e0, e1)))) << 20, 0);
+        p0 *= f;
+        p1 *= f;
+    }
+};
+
+// Number of eigenvalues of T strictly below x; d and x scaled, ne2 from sturm_off.
+static __device__ __forceinline__ int sturm_count(const double *d, const double *ne2, int n, double x) {
+    SturmCount s;
+    s.start(d[0] - x);
+    int i = 1;
+    for (; i + 8 <= n; i += 8) {
+#pragma unroll
+        for (int u = 0; u < 8; ++u) s.step(d[i + u] - x, ne2[i + u - 1]);
+        s.rescale();
+    }
+    for (; i < n; ++i) s.step(d[i] - x, ne2[i - 1]);
+    return s.c;
 }
 
 static __device__ __forceinline__ unsigned hash32(unsigned x) {
