@@ -1,5 +1,7 @@
 // eig_batched.cu -- batched FP64 symmetric eigensolver kernels (one CTA per block).
 // See eig_batched.cuh for the role of each stage and the reference routines replaced.
+#include <cooperative_groups.h>
+
 #include <algorithm>
 #include <cfloat>
 #include <cmath>
@@ -13,143 +15,317 @@ namespace dvr3d {
 
 namespace {
 
-constexpr int kTriMaxThreads = 1024;  // one row per thread -> n <= 1024
-
 // ------------------------------------------------------------------ tridiagonalisation
-// Lower Householder reduction as dsytd2('L'): for k = 0..n-3 the reflector
-// H_k = I - tau_k v v^T, v = (0..0, 1, v_{k+2..n-1}), annihilates A[k+2:, k].
-// The rank-2 update of step k-1 is applied lazily: to column k first (so the reflector
-// of step k can be formed), then fused with the symmetric product A22 v_k of step k, so
-// the trailing block is read and written once per step.
-__global__ void __launch_bounds__(kTriMaxThreads) tridiag_kernel(BatchDesc bd, double *A, double *dg,
-                                                               double *eo, double *tauo) {
-    const int b = blockIdx.x;
-    if (b >= bd.nblk) return;
+// Lower Householder reduction as dsytd2('L'): for k = 0..n-3 the reflector H_k = I - tau_k v v^T,
+// v = (0..0, 1, v_{k+2..n-1}), annihilates A[k+2:, k]. Columns are formed in panels of eight from the
+// panel-start matrix (the dlatrd scheme: A v needs one read of the trailing matrix and no write; the
+// matrix itself is updated once a panel, a rank-16 DMMA product over both triangles). A column k is a
+// chain, kept short: the product with the trailing matrix and the panel's dot products use the
+// column x itself and run beside its norm (v = e_{k+1} + sc x), every thread forms the reflector's
+// scalars, and three block barriers and one exchange are left. A cluster of C CTAs shares a block:
+// each takes every C-th column of the product and writes its partial sums to all; the vectors are
+// replicated; the block stays in L2.
+// Bound by that read (about 20 bytes a cycle and SM from L2) and, for small blocks, by the chain. 64
+// blocks of order 465: 10.8 -> 5.1 ms against one CTA a block that read and wrote the trailing matrix
+// for every column; 80 of order 300: 3.6 -> 2.4, 500 of order 300: 15.4 -> 9.5, 20 of order 1000:
+// 90 -> 40 ms. Two CTAs a block (8.3 -> 5.1 ms for the 64) lose once they share an SM's L2 port.
+constexpr int kTriNb = 8;
+constexpr int kTriSmem = 152;
+constexpr int kTriParts = 4;  // partial sums a row: C CTAs x 4 / C column subsets
+
+template <int C>
+__global__ void __launch_bounds__(1024) tridiag_kernel(BatchDesc bd, double *A, double *dg, double *eo, double *tauo, int ns) {
+    namespace cg = cooperative_groups;
+    const int b = blockIdx.x / C, rank = blockIdx.x % C;
     const int n = bd.n[b];
-    double *a = A + bd.aoff[b];
+    double *ag = A + bd.aoff[b];
     double *d = dg + bd.voff[b], *e = eo + bd.voff[b], *tau = tauo + bd.voff[b];
     extern __shared__ double sm[];
-    double *vp = sm, *wp = sm + n, *v = sm + 2 * n;  // pending (v, w) and current v
-    __shared__ double red[32];
-    __shared__ double s_beta, s_tau, s_scal;
-    const int tid = threadIdx.x;
-    if (n == 1) {
-        if (tid == 0) {
-            d[0] = a[0];
-            e[0] = 0.0;
-            tau[0] = 0.0;
-        }
-        return;
-    }
-    bool pending = false;
+    double *V = sm, *W = V + kTriNb * ns, *xs = W + kTriNb * ns, *sp0 = xs + ns;
+    __shared__ double part[32], part2[32], zs[2 * kTriNb];
+    const int T = blockDim.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = T >> 5;
+    auto get = [&](int r, int c) { return __ldcg(ag + (unsigned)(c * n + r)); };
+    auto exchange = [&]() {
+        if constexpr (C > 1) cg::this_cluster().sync();
+        else __syncthreads();
+    };
+    if (tid < 32) part[tid] = part2[tid] = 0.0;
+    __syncthreads();
+    const int row = tid;  // the row of this thread in the vector steps
+    double acol = (row < n) ? get(row, 0) : 0.0, x = 0.0;
     for (int k = 0; k + 2 < n; ++k) {
-        // (1) finish column k: A[i,k] -= vp_i wp_k + wp_i vp_k, i >= k
-        if (pending) {
-            const double vk = vp[k], wk = wp[k];
-            for (int i = k + tid; i < n; i += blockDim.x) a[(size_t)k * n + i] -= vp[i] * wk + wp[i] * vk;
+        const int i = k % kTriNb;
+        if (i == 0 && k > 0) {
+            // ---- A -= V W^T + W V^T on rows and columns k.. (16 rows x 16 columns a task)
+            const int m = n - k, rt = (m + 15) / 16, ct = (m + 15) / 16, g = lane >> 2, t = lane & 3;
+            for (int q = rank * nw + warp; q < rt * ct; q += C * nw) {
+                const int r0 = k + (q % rt) * 16, c0 = k + (q / rt) * 16;
+                double af[8];
+#pragma unroll
+                for (int h = 0; h < 8; ++h) af[h] = ((h >> 2) ? W : V)[(t + 4 * ((h >> 1) & 1)) * ns + r0 + g + 8 * (h & 1)];
+                double acc[2][4];
+#pragma unroll
+                for (int y = 0; y < 2; ++y)
+#pragma unroll
+                    for (int h = 0; h < 4; ++h) {
+                        const int r = r0 + g + 8 * (h >> 1), c = c0 + 8 * y + 2 * t + (h & 1);
+                        acc[y][h] = (r < n && c < n) ? -get(r, c) : 0.0;
+                    }
+#pragma unroll
+                for (int y = 0; y < 2; ++y) {
+                    double bf[4];
+#pragma unroll
+                    for (int h = 0; h < 4; ++h) bf[h] = ((h >> 1) ? V : W)[(t + 4 * (h & 1)) * ns + c0 + 8 * y + g];
+                    dmma16(acc[y], af, bf);
+                }
+#pragma unroll
+                for (int y = 0; y < 2; ++y)
+#pragma unroll
+                    for (int h = 0; h < 4; ++h) {
+                        const int r = r0 + g + 8 * (h >> 1), c = c0 + 8 * y + 2 * t + (h & 1);
+                        if (r < n && c < n) ag[(size_t)c * n + r] = -acc[y][h];
+                    }
+            }
+            exchange();
+            acol = (row >= k && row < n) ? get(row, k) : 0.0;
         }
-        __syncthreads();
-        // (2) Householder vector from x = A[k+1:, k]
+        // ---- the column, and its norm below the subdiagonal
         double ss = 0.0;
-        for (int i = k + 2 + tid; i < n; i += blockDim.x) {
-            const double x = a[(size_t)k * n + i];
-            ss += x * x;
+        const bool live = row > k && row < n;
+        if (row >= k && row < n) {
+            double v = acol;
+            for (int t = 0; t < i; ++t) v -= V[t * ns + row] * W[t * ns + k] + W[t * ns + row] * V[t * ns + k];
+            x = v;
+            xs[row] = v;
+            if (row == k && rank == 0) d[k] = v;
+            if (row >= k + 2) ss = v * v;
         }
-        ss = block_sum(ss, red);
-        if (tid == 0) {
-            const double alpha = a[(size_t)k * n + k + 1];
-            d[k] = a[(size_t)k * n + k];
-            if (ss == 0.0) {
-                s_tau = 0.0;
-                s_beta = alpha;
-                s_scal = 0.0;
-            } else {
-                const double beta = -copysign(sqrt(alpha * alpha + ss), alpha);
-                s_tau = (beta - alpha) / beta;
-                s_beta = beta;
-                s_scal = 1.0 / (alpha - beta);
-            }
-            e[k] = s_beta;
-            tau[k] = s_tau;
-        }
+        ss = warp_sum(ss);
+        if (lane == 0) part[warp] = ss;
         __syncthreads();
-        const double tk = s_tau, scal = s_scal;
-        for (int i = tid; i < n; i += blockDim.x) {
-            double vi = 0.0;
-            if (i == k + 1) vi = 1.0;
-            else if (i > k + 1) {
-                vi = a[(size_t)k * n + i] * scal;
-                a[(size_t)k * n + i] = vi;  // reflector kept below the subdiagonal
-            }
-            v[i] = vi;
-        }
-        __syncthreads();
-        // (3) fused: apply pending update to A22 and accumulate s = A22 v. One row per thread,
-        // or per pair of adjacent threads (the two take alternate columns) when the block has
-        // threads to spare: twice the loads in flight per row. Four columns per iteration.
-        const int R = (blockDim.x >= 2u * (unsigned)n) ? 2 : 1;
-        const int i = k + 1 + tid / R, h = tid % R;
-        const bool act = i < n;
-        const double vpi = (pending && act) ? vp[i] : 0.0, wpi = (pending && act) ? wp[i] : 0.0;
-        double s_acc = 0.0;
-        if (act && (tk != 0.0 || pending)) {
-            const size_t sn = (size_t)R * n;  // stride between this thread's columns
-            int j = k + 1 + h;
-            for (; j + 3 * R < n; j += 4 * R) {
-                double *c0 = a + (size_t)j * n + i;
-                double x0 = c0[0], x1 = c0[sn], x2 = c0[2 * sn], x3 = c0[3 * sn];
-                if (pending) {
-                    x0 -= vpi * wp[j] + wpi * vp[j];
-                    x1 -= vpi * wp[j + R] + wpi * vp[j + R];
-                    x2 -= vpi * wp[j + 2 * R] + wpi * vp[j + 2 * R];
-                    x3 -= vpi * wp[j + 3 * R] + wpi * vp[j + 3 * R];
-                    c0[0] = x0;
-                    c0[sn] = x1;
-                    c0[2 * sn] = x2;
-                    c0[3 * sn] = x3;
+        // ---- A x (columns k+2..) in partial sums, and the panel's dot products with x
+        double *sp = sp0 + (k & 1) * kTriParts * ns;  // the other CTAs may still read the last column's
+        const int c0 = (k + 1) >> 5, nch = ((n - 1) >> 5) - c0 + 1;
+        const int sub_n = max(1, min(kTriParts / C, nw / nch));
+        const int sub = warp / nch;
+        const double a1 = live ? get(row, k + 1) : 0.0;
+        if (sub < sub_n) {
+            const int g = rank * sub_n + sub, G = C * sub_n;  // this warp's columns: k + 2 + g mod G
+            for (int ch = c0 + warp % nch; ch <= ((n - 1) >> 5); ch += (nch > nw) ? nw : nch) {
+                const int r = 32 * ch + lane;
+                const bool in = r > k && r < n;
+                const int rc = in ? r : n - 1;
+                double s0 = 0.0, s1 = 0.0, s2 = 0.0, s3 = 0.0;
+                int j = k + 2 + g;
+                const double *col = ag + (unsigned)(j * n + rc);
+                const unsigned st = (unsigned)(G * n);
+                for (; j + 7 * G < n; j += 8 * G, col += 8 * st) {
+                    double y[8];
+#pragma unroll
+                    for (int h = 0; h < 8; ++h) y[h] = __ldcg(col + h * st);
+#pragma unroll
+                    for (int h = 0; h < 8; h += 4) {
+                        s0 = fma(y[h], xs[j + h * G], s0);
+                        s1 = fma(y[h + 1], xs[j + (h + 1) * G], s1);
+                        s2 = fma(y[h + 2], xs[j + (h + 2) * G], s2);
+                        s3 = fma(y[h + 3], xs[j + (h + 3) * G], s3);
+                    }
                 }
-                s_acc += (x0 * v[j] + x1 * v[j + R]) + (x2 * v[j + 2 * R] + x3 * v[j + 3 * R]);
-            }
-            for (; j < n; j += R) {
-                double *cj = a + (size_t)j * n + i;
-                double x = *cj;
-                if (pending) {
-                    x -= vpi * wp[j] + wpi * vp[j];
-                    *cj = x;
+                if (j < n) {  // the last columns, loads first
+                    double y[7];
+#pragma unroll
+                    for (int h = 0; h < 7; ++h) y[h] = (j + h * G < n) ? __ldcg(col + h * st) : 0.0;
+#pragma unroll
+                    for (int h = 0; h < 7; ++h) s0 = fma(y[h], (j + h * G < n) ? xs[j + h * G] : 0.0, s0);
                 }
-                s_acc += x * v[j];
+                if (in) {
+                    const double s = (s0 + s1) + (s2 + s3);
+                    double *mine = sp + g * ns + r;
+                    *mine = s;
+                    if constexpr (C > 1) {
+#pragma unroll
+                        for (int q = 1; q < C; ++q) *cg::this_cluster().map_shared_rank(mine, (rank + q) % C) = s;
+                    }
+                }
             }
         }
-        if (R == 2) s_acc += __shfl_xor_sync(0xffffffffu, s_acc, 1);  // partner thread, same warp
-        // p = tau s ; w = p - (tau/2)(p.v) v
-        double pv = (act && h == 0) ? tk * s_acc * v[i] : 0.0;
-        pv = block_sum(pv, red);
-        const double alpha2 = -0.5 * tk * pv;
-        __syncthreads();
-        for (int q = tid; q < n; q += blockDim.x) {
-            vp[q] = v[q];
-            wp[q] = 0.0;
+        for (int t = warp; t < 2 * i; t += nw) {
+            const double *col = (t < i) ? V + t * ns : W + (t - i) * ns;
+            double s = 0.0;
+            for (int r = k + 2 + lane; r < n; r += 32) s = fma(col[r], xs[r], s);
+            s = warp_sum(s);
+            if (lane == 0) zs[t] = s;
         }
+        const double sig = warp_sum(part[lane]);
+        const double alpha = xs[k + 1];
+        double tk = 0.0, beta = alpha, sc = 0.0;
+        if (sig != 0.0) {
+            beta = -copysign(sqrt(alpha * alpha + sig), alpha);
+            sc = 1.0 / (alpha - beta);
+            tk = (beta - alpha) / beta;
+        }
+        exchange();
+        // ---- q = A v on the current matrix, p.v, w = tau q - (tau^2 / 2)(q.v) v
+        double qv = 0.0, v2 = 0.0;
+        if (live) {
+            double s = 0.0;
+            for (int q = 0; q < C * sub_n; ++q) s += sp[q * ns + row];
+            s = fma(sc, s, a1);
+            for (int t = 0; t < i; ++t)
+                s -= V[t * ns + row] * fma(sc, zs[i + t], W[t * ns + k + 1]) + W[t * ns + row] * fma(sc, zs[t], V[t * ns + k + 1]);
+            v2 = (row == k + 1) ? 1.0 : sc * x;
+            qv = s;
+        }
+        const double ps = warp_sum(qv * v2);
+        if (lane == 0) part2[warp] = ps;
         __syncthreads();
-        if (act && h == 0) wp[i] = tk * s_acc + alpha2 * v[i];
-        pending = (tk != 0.0);
+        const double al = -0.5 * tk * tk * warp_sum(part2[lane]);
+        if (live) {
+            V[i * ns + row] = v2;
+            W[i * ns + row] = fma(al, v2, tk * qv);
+            if (rank == 0 && row > k + 1) ag[(size_t)k * n + row] = v2;  // reflector kept below the subdiagonal
+        }
+        acol = a1;
+        if (tid == 0 && rank == 0) {
+            e[k] = beta;
+            tau[k] = tk;
+        }
         __syncthreads();
     }
-    // trailing 2x2 block
-    if (tid == 0) {
-        double a00 = a[(size_t)(n - 2) * n + (n - 2)];
-        double a10 = a[(size_t)(n - 2) * n + (n - 1)];
-        double a11 = a[(size_t)(n - 1) * n + (n - 1)];
-        if (pending) {
-            a00 -= 2.0 * vp[n - 2] * wp[n - 2];
-            a10 -= vp[n - 1] * wp[n - 2] + wp[n - 1] * vp[n - 2];
-            a11 -= 2.0 * vp[n - 1] * wp[n - 1];
+    // trailing 2 x 2 block: the last panel's columns are still pending
+    if (tid == 0 && rank == 0) {
+        const int cnt = (n > 2) ? (n - 3) % kTriNb + 1 : 0;
+        auto cur = [&](int r, int c) {
+            double v = get(r, c);
+            for (int t = 0; t < cnt; ++t) v -= V[t * ns + r] * W[t * ns + c] + W[t * ns + r] * V[t * ns + c];
+            return v;
+        };
+        if (n >= 2) {
+            d[n - 2] = cur(n - 2, n - 2);
+            e[n - 2] = cur(n - 1, n - 2);
+            tau[n - 2] = 0.0;
         }
-        d[n - 2] = a00;
-        d[n - 1] = a11;
-        e[n - 2] = a10;
+        d[n - 1] = cur(n - 1, n - 1);
         e[n - 1] = 0.0;
-        tau[n - 2] = 0.0;
+        tau[n - 1] = 0.0;
+    }
+    if constexpr (C > 1) cg::this_cluster().sync();
+}
+
+// Blocks that fit in shared memory: unblocked, the rank-2 update of the previous column fused with
+// the product A x in one pass over shared memory. The same short chain a column: products with x
+// beside its norm, three reductions, four barriers. One block of order 144: 0.64 -> 0.34 ms (the
+// kernel above takes 0.59), 3200 of order 40: 0.31 -> 0.23, 500 of order 64: 0.20 -> 0.16 ms. The
+// panel scheme loses here, its dot products cost more than the writes they save; at order 153 the
+// block no longer fits beside its vectors.
+__global__ void __launch_bounds__(512) tridiag_small_kernel(BatchDesc bd, double *A, double *dg, double *eo,
+                                                            double *tauo) {
+    const int b = blockIdx.x;
+    const int n = bd.n[b];
+    double *ag = A + bd.aoff[b];
+    double *d = dg + bd.voff[b], *e = eo + bd.voff[b], *tau = tauo + bd.voff[b];
+    extern __shared__ __align__(16) double sm[];
+    double2 *xv = reinterpret_cast<double2 *>(sm);  // the column x; the previous reflector v
+    double *ws = sm + 2 * n, *sp = ws + n, *as = sp + kTriParts * n;
+    __shared__ double part[16], part2[16], s_alpha;
+    const int T = blockDim.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = T >> 5, row = tid;
+    for (int q = tid; q < n * n; q += T) as[q] = ag[q];
+    for (int q = tid; q < n; q += T) {
+        xv[q] = make_double2(0.0, 0.0);
+        ws[q] = 0.0;
+    }
+    if (tid < 16) part[tid] = part2[tid] = 0.0;
+    __syncthreads();
+    double acol = (row < n) ? as[row] : 0.0, vp = 0.0, wp = 0.0;
+    for (int k = 0; k + 2 < n; ++k) {
+        const bool live = row > k && row < n;
+        double x = 0.0, ss = 0.0;
+        if (row >= k && row < n) {
+            x = acol - (vp * ws[k] + wp * xv[k].y);
+            if (row == k) d[k] = x;
+            else if (row == k + 1) s_alpha = x;
+            else ss = x * x;
+            xv[row].x = (row >= k + 2) ? x : 0.0;
+        }
+        ss = warp_sum(ss);
+        if (lane == 0) part[warp] = ss;
+        __syncthreads();
+        const int c0 = (k + 1) >> 5, nch = ((n - 1) >> 5) - c0 + 1;
+        const int sub_n = max(1, min(kTriParts, nw / nch)), sub = warp / nch;
+        if (sub < sub_n) {
+            const int r = 32 * (c0 + warp % nch) + lane;
+            if (r > k && r < n) {
+                const double vr = xv[r].y, wr = ws[r];
+                double s0 = 0.0, s1 = 0.0;
+                int j = k + 1 + sub;
+                double *col = as + (size_t)j * n + r;
+                const int st = sub_n * n;
+                for (; j + 3 * sub_n < n; j += 4 * sub_n, col += 4 * st) {
+                    double a0 = col[0], a1 = col[st], a2 = col[2 * st], a3 = col[3 * st];
+                    const double2 q0 = xv[j], q1 = xv[j + sub_n], q2 = xv[j + 2 * sub_n], q3 = xv[j + 3 * sub_n];
+                    a0 -= vr * ws[j] + wr * q0.y;
+                    a1 -= vr * ws[j + sub_n] + wr * q1.y;
+                    a2 -= vr * ws[j + 2 * sub_n] + wr * q2.y;
+                    a3 -= vr * ws[j + 3 * sub_n] + wr * q3.y;
+                    col[0] = a0;
+                    col[st] = a1;
+                    col[2 * st] = a2;
+                    col[3 * st] = a3;
+                    s0 = fma(a0, q0.x, fma(a1, q1.x, s0));
+                    s1 = fma(a2, q2.x, fma(a3, q3.x, s1));
+                }
+                for (; j < n; j += sub_n, col += st) {
+                    const double2 q0 = xv[j];
+                    const double a0 = col[0] - (vr * ws[j] + wr * q0.y);
+                    col[0] = a0;
+                    s0 = fma(a0, q0.x, s0);
+                }
+                sp[sub * n + r] = s0 + s1;
+            }
+        }
+        const double sig = warp_sum(lane < 16 ? part[lane] : 0.0);
+        const double alpha = s_alpha;
+        double tk = 0.0, beta = alpha, sc = 0.0;
+        if (sig != 0.0) {
+            beta = -copysign(sqrt(alpha * alpha + sig), alpha);
+            sc = 1.0 / (alpha - beta);
+            tk = (beta - alpha) / beta;
+        }
+        __syncthreads();
+        double qv = 0.0, v2 = 0.0;
+        if (live) {
+            acol = as[(size_t)(k + 1) * n + row];
+            double s = 0.0;
+            for (int q = 0; q < sub_n; ++q) s += sp[q * n + row];
+            qv = fma(sc, s, acol);
+            v2 = (row == k + 1) ? 1.0 : sc * x;
+        }
+        const double ps = warp_sum(qv * v2);
+        if (lane == 0) part2[warp] = ps;
+        __syncthreads();
+        const double al = -0.5 * tk * tk * warp_sum(lane < 16 ? part2[lane] : 0.0);
+        vp = v2;
+        wp = fma(al, v2, tk * qv);
+        if (live) {
+            xv[row].y = vp;
+            ws[row] = wp;
+            if (row > k + 1) ag[(size_t)k * n + row] = v2;  // reflector kept below the subdiagonal
+        }
+        if (tid == 0) {
+            e[k] = beta;
+            tau[k] = tk;
+        }
+        __syncthreads();
+    }
+    if (tid == 0) {  // trailing 2 x 2 block: the last column is still pending
+        auto cur = [&](int r, int c) { return as[(size_t)c * n + r] - (xv[r].y * ws[c] + ws[r] * xv[c].y); };
+        if (n >= 2) {
+            d[n - 2] = cur(n - 2, n - 2);
+            e[n - 2] = cur(n - 1, n - 2);
+            tau[n - 2] = 0.0;
+        }
+        d[n - 1] = cur(n - 1, n - 1);
+        e[n - 1] = 0.0;
         tau[n - 1] = 0.0;
     }
 }
@@ -682,17 +858,6 @@ void launch_symmetrize_lower(const BatchDesc &bd, double *A, int nmax, cudaStrea
     symmetrize_lower_kernel<<<grid, 256, 0, st>>>(bd, A);
 }
 
-void launch_tridiag_batched(const BatchDesc &bd, double *A, double *d, double *e, double *tau,
-                            int nmax, cudaStream_t st) {
-    if (bd.nblk <= 0) return;
-    const size_t smem = (size_t)3 * nmax * sizeof(double);
-    DVR3D_COUNT_LAUNCH(1);
-    // two threads per row while 2 nmax fits in one block (see the fused loop)
-    const int rows_thr = (2 * nmax <= kTriMaxThreads) ? 2 * nmax : nmax;
-    const int threads = std::min(kTriMaxThreads, std::max(64, (rows_thr + 31) / 32 * 32));
-    tridiag_kernel<<<bd.nblk, threads, smem, st>>>(bd, A, d, e, tau);
-}
-
 namespace {
 int sm_count() {
     int dev = 0, nsm = 0;
@@ -701,6 +866,58 @@ int sm_count() {
     return std::max(nsm, 1);
 }
 }  // namespace
+
+namespace {
+template <int C>
+void launch_tridiag(const BatchDesc &bd, double *A, double *d, double *e, double *tau, int nmax, cudaStream_t st) {
+    const int ns = (nmax + 32) / 8 * 8;  // the update's tiles run past the end
+    const size_t smem = (size_t)(2 * kTriNb + 1 + 2 * kTriParts) * ns * sizeof(double);
+    int dev = 0;
+    cudaGetDevice(&dev);
+    static bool attr[kMaxAttrDevices] = {};
+    if (dev < 0 || dev >= kMaxAttrDevices || !attr[dev]) {
+        cudaFuncSetAttribute(tridiag_kernel<C>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
+        if (dev >= 0 && dev < kMaxAttrDevices) attr[dev] = true;
+    }
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(bd.nblk * C);
+    cfg.blockDim = dim3(1024);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = C;
+    at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, tridiag_kernel<C>, bd, A, d, e, tau, ns);
+}
+}  // namespace
+
+void launch_tridiag_batched(const BatchDesc &bd, double *A, double *d, double *e, double *tau,
+                            int nmax, cudaStream_t st) {
+    if (bd.nblk <= 0) return;
+    DVR3D_COUNT_LAUNCH(1);
+    if (nmax <= kTriSmem) {
+        int dev = 0;
+        cudaGetDevice(&dev);
+        static bool attr[kMaxAttrDevices] = {};
+        if (dev < 0 || dev >= kMaxAttrDevices || !attr[dev]) {
+            cudaFuncSetAttribute(tridiag_small_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
+            if (dev >= 0 && dev < kMaxAttrDevices) attr[dev] = true;
+        }
+        // three column subsets a row chunk while the blocks are few
+        const int rows = (nmax + 31) / 32;
+        const int warps = std::max(2, std::min(16, bd.nblk > 4 * sm_count() ? rows : 3 * rows));
+        const size_t smem = ((size_t)nmax * nmax + (3 + kTriParts) * (size_t)nmax) * sizeof(double);
+        tridiag_small_kernel<<<bd.nblk, 32 * warps, smem, st>>>(bd, A, d, e, tau);
+    } else if (2 * bd.nblk <= sm_count()) {  // two CTAs a block while they find an SM each
+        launch_tridiag<2>(bd, A, d, e, tau, nmax, st);
+    } else {
+        launch_tridiag<1>(bd, A, d, e, tau, nmax, st);
+    }
+}
 
 void launch_eigvals_batched(const BatchDesc &bd, const double *d, const double *e, double *w,
                             int *cnt, int mode, double cut, cudaStream_t st) {
