@@ -16,12 +16,13 @@
 //                    D_s and from the right to O_{s+1}; the remainder of the bulge is
 //                    eliminated by later sweeps.
 // One CTA owns a whole sweep, keeping O_{s+1} between its tasks. Sweep j+1 may start task s once
-// sweep j has written the beta of its task s + 2 (the only entry the two share), published
-// through per-sweep progress counters with release / acquire ordering and bounded waits.
+// sweep j has formed the beta of its task s + 2 (the only entry the two share).
 // Back-transformation: Q = prod over sweeps (in order) of prod over tasks of H; the
 // reflectors of one sweep act on disjoint rows, so a CTA holding a slab of eigenvector
 // columns in shared memory applies sweep after sweep (last first), its warps taking the
 // tasks of a sweep in parallel.
+#include <cooperative_groups.h>
+
 #include <algorithm>
 
 #include "band_eig.cuh"
@@ -34,6 +35,7 @@ namespace {
 constexpr int kBW = kBandMaxBw;
 constexpr int kTS = kBW + 1;            // shared-memory row stride of a block
 constexpr int kBlk = kBW * kTS;         // doubles of one 32 x 32 block in shared memory
+constexpr int kSlotDoubles = 2 * kBlk + 2;  // doubles of a slot of the chase
 constexpr unsigned long long kSpinLimit = 1ull << 24;
 constexpr unsigned kFull = 0xffffffffu;
 
@@ -88,170 +90,335 @@ __device__ __forceinline__ void house_scalars(double alpha, double sig, double &
     }
 }
 
-// One CTA per sweep in flight. The band lives in compact storage (kBandLd doubles a column, both
-// triangles within b of the diagonal, bulge space below): element (i, j) at C[j (kBandLd - 1) + i +
-// kBW], so a column window is contiguous, nothing is clamped at the matrix end (zero padding) and
-// the whole band stays in L2.
-// The chase is a dependency chain, so everything is arranged around its length. Task s needs the
-// column x that task s - 1 leaves in the bulge; all matrix-vector products of the task are formed
-// with x itself (O x, D x, O^T x) beside the norm of x, and the reflector's three scalars are
-// computed by every warp for itself, so one barrier (X) a task is all that stands between x and
-// the next x. 18 warps:
-//   L D (4)  wait for the previous sweep's flag, load task s+1's D and O into registers, then into
-//            the raw buffer that task s-1 has left (barrier E);
-//   O (4)    O_{s+1} <- O_{s+1} H: eight rows a warp, four lanes a row; the first column is the
-//            next x, written first with its partial norms; the whole block goes to shared memory;
-//   D (4)    D_s <- H D_s H, kept as a full symmetric block, to global memory;
-//   L (4)    O_s <- H O_s (the bulge), to global memory, its first row mirrored above the diagonal;
-//   P1       the reflector for the back-transformation, beta;
-//   P2       publishes: flag f = reflector f-1 known (beta written) and tasks < f-1 complete
-//            (counters in shared memory), the release off the chain.
-// Sweep j+1 runs task s once sweep j's flag reaches s + 3: its blocks were completed by task s+1
-// and the one entry that task s+2 changes is its beta. Sweeps follow one another at
-// (task time) + (flag, fence and load latency): 2656 columns of half-bandwidth 32 (the projected
-// matrix of 500 levels) take 17.7 ms, against 27.8 ms for five warps with the reflector broadcast
-// through a second barrier and the blocks at the matrix's own stride; 12202 columns 119 ms. Of a
-// task's 3400 cycles the D warps need 3000; fence, flag and loads take 1000 + 1900 + 1500.
-constexpr int kChaseThreads = 18 * 32;
-constexpr int kBarX = 1, kBarE = 3, kBarD = 5;
+// One CTA per sweep in flight, sixteen consecutive sweeps a thread-block cluster. The chase is a
+// dependency chain: task s of sweep j+1 needs what tasks s, s+1 of sweep j leave and the beta of its
+// task s+2, so sweeps follow one another at about two task times plus one hand-off, and everything is
+// arranged around these. A sweep's results are put together in slots, one a task, already shifted to
+// the next sweep's window: D(r,c) = D_s(r+1,c+1), its last row and column the first row of O_{s+1}
+// and D_{s+1}(0,0); O(r,c) = O_{s+1}(r+1,c+1), its last column D_{s+1}(r+1,0) and, apart from the
+// block, the beta of task s+2. A slot is complete, and leaves, when task s+2 begins; parts that a
+// sweep's last tasks do not have are zeros. Inside a cluster it goes to the next CTA's ring of slots
+// in one bulk copy that an mbarrier counts (no flag, no trip through L2), with credits for the slots
+// coming back. The last CTA of a cluster copies its slots to global memory behind a flag, where the
+// first CTA of the next one fetches them; one buffer serves all, since a slot is written only after
+// every earlier sweep has used it. The band itself enters as the slots of sweep 0.
+// A task needs the column x that the task before left in the bulge; all its products are formed with
+// x itself (O x, D x, O^T x) while one warp forms the reflector's scalars from its norm, so the
+// barriers X (x is known) and Y (the scalars are) are all that a task waits for. 16 warps:
+//   LD (1)   first CTA: waits for the flag, fetches slots into the ring; others: returns the ring's
+//            credits;
+//   ST (1)   sends the slots (fences and remote arrivals take longer than the scalars);
+//   P1 (1)   the scalars; the betas; e, the reflector for the back-transformation;
+//   O (4)    O_{s+1} <- O_{s+1} H: eight rows a warp, four lanes a row; the first column is the next
+//            x, written first with its partial norms; the whole block goes to shared memory;
+//   D (4)    D_s <- H D_s H, kept as a full symmetric block;
+//   L (4)    O_s <- H O_s (the bulge).
+// Half-bandwidth 32: 2656 columns (the projected matrix of 500 levels) 27.8 -> 9.7 ms, 913 columns 3.2
+// ms, 12202 columns 119 (before slots, every sweep through L2) -> 49 ms. A task takes 1.15 us, of it
+// 0.32 the scalars and 0.6 the D warps' chain through shared memory; sweeps follow at 3.5 us, 6.6
+// across clusters. Seven clusters of sixteen fit a B200 (fifteen of eight: 50 ms, more hand-offs
+// through L2).
+constexpr int kChaseThreads = 16 * 32;
+constexpr int kChaseCluster = 16;
+constexpr int kRing = 5;
+constexpr int kBarX = 1, kBarD = 3, kBarY = 4;  // kBarY + role: the scalars reach each group by itself
 
 __device__ __forceinline__ void bar_sync(int id, int count) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(count) : "memory"); }
 __device__ __forceinline__ void bar_arrive(int id, int count) { asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(count) : "memory"); }
+__device__ __forceinline__ unsigned smem_u32(const void *p) { return (unsigned)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ unsigned map_rank(unsigned addr, unsigned rank) {
+    unsigned r;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+    return r;
+}
+__device__ __forceinline__ void mbar_init(unsigned bar, unsigned count) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
+}
+__device__ __forceinline__ bool mbar_test(unsigned bar, unsigned parity) {
+    unsigned ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tmbarrier.test_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(bar), "r"(parity)
+        : "memory");
+    return ok != 0;
+}
+__device__ __forceinline__ void mbar_arrive(unsigned bar) {  // this CTA's barrier
+    asm volatile("mbarrier.arrive.release.cta.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+__device__ __forceinline__ void mbar_arrive_remote(unsigned bar) {
+    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+__device__ __forceinline__ void mbar_expect(unsigned bar, unsigned bytes) {
+    asm volatile("mbarrier.arrive.expect_tx.release.cta.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void st_async(unsigned addr, double v, unsigned bar) {
+    asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.b64 [%0], %1, [%2];" ::"r"(addr),
+                 "l"(__double_as_longlong(v)), "r"(bar)
+                 : "memory");
+}
+// Bulk copies of `bytes` (a multiple of 16): to another CTA's shared memory, from and to global memory.
+__device__ __forceinline__ void bulk_to_cta(unsigned dst, unsigned src, unsigned bytes, unsigned bar) {
+    asm volatile("cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst), "r"(src),
+                 "r"(bytes), "r"(bar)
+                 : "memory");
+}
+__device__ __forceinline__ void bulk_load(unsigned dst, const void *src, unsigned bytes, unsigned bar) {
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst), "l"(src),
+                 "r"(bytes), "r"(bar)
+                 : "memory");
+}
+__device__ __forceinline__ void bulk_store_wait(void *dst, unsigned src, unsigned bytes) {
+    asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(dst), "r"(src), "r"(bytes) : "memory");
+    asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+    asm volatile("cp.async.bulk.wait_group 0;\n\tfence.proxy.async;" ::: "memory");
+}
+__device__ __forceinline__ void fence_async() { asm volatile("fence.proxy.async;" ::: "memory"); }
 
-struct ChaseSmem {
-    double raw[2][2][kBlk];  // [buffer][D, O_{s+1}] as loaded
-    double bulge[2][kBlk];   // O_s after the right-hand update
-    double x[2][kBW];        // the task's column
-    double part[2][4];       // its sum of squares without x_0, eight rows each
-    double ya[kBW], p2[4];   // D x and x^T D x (without x_0)
-    volatile int done[8];    // tasks completed by each of the D and L warps
-    volatile int refl;       // reflectors known
+__device__ __forceinline__ void load8(double (&v)[8], const double *p) {  // 16-byte aligned
+#pragma unroll
+    for (int k = 0; k < 8; k += 2) {
+        const double2 q = *reinterpret_cast<const double2 *>(p + k);
+        v[k] = q.x;
+        v[k + 1] = q.y;
+    }
+}
+
+struct alignas(16) ChaseSlot {
+    double d[kBlk], o[kBlk];  // [column][row]
+    double beta, pad;         // last element of o
+};
+static_assert(sizeof(ChaseSlot) == kSlotDoubles * sizeof(double) && sizeof(ChaseSlot) % 16 == 0, "slots are copied in bulk");
+
+struct alignas(128) ChaseSmem {
+    ChaseSlot raw[kRing];      // the sweep's input
+    ChaseSlot stage[kRing];    // the next sweep's, until they are complete
+    double bulge[2][kBlk];     // O_s after the right-hand update, [column][row]
+    alignas(16) double x[2][kBW];  // the task's column
+    double xin[kBW];           // the sweep's first column
+    double xout[kBW];          // the next sweep's
+    double part[2][4];         // the column's sum of squares without x_0, eight rows each
+    double scal[2][4];         // the reflector: tau, beta, sc
+    alignas(16) double ya[kBW];
+    double p2[4];              // D x and x^T D x (without x_0)
+    unsigned long long full[kRing], fullx;  // slots of the ring and xin filled
+    unsigned long long own[kRing];          // first CTA: slots of its ring free again
+    unsigned long long credit[kRing];       // staged slots free again, here and at the next CTA
+    volatile int tasks, refl;               // tasks begun; reflectors known, their betas staged
     volatile int abort;
 };
 
 __global__ void __launch_bounds__(kChaseThreads, 1) band_chase_kernel(BandTri t) {
-    extern __shared__ __align__(16) unsigned char chase_sm[];
+    extern __shared__ __align__(128) unsigned char chase_sm[];
     ChaseSmem &S = *reinterpret_cast<ChaseSmem *>(chase_sm);
+    namespace cg = cooperative_groups;
+    cg::cluster_group cluster = cg::this_cluster();
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, role = warp >> 2, w = warp & 3;
     const int n = t.n, b = t.b;
-    constexpr long long ld = kBandLd - 1;
-    constexpr int nX = 17 * 32, nE = 12 * 32;  // X: all but P2; E: O, D and the loaders
-    const unsigned long long spin_limit = t.wait_limit ? t.wait_limit : kSpinLimit;
-    double *A = t.C + kBW;
-    if (tid == 0) S.abort = 0;
-    int q = 0;  // tasks of this CTA so far: the parity of buffers and barriers
-    for (int j = blockIdx.x; j <= n - 3; j += gridDim.x) {
+    const int K = (int)cluster.num_blocks(), rank = (int)cluster.block_rank();
+    const bool first = rank == 0, last = rank == K - 1;
+    constexpr int nX = 13 * 32;  // O, D, L and P1
+    constexpr unsigned slot_bytes = sizeof(ChaseSlot), block_bytes = 2 * kBlk * 8;
+    const unsigned x_bytes = 8u * (unsigned)b;
+    const unsigned long long flag_limit = t.wait_limit ? t.wait_limit : kSpinLimit;
+    const unsigned long long smem_limit = t.wait_limit ? t.wait_limit : 4 * kSpinLimit;
+    ChaseSlot *G = reinterpret_cast<ChaseSlot *>(t.slots);  // [0]: first column, [1 + s]: slot s
+    for (int q = tid; q < (int)(2 * kRing * sizeof(ChaseSlot) / 8); q += kChaseThreads) reinterpret_cast<double *>(S.raw)[q] = 0.0;
+    if (tid < kBW) S.xin[tid] = S.xout[tid] = 0.0;
+    if (tid == 0) {
+        S.abort = 0;
+        for (int q = 0; q < kRing; ++q) {
+            mbar_init(smem_u32(&S.full[q]), 1);
+            mbar_init(smem_u32(&S.own[q]), 1);
+            mbar_init(smem_u32(&S.credit[q]), 1);
+        }
+        mbar_init(smem_u32(&S.fullx), 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        if (!first) {
+            for (int q = 0; q < kRing; ++q) mbar_expect(smem_u32(&S.full[q]), block_bytes + 8);
+            mbar_expect(smem_u32(&S.fullx), x_bytes);
+        }
+    }
+    cluster.sync();
+    // bounded wait for a phase of one of this CTA's barriers; when it runs out the CTA runs on
+    // without waits to the end of its sweep, and leaves
+    auto wait = [&](unsigned long long *bar, unsigned parity) {
+        const unsigned a = smem_u32(bar);
+        unsigned long long spins = 0;
+        while (!mbar_test(a, parity)) {
+            if (S.abort) return;
+            ++spins;
+            if ((spins & 1023ull) == 0 && *(volatile int *)t.err != 0) S.abort = 1;
+            if (spins > smem_limit) {
+                atomicExch(t.err, (int)kDevBarrierTimeout);
+                S.abort = 1;
+            }
+        }
+    };
+    // the same address in the next and the previous CTA of the cluster
+    const unsigned noff = map_rank(smem_u32(&S), (unsigned)(last ? rank : rank + 1)) - smem_u32(&S);
+    const unsigned poff = map_rank(smem_u32(&S), (unsigned)(first ? rank : rank - 1)) - smem_u32(&S);
+    auto rem = [&](const void *p) { return smem_u32(p) + noff; };
+    int q = 0;       // tasks of this CTA so far: the parity of buffers and barriers
+    int in0 = 0;     // slots of this CTA's ring consumed by earlier sweeps
+    int out0 = 0;    // slots sent by earlier sweeps
+    int sweeps = 0;  // sweeps so far
+    for (int j = (int)(blockIdx.x / K) * K + rank; j <= n - 3; j += gridDim.x, ++sweeps) {
         const int nt = band_ntask(n, b, j);
         const int ntp = (j > 0) ? band_ntask(n, b, j - 1) : 0;
-        if (tid < 8) S.done[tid] = 0;
-        if (tid == 8) S.refl = 0;
+        const bool send = j + 1 <= n - 3, near = send && !last, far = send && last;  // next CTA; global memory
+        if (tid == 0) S.refl = S.tasks = 0;
         __syncthreads();
-        if (S.abort) return;
-        if (role == 0) {
-            // ---- loaders: columns 8w .. 8w+7, lane = row
-            unsigned seen = (j > 0) ? 0u : 0xffffffffu;
-            for (int s = 0; s < nt; ++s) {
-                const int pb = (q + s) & 1;
-                const unsigned need = (unsigned)min(s + 3, ntp + 1);
-                if (seen < need && !S.abort) {
-                    unsigned f = 0;
-                    int ok = 1;
-                    if (lane == 0) {
-                        unsigned long long spins = 0;
-                        while ((f = ld_acquire_u32(t.progress + j - 1)) < need) {
-                            if (++spins > spin_limit) {
-                                atomicExch(t.err, (int)kDevBarrierTimeout);
-                                ok = 0;
-                                break;
-                            }
-                            if ((spins & 255ull) == 0 && *(volatile int *)t.err != 0) {
-                                ok = 0;
-                                break;
-                            }
-                        }
-                        if (!ok) S.abort = 1;  // this sweep runs on without waits; all leave at its end
-                    }
-                    seen = __shfl_sync(kFull, f, 0);
-                }
-                __syncwarp();
-                const int r0 = j + 1 + s * b, L = min(b, n - r0), r1 = r0 + b, L1 = min(b, n - r1);
-                double dv[8], ov[8], xv = 0.0;
-#pragma unroll
-                for (int k = 0; k < 8; ++k) {
-                    const int c = 8 * w + k;
-                    const double *col = A + (long long)(r0 + c) * ld;
-                    dv[k] = (c < L && lane < L) ? __ldcg(col + r0 + lane) : 0.0;
-                    ov[k] = (c < L && lane < L1) ? __ldcg(col + r1 + lane) : 0.0;
-                }
-                if (s == 0 && lane < 8 && 8 * w + lane < L) xv = __ldcg(A + (long long)j * ld + r0 + 8 * w + lane);
-                if (q + s >= 2) bar_sync(kBarE + pb, nE);
-                double *D = S.raw[pb][0], *O = S.raw[pb][1];
-#pragma unroll
-                for (int k = 0; k < 8; ++k) {
-                    D[lane * kTS + 8 * w + k] = dv[k];
-                    O[lane * kTS + 8 * w + k] = ov[k];
-                }
-                if (s == 0) {
-                    if (lane < 8) S.x[pb][8 * w + lane] = xv;
-                    double sq = (w == 0 && lane == 0) ? 0.0 : xv * xv;
-                    sq += __shfl_xor_sync(kFull, sq, 4);
-                    sq += __shfl_xor_sync(kFull, sq, 2);
-                    sq += __shfl_xor_sync(kFull, sq, 1);
-                    if (lane == 0) S.part[pb][w] = sq;
-                }
-                bar_arrive(kBarX + pb, nX);
+        const int gave_up = S.abort;
+        __syncthreads();
+        if (gave_up) break;
+        // last CTA: slot s to global memory (s < 0: the first column), then its flag and credit
+        auto copy_out = [&](int s) {
+            if (s < 0) {
+                for (int c = 0; c < b; ++c) G->d[c] = S.xout[c];
+            } else {
+                const int u = (out0 + s) % kRing;
+                fence_async();
+                bulk_store_wait(G + 1 + s, smem_u32(&S.stage[u]), slot_bytes);
+                mbar_arrive(smem_u32(&S.credit[u]));
             }
-        } else if (warp < 17) {
-            const int rr = lane & 7, cg = lane >> 3, r = 8 * w + rr;
+            st_release_u32(t.progress + j, (unsigned)(s + 2));
+        };
+        auto give_back = [&](int m) {
+            const int u = m % kRing;
+            mbar_expect(smem_u32(&S.full[u]), block_bytes + 8);
+            mbar_arrive_remote(smem_u32(&S.credit[u]) + poff);
+        };
+        if (role == 0 && w == 0) {
+            if (first && lane == 0) {
+                // ---- LD
+                unsigned seen = (j > 0) ? 0u : 0xffffffffu;
+                for (int s = -1; s < nt; ++s) {
+                    unsigned long long spins = 0;
+                    while (seen < (unsigned)(s + 2) && !S.abort) {
+                        seen = ld_acquire_u32(t.progress + j - 1);
+                        if (++spins > flag_limit) {
+                            atomicExch(t.err, (int)kDevBarrierTimeout);
+                            S.abort = 1;
+                        }
+                        if ((spins & 255ull) == 0 && *(volatile int *)t.err != 0) S.abort = 1;
+                    }
+                    if (s < 0) {
+                        for (int c = 0; c < b; ++c) S.xin[c] = __ldcg(&G->d[c]);
+                        mbar_arrive(smem_u32(&S.fullx));
+                    } else {
+                        const int m = in0 + s, sl = m % kRing;
+                        wait(&S.own[sl], ((m / kRing) & 1) ^ 1);
+                        if (!S.abort) {
+                            mbar_expect(smem_u32(&S.full[sl]), slot_bytes);
+                            fence_async();
+                            bulk_load(smem_u32(&S.raw[sl]), G + 1 + s, slot_bytes, smem_u32(&S.full[sl]));
+                        }
+                    }
+                }
+            } else if (!first && lane == 0) {
+                // credits: slot s is read when task s + 1 begins, or the sweep ends; one more slot
+                // where the sweep before had one task more
+                for (int s = -1; s + 1 < nt && !S.abort; ++s) {
+                    while (S.tasks < s + 2 && !S.abort) {}
+                    if (S.abort) break;
+                    if (s < 0) mbar_expect(smem_u32(&S.fullx), x_bytes);  // the first column, for the next sweep
+                    else give_back(in0 + s);
+                }
+            }
+        } else if (role == 0 && w == 1) {
+            if (near && lane == 0) {
+                // ---- ST: slot s is complete when task s + 2 begins (its beta goes by itself)
+                for (int s = 0; s + 2 < nt && !S.abort; ++s) {
+                    while (S.tasks < s + 3 && !S.abort) {}
+                    if (S.abort) break;
+                    const int u = (out0 + s) % kRing;
+                    fence_async();
+                    bulk_to_cta(rem(&S.raw[u]), smem_u32(&S.stage[u]), block_bytes, rem(&S.full[u]));
+                }
+            } else if (far && lane == 0) {
+                // the first column is known with task 1's beta, slot s with task s + 2's
+                for (int s = -1; s + 2 < nt && !S.abort; ++s) {
+                    while (S.refl < s + 3 && !S.abort) {}
+                    __threadfence_block();
+                    if (!S.abort) copy_out(s);
+                }
+            }
+        } else if (role > 0 || w == 2) {
+            const int rr = lane & 7, cg8 = lane >> 3, r = 8 * w + rr;
+            // D: where this thread's elements go in a slot, and which of its columns do
+            const int off = (8 * cg8 - 1) * kTS + r - 1, ecol = (b - 1) * kTS + (r == 0 ? b - 1 : kBlk + r - 1);
+            unsigned cols = 0;
+#pragma unroll
+            for (int k = 0; k < 8; ++k)
+                if (r >= 1 && r < b && 8 * cg8 + k >= 1 && 8 * cg8 + k < b) cols |= 1u << k;
+            if (role == 1) {  // the first column
+                wait(&S.fullx, sweeps & 1);
+                double xv = (cg8 == 0) ? S.xin[r] : 0.0;
+                if (cg8 == 0) S.x[q & 1][r] = xv;
+                double sq = (r == 0) ? 0.0 : xv * xv;
+                sq += __shfl_xor_sync(kFull, sq, 4);
+                sq += __shfl_xor_sync(kFull, sq, 2);
+                sq += __shfl_xor_sync(kFull, sq, 1);
+                if (lane == 0) S.part[q & 1][w] = sq;
+            }
             for (int s = 0; s < nt; ++s) {
-                const int pb = (q + s) & 1;
-                const int r0 = j + 1 + s * b, L = min(b, n - r0);
+                const int pb = (q + s) & 1, m = in0 + s, sl = m % kRing;
+                // this task's staged slot and the two before it
+                const int o = out0 + s, so = o % kRing, so1 = (o + kRing - 1) % kRing, so2 = (o + kRing - 2) % kRing;
+                const bool end = s + 1 == nt, snd = send && !S.abort;
                 bar_sync(kBarX + pb, nX);
                 const double *x = S.x[pb];
-                const double alpha = x[0], sig = (S.part[pb][0] + S.part[pb][1]) + (S.part[pb][2] + S.part[pb][3]);
                 if (role == 1) {
                     // ---- O_{s+1} <- O_{s+1} H
-                    const double *R = S.raw[pb][1] + r * kTS;
-                    double o[8], xc[8], a0 = 0.0, a1 = 0.0;
+                    double xc[8];
+                    load8(xc, x + 8 * cg8);
+                    if (cg8 == 0) xc[0] = 0.0;
+                    wait(&S.full[sl], (m / kRing) & 1);
+                    const double *R = S.raw[sl].o + r;
+                    double o8[8], a0 = 0.0, a1 = 0.0;
                     const double o0 = R[0];
 #pragma unroll
-                    for (int k = 0; k < 8; ++k) {
-                        o[k] = R[8 * cg + k];
-                        xc[k] = (k == 0 && cg == 0) ? 0.0 : x[8 * cg + k];
+                    for (int k = 0; k < 8; ++k) o8[k] = R[(8 * cg8 + k) * kTS];
+                    if (r == b - 1 && cg8 == (b - 1) / 8) {
+                        const double bt = S.raw[sl].beta;
+#pragma unroll
+                        for (int k = 0; k < 8; ++k)
+                            if (k == (b - 1) % 8) o8[k] = bt;
                     }
 #pragma unroll
                     for (int k = 0; k < 8; k += 2) {
-                        a0 = fma(o[k], xc[k], a0);
-                        a1 = fma(o[k + 1], xc[k + 1], a1);
+                        a0 = fma(o8[k], xc[k], a0);
+                        a1 = fma(o8[k + 1], xc[k + 1], a1);
                     }
                     double a = a0 + a1;
                     a += __shfl_xor_sync(kFull, a, 8);
                     a += __shfl_xor_sync(kFull, a, 16);
-                    double tau, beta, sc;
-                    house_scalars(alpha, sig, tau, beta, sc);
+                    bar_sync(kBarY + role, 5 * 32);
+                    const double tau = S.scal[pb][0], sc = S.scal[pb][2];
                     const double tu = tau * fma(sc, a, o0);
                     const double xn = o0 - tu;
-                    if (cg == 0) S.x[pb ^ 1][r] = xn;
+                    if (cg8 == 0) S.x[pb ^ 1][r] = xn;
                     double sq = (r == 0) ? 0.0 : xn * xn;
                     sq += __shfl_xor_sync(kFull, sq, 4);
                     sq += __shfl_xor_sync(kFull, sq, 2);
                     sq += __shfl_xor_sync(kFull, sq, 1);
                     if (lane == 0) S.part[pb ^ 1][w] = sq;
-                    double *B = S.bulge[pb ^ 1] + r * kTS + 8 * cg;
+                    double *B = S.bulge[pb ^ 1] + 8 * cg8 * kTS + r;
                     const double tus = tu * sc;
 #pragma unroll
-                    for (int k = 0; k < 8; ++k) B[k] = (k == 0 && cg == 0) ? xn : fma(-tus, xc[k], o[k]);
-                    bar_arrive(kBarE + pb, nE);
+                    for (int k = 0; k < 8; ++k) B[k * kTS] = (k == 0 && cg8 == 0) ? xn : fma(-tus, xc[k], o8[k]);
                 } else if (role == 2) {
                     // ---- D_s <- H D_s H
-                    const double *R = S.raw[pb][0];
                     double d[8], xc[8], a0 = 0.0, a1 = 0.0;
-                    const double xr = (r == 0) ? 0.0 : x[r], d0 = R[r * kTS], d00 = R[0];
+                    load8(xc, x + 8 * cg8);
+                    if (cg8 == 0) xc[0] = 0.0;
+                    const double xr = (r == 0) ? 0.0 : x[r];
+                    wait(&S.full[sl], (m / kRing) & 1);
+                    const double *R = S.raw[sl].d;
+                    const double d0 = R[r], d00 = R[0];
 #pragma unroll
-                    for (int k = 0; k < 8; ++k) {
-                        d[k] = R[r * kTS + 8 * cg + k];
-                        xc[k] = (k == 0 && cg == 0) ? 0.0 : x[8 * cg + k];
-                    }
+                    for (int k = 0; k < 8; ++k) d[k] = R[(8 * cg8 + k) * kTS + r];
 #pragma unroll
                     for (int k = 0; k < 8; k += 2) {
                         a0 = fma(d[k], xc[k], a0);
@@ -260,90 +427,120 @@ __global__ void __launch_bounds__(kChaseThreads, 1) band_chase_kernel(BandTri t)
                     double a = a0 + a1;
                     a += __shfl_xor_sync(kFull, a, 8);
                     a += __shfl_xor_sync(kFull, a, 16);
-                    if (cg == 0) S.ya[r] = a;
+                    if (cg8 == 0) S.ya[r] = a;
                     double p = xr * a;
                     p += __shfl_xor_sync(kFull, p, 4);
                     p += __shfl_xor_sync(kFull, p, 2);
                     p += __shfl_xor_sync(kFull, p, 1);
                     if (lane == 0) S.p2[w] = p;
+                    if (snd) wait(&S.credit[so], ((o / kRing) & 1) ^ 1);
                     bar_sync(kBarD, 4 * 32);
-                    double tau, beta, sc;
-                    house_scalars(alpha, sig, tau, beta, sc);
-                    const double p2 = (S.p2[0] + S.p2[1]) + (S.p2[2] + S.p2[3]);
+                    double ys[8], dc[8];
+                    load8(ys, S.ya + 8 * cg8);
+                    load8(dc, R + 8 * cg8);  // the first column
+                    const double p2 = (S.p2[0] + S.p2[1]) + (S.p2[2] + S.p2[3]), ya0 = S.ya[0];
+                    bar_sync(kBarY + role, 5 * 32);
+                    const double tau = S.scal[pb][0], sc = S.scal[pb][2];
                     // v^T D v with v = e_0 + sc x
-                    const double K = fma(sc, fma(sc, p2, 2.0 * S.ya[0]), d00);
-                    const double hk = 0.5 * tau * tau * K;
+                    const double Kq = fma(sc, fma(sc, p2, 2.0 * ya0), d00);
+                    const double hk = 0.5 * tau * tau * Kq;
                     const double vr = (r == 0) ? 1.0 : sc * xr;
                     const double wr = fma(-hk, vr, tau * fma(sc, a, d0));
-                    double *dst = A + (long long)(r0 + 8 * cg) * ld + r0 + r;
 #pragma unroll
                     for (int k = 0; k < 8; ++k) {
-                        const double vc = (k == 0 && cg == 0) ? 1.0 : sc * xc[k];
-                        const double wc = fma(-hk, vc, tau * fma(sc, S.ya[8 * cg + k], R[(8 * cg + k) * kTS]));
+                        const double vc = (k == 0 && cg8 == 0) ? 1.0 : sc * xc[k];
+                        const double wc = fma(-hk, vc, tau * fma(sc, ys[k], dc[k]));
                         // the same rounding for (r, c) and (c, r): the block stays symmetric
-                        const double g = __dadd_rn(__dmul_rn(vr, wc), __dmul_rn(wr, vc));
-                        if (r < L && 8 * cg + k < L) dst[(long long)k * ld] = d[k] - g;
+                        d[k] -= __dadd_rn(__dmul_rn(vr, wc), __dmul_rn(wr, vc));
                     }
-                    bar_arrive(kBarE + pb, nE);
-                    __syncwarp();
-                    if (lane == 0) {
-                        __threadfence_block();
-                        S.done[w] = s + 1;
+                    if (s == 0 && cg8 == 0) {
+                        if (r == 0) t.d[j + 1] = d[0];
+                        if (j == n - 3 && r == 1) {
+                            t.e[n - 2] = d[0];
+                            t.d[n - 1] = d[1];
+                            t.e[n - 1] = 0.0;
+                        }
+                    }
+                    if (snd) {
+                        double *T = S.stage[so].d, *Tc = T + off;
+#pragma unroll
+                        for (int k = 0; k < 8; ++k)
+                            if (cols & (1u << k)) Tc[k * kTS] = d[k];
+                        if (cg8 == 0 && r < b) {  // the first column
+                            if (s > 0) S.stage[so1].d[ecol] = d[0];
+                            else if (r >= 1) S.xout[r - 1] = d[0];
+                            if (end) T[ecol] = 0.0;  // task s + 1 has none
+                        }
                     }
                 } else if (role == 3) {
                     // ---- O_s <- H O_s: columns 8w .. 8w+7, four lanes a column
-                    if (s > 0) {
-                        const int c = 8 * w + (lane >> 2), rg = lane & 3;
-                        const double *B = S.bulge[pb] + c;
-                        double o[8], xk[8], z0 = 0.0, z1 = 0.0;
-                        const double o0 = B[0];
+                    const int c = 8 * w + rr;
+                    const double *B = S.bulge[pb] + c * kTS + 8 * cg8;
+                    double o8[8], xk[8], z0 = 0.0, z1 = 0.0;
+                    const double o0 = S.bulge[pb][c * kTS];
+                    load8(xk, x + 8 * cg8);
+                    if (cg8 == 0) xk[0] = 0.0;
+#pragma unroll
+                    for (int k = 0; k < 8; ++k) o8[k] = B[k];
+#pragma unroll
+                    for (int k = 0; k < 8; k += 2) {
+                        z0 = fma(o8[k], xk[k], z0);
+                        z1 = fma(o8[k + 1], xk[k + 1], z1);
+                    }
+                    double z = z0 + z1;
+                    z += __shfl_xor_sync(kFull, z, 8);
+                    z += __shfl_xor_sync(kFull, z, 16);
+                    bar_sync(kBarY + role, 5 * 32);
+                    const double tau = S.scal[pb][0], sc = S.scal[pb][2];
+                    const double tz = tau * fma(sc, z, o0);
+                    const double tzs = tz * sc;
+                    auto put = [&](ChaseSlot &T, bool zero) {
+                        if (c < 1 || c >= b) return;
+                        double *od = T.o + (c - 1) * kTS + 8 * cg8 - 1;
 #pragma unroll
                         for (int k = 0; k < 8; ++k) {
-                            o[k] = B[(rg + 4 * k) * kTS];
-                            xk[k] = (k == 0 && rg == 0) ? 0.0 : x[rg + 4 * k];
-                        }
-#pragma unroll
-                        for (int k = 0; k < 8; k += 2) {
-                            z0 = fma(o[k], xk[k], z0);
-                            z1 = fma(o[k + 1], xk[k + 1], z1);
-                        }
-                        double z = z0 + z1;
-                        z += __shfl_xor_sync(kFull, z, 1);
-                        z += __shfl_xor_sync(kFull, z, 2);
-                        double tau, beta, sc;
-                        house_scalars(alpha, sig, tau, beta, sc);
-                        const double tz = tau * fma(sc, z, o0);
-                        const double tzs = tz * sc;
-                        if (c < b) {
-                            double *dst = A + (long long)(r0 - b + c) * ld + r0;
-#pragma unroll
-                            for (int k = 0; k < 8; ++k) {
-                                const int row = rg + 4 * k;
-                                double v = (row == 0) ? o[k] - tz : fma(-tzs, xk[k], o[k]);
-                                if (c == 0) v = (row == 0) ? beta : 0.0;
-                                if (row < L) dst[row] = v;
-                                if (row == 0) A[(long long)r0 * ld + (r0 - b + c)] = v;
+                            const double v = zero ? 0.0 : fma(-tzs, xk[k], o8[k]);
+                            if (k > 0 || cg8 > 0) {
+                                if (8 * cg8 + k < b) od[k] = v;
+                            } else {  // the first row
+                                T.d[(c - 1) * kTS + b - 1] = T.d[(b - 1) * kTS + c - 1] = zero ? 0.0 : o8[0] - tz;
                             }
                         }
-                        __syncwarp();
-                    }
-                    if (lane == 0) {
-                        __threadfence_block();
-                        S.done[4 + w] = s + 1;
+                    };
+                    if (snd && s > 0) put(S.stage[so1], false);
+                    if (snd && end) {  // zeros for O_{s+1}, which task s + 1 does not finish
+                        wait(&S.credit[so], ((o / kRing) & 1) ^ 1);
+                        put(S.stage[so], true);
                     }
                 } else {
-                    // ---- P1: the reflector and beta
+                    // ---- P1
+                    if (lane == 0) S.tasks = s + 1;
+                    const double alpha = x[0], sig = (S.part[pb][0] + S.part[pb][1]) + (S.part[pb][2] + S.part[pb][3]);
                     double tau, beta, sc;
                     house_scalars(alpha, sig, tau, beta, sc);
-                    if (s == 0) {
-                        if (lane < L) A[(long long)j * ld + r0 + lane] = (lane == 0) ? beta : 0.0;
-                    } else if (lane == 0) {
-                        A[(long long)(r0 - b) * ld + r0] = beta;
+                    if (lane == 0) {
+                        S.scal[pb][0] = tau;
+                        S.scal[pb][1] = beta;
+                        S.scal[pb][2] = sc;
                     }
                     __syncwarp();
-                    if (lane == 0) {
+#pragma unroll
+                    for (int g = 1; g <= 3; ++g) bar_arrive(kBarY + g, 5 * 32);
+                    if (near && !S.abort) {
+                        if (s == 1 && lane < b) st_async(rem(&S.xin[lane]), (lane == b - 1) ? beta : S.xout[lane], rem(&S.fullx));
+                        if (s >= 2 && lane == 0) st_async(rem(&S.raw[so2].beta), beta, rem(&S.full[so2]));
+                    }
+                    if (far && lane == 0) {
+                        if (s == 1) S.xout[b - 1] = beta;
+                        if (s >= 2) S.stage[so2].beta = beta;
                         __threadfence_block();
                         S.refl = s + 1;
+                    }
+                    // the slot that the task before has read is free
+                    if (first && lane == 0 && s > 0 && !S.abort) mbar_arrive(smem_u32(&S.own[(m - 1) % kRing]));
+                    if (s == 0 && lane == 0) {
+                        t.e[j] = beta;
+                        if (j == 0) t.d[0] = G->beta;
                     }
                     if (t.vs) {
                         t.vs[((size_t)j * t.ntmax + s) * kBW + lane] = (lane == 0) ? 1.0 : sc * x[lane];
@@ -351,43 +548,73 @@ __global__ void __launch_bounds__(kChaseThreads, 1) band_chase_kernel(BandTri t)
                     }
                 }
             }
-        } else {
-            // ---- P2: publication
-            int pub = 0;
-            while (pub <= nt) {
-                int v = (lane < 8) ? S.done[lane] : 0x7fffffff;
-                v = __reduce_min_sync(kFull, v);
-                const int refl = S.refl;
-                const int f = __shfl_sync(kFull, (v >= nt) ? nt + 1 : min(refl, v + 1), 0);
-                if (f > pub) {
-                    pub = f;
-                    if (lane == 0) {
-                        __threadfence_block();  // the counters' values before the release, which covers their writers' stores
-                        st_release_u32(t.progress + j, (unsigned)f);
-                    }
+        }
+        __syncthreads();
+        // the last two slots (and the first column of a sweep of one task); the betas of tasks nt and
+        // nt + 1 are zero
+        if (near && warp == 2 && !S.abort) {
+            if (nt == 1 && lane < b) st_async(rem(&S.xin[lane]), (lane == b - 1) ? 0.0 : S.xout[lane], rem(&S.fullx));
+            if (lane == 0) {
+                fence_async();
+                for (int s = max(0, nt - 2); s < nt; ++s) {
+                    const int u = (out0 + s) % kRing;
+                    bulk_to_cta(rem(&S.raw[u]), smem_u32(&S.stage[u]), block_bytes, rem(&S.full[u]));
+                    st_async(rem(&S.raw[u].beta), 0.0, rem(&S.full[u]));
                 }
             }
         }
+        if (far && warp == 1 && lane == 0 && !S.abort) {
+            if (nt == 1) {
+                S.xout[b - 1] = 0.0;
+                copy_out(-1);
+            }
+            for (int s = max(0, nt - 2); s < nt; ++s) {
+                S.stage[(out0 + s) % kRing].beta = 0.0;
+                copy_out(s);
+            }
+        }
+        // credits for the last slot, and for the one that the sweep before had more
+        if (warp == 2 && lane == 0 && !S.abort) {
+            if (first) mbar_arrive(smem_u32(&S.own[(in0 + nt - 1) % kRing]));
+            else
+                for (int s = nt - 1; s < ntp; ++s) {
+                    const int m = in0 + s;
+                    if (s >= nt) wait(&S.full[m % kRing], (m / kRing) & 1);
+                    give_back(m);
+                }
+        }
         q += nt;
-        __syncthreads();
+        in0 += first ? nt : ntp;
+        if (send) out0 += nt;
     }
+    if (S.abort) __nanosleep(20000);  // copies of a neighbour that gave up may still be on their way
+    cluster.sync();
 }
 
-// The band of a symmetric matrix (lower triangle read) into the chase's compact storage: both
-// triangles within b of the diagonal, zeros elsewhere, kBW zero columns at the end.
-__global__ void band_compact_kernel(const double *A, long long lda, int n, int b, double *C) {
+// The band of a symmetric matrix (lower triangle read, element (i, j) at A[j lda + i]) as the slots
+// of the first sweep.
+__global__ void band_slots_kernel(const double *A, long long lda, int n, int b, int nt, double *slots) {
     const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= (long long)(n + kBW) * kBandLd) return;
-    const int j = (int)(t / kBandLd), i = j + (int)(t % kBandLd) - kBW;
-    const int lo = min(i, j), hi = max(i, j);
-    C[t] = (lo >= 0 && hi < n && hi - lo <= b) ? A[(size_t)lo * lda + hi] : 0.0;
-}
-
-__global__ void band_diag_kernel(const double *C, int n, double *d, double *e) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    d[i] = C[(size_t)i * kBandLd + kBW];
-    e[i] = (i + 1 < n) ? C[(size_t)i * kBandLd + kBW + 1] : 0.0;
+    if (t >= (long long)(nt + 1) * kSlotDoubles) return;
+    const int s = (int)(t / kSlotDoubles) - 1, e = (int)(t % kSlotDoubles);
+    int i = -1, j = -1;
+    if (s < 0) {  // the first column, and the first diagonal element
+        if (e < b) i = 1 + e, j = 0;
+        else if (e == 2 * kBlk) i = j = 0;
+    } else {
+        const int r0 = 1 + s * b, c = (e % kBlk) / kTS, r = (e % kBlk) % kTS;
+        if (e < kBlk) i = r0 + r, j = r0 + c;
+        else if (e < 2 * kBlk) i = r0 + b + r, j = r0 + c;
+        if (e < 2 * kBlk && (r >= b || c >= b)) i = -1;
+        if (e >= kBlk && r == b - 1) i = -1;
+        if (e == 2 * kBlk) i = r0 + 2 * b - 1, j = r0 + b - 1;
+    }
+    double v = 0.0;
+    if (i >= 0 && i < n && j < n) {
+        const int lo = min(i, j), hi = max(i, j);
+        if (hi - lo <= b) v = A[(size_t)lo * lda + hi];
+    }
+    slots[t] = v;
 }
 
 // Back-transformation, COLS eigenvector columns per CTA held in shared memory (column c at
@@ -506,38 +733,53 @@ cudaError_t launch_band_prepare(double *A, long long lda, int n, int b, unsigned
     return cudaGetLastError();
 }
 
-size_t band_compact_doubles(int n) { return (size_t)(n + kBW) * kBandLd; }
+size_t band_slot_doubles(int n, int b) { return (size_t)(band_ntask(n, b, 0) + 1) * kSlotDoubles; }
 
-cudaError_t launch_band_compact(const double *A, long long lda, int n, int b, double *C, cudaStream_t st) {
-    const long long tot = (long long)(n + kBW) * kBandLd;
+cudaError_t launch_band_slots(const double *A, long long lda, int n, int b, double *slots, cudaStream_t st) {
+    const long long tot = (long long)band_slot_doubles(n, b);
     DVR3D_COUNT_LAUNCH(1);
-    band_compact_kernel<<<(unsigned)((tot + 255) / 256), 256, 0, st>>>(A, lda, n, b, C);
+    band_slots_kernel<<<(unsigned)((tot + 255) / 256), 256, 0, st>>>(A, lda, n, b, band_ntask(n, b, 0), slots);
     return cudaGetLastError();
 }
 
 cudaError_t launch_band_chase(BandTri &t, cudaStream_t st) {
-    if (t.b < 1 || t.b > kBW || t.n < 3) return cudaErrorInvalidValue;
+    if (t.b < 2 || t.b > kBW || t.n < 3) return cudaErrorInvalidValue;
     t.ntmax = band_ntask(t.n, t.b, 0);
     cudaError_t e = cudaMemsetAsync(t.progress, 0, sizeof(unsigned) * t.n, st);
     if (e != cudaSuccess) return e;
-    const size_t smem = sizeof(ChaseSmem);
-    e = cudaFuncSetAttribute(band_chase_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-    // one CTA per sweep in flight: sweeps follow at least three tasks apart and a CTA is busy
-    // for ntask tasks, so ntask / 2 plus slack keeps every sweep's successor supplied
-    int grid = std::min(t.n - 2, std::max(8, t.ntmax / 2 + 8));
-    int dev = 0, nsm = 0, per = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, band_chase_kernel, kChaseThreads, smem);
-    grid = std::max(1, std::min(grid, nsm * std::max(per, 1)));
-    void *args[] = {&t};
-    DVR3D_COUNT_LAUNCH(1);
-    e = cudaLaunchCooperativeKernel((void *)band_chase_kernel, dim3(grid), dim3(kChaseThreads), args, smem, st);
-    if (e != cudaSuccess) return e;
-    DVR3D_COUNT_LAUNCH(1);
-    band_diag_kernel<<<(t.n + 255) / 256, 256, 0, st>>>(t.C, t.n, t.d, t.e);
-    return cudaGetLastError();
+    const int smem = (int)sizeof(ChaseSmem);
+    if ((e = cudaFuncSetAttribute(band_chase_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)) != cudaSuccess) return e;
+    if ((e = cudaFuncSetAttribute(band_chase_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1)) != cudaSuccess) return e;
+    // sweeps follow at least two tasks apart and a CTA is busy for ntask tasks, so ntask / 2 plus
+    // slack keeps every sweep's successor supplied; clusters wait for one another, so no more than
+    // the device holds at a time (a cooperative launch)
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeCooperative;
+    attr[1].val.cooperative = 1;
+    cfg.blockDim = dim3(kChaseThreads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cfg.attrs = attr;
+    for (int K = kChaseCluster; K >= 1; K /= 2) {
+        attr[0].val.clusterDim.x = K;
+        cfg.gridDim = dim3(K);
+        cfg.numAttrs = 1;
+        int most = 0;
+        if (cudaOccupancyMaxActiveClusters(&most, band_chase_kernel, &cfg) != cudaSuccess || most < 1) {
+            cudaGetLastError();
+            continue;
+        }
+        const int want = (std::min(t.n - 2, std::max(8, t.ntmax / 2 + 8)) + K - 1) / K;
+        cfg.gridDim = dim3(K * std::max(1, std::min(want, most)));
+        cfg.numAttrs = 2;
+        DVR3D_COUNT_LAUNCH(1);
+        return cudaLaunchKernelEx(&cfg, band_chase_kernel, t);
+    }
+    return cudaErrorNotSupported;
 }
 
 cudaError_t launch_band_backtransform(const BandTri &t, double *Z, long long ldz, int nev, cudaStream_t st) {

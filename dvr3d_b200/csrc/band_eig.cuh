@@ -9,10 +9,8 @@ namespace dvr3d {
 
 constexpr int kBandMaxBw = 32;  // widest band handled (one warp lane per row of a block)
 
-constexpr int kBandLd = 3 * kBandMaxBw;  // doubles a column of the chase's compact band storage
-
 struct BandTri {
-    double *C;              // the band in compact storage (launch_band_compact); overwritten
+    double *slots;          // the band as the chase reads it (launch_band_slots); overwritten
     int n, b;
     int ntmax;              // tasks per sweep at most: (n - 2) / b + 1 (set by launch_band_chase)
     double *d, *e;          // out: tridiagonal (d[i] = A[i][i], e[i] = A[i+1][i])
@@ -30,10 +28,10 @@ cudaError_t launch_band_prepare(double *A, long long lda, int n, int b, unsigned
                                 cudaStream_t st);
 size_t band_reflector_doubles(int n, int b);  // vs
 size_t band_tau_doubles(int n, int b);        // taus
-size_t band_compact_doubles(int n);           // C
-cudaError_t launch_band_compact(const double *A, long long lda, int n, int b, double *C, cudaStream_t st);
-// Bulge chasing (one CTA per sweep in flight, sweeps pipelined through progress flags),
-// then d and e from the reduced matrix.
+// The band of A (lower triangle, column-major) in the chase's input form; b >= 2.
+size_t band_slot_doubles(int n, int b);
+cudaError_t launch_band_slots(const double *A, long long lda, int n, int b, double *slots, cudaStream_t st);
+// Bulge chasing (one CTA per sweep in flight) to the tridiagonal d, e.
 cudaError_t launch_band_chase(BandTri &t, cudaStream_t st);
 constexpr int kBandBackMax = 22000;  // largest order launch_band_backtransform takes
 // Z (n x nev, ldz) <- Q Z with Q the product of the chase's reflectors (A = Q T Q^T).

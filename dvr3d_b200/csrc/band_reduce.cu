@@ -117,8 +117,7 @@ __global__ void __launch_bounds__((kPanelWarps + 1) * 32, 1) panel_qr_kernel(Pan
             const int r = q & 31, c = q >> 5;
             if (r < c || p.j0 + r >= p.n) continue;
             const double v = __ldcg(p.P + (size_t)c * p.ldp + r);
-            p.C[(size_t)(p.j0 + c) * kBandLd + kB + r - c] = v;
-            p.C[(size_t)(p.j0 + r) * kBandLd + kB + c - r] = v;
+            p.C[(size_t)(p.j0 + c) * kBandLd + r - c] = v;
         }
     }
     for (int q = tid; q < 32 * 33; q += blockDim.x) (&S.T[0][0])[q] = 0.0;
@@ -261,8 +260,7 @@ __global__ void __launch_bounds__((kPanelWarps + 1) * 32, 1) panel_qr_kernel(Pan
         double o = v;
         if (b == 0 && r <= c) {  // R
             const int i = p.j0 + 32 + r, j = p.j0 + c;
-            p.C[(size_t)j * kBandLd + kB + i - j] = v;
-            p.C[(size_t)i * kBandLd + kB + j - i] = v;
+            p.C[(size_t)j * kBandLd + i - j] = v;
             o = (r == c) ? 1.0 : 0.0;
         }
         if (c >= p.nr) o = 0.0;
@@ -719,7 +717,7 @@ cudaError_t launch_band_reduce(const BandReduce &b, cudaStream_t st) {
     double *VWV = b.work, *X = VWV + 96 * ld, *P = X + 32 * ld, *M = P + 32 * ld;
     if (!band_reduce_available()) return cudaErrorNotSupported;
     cudaError_t e;
-    if ((e = cudaMemsetAsync(b.C, 0, band_compact_doubles(n) * sizeof(double), st)) != cudaSuccess) return e;
+    if ((e = cudaMemsetAsync(b.C, 0, band_storage_doubles(n) * sizeof(double), st)) != cudaSuccess) return e;
     int dev = 0, nsm = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);

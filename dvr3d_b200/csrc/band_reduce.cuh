@@ -13,13 +13,16 @@ struct BandReduce {
     long long lda;     // panel q's block reflector vectors V stay in A[32 (q + 1) :, 32 q : 32 q + 32]
     int n;
     bool keep;         // keep V and T for launch_band_reduce_back
-    double *C;         // out: the band in the chase's compact storage (band_compact_doubles(n))
+    double *C;         // out: the band's lower triangle, element (i, j) at C[j (kBandLd - 1) + i]
+                       // (band_storage_doubles(n))
     double *T;         // [band_reduce_panels(n)][32 x 32] triangular factors
     double *work;      // band_reduce_work_doubles(n)
 };
 
 // Whether the current device takes the panel kernel's cluster.
 bool band_reduce_available();
+constexpr int kBandLd = kBandMaxBw + 1;
+inline size_t band_storage_doubles(int n) { return (size_t)n * kBandLd; }
 inline int band_reduce_panels(int n) { return (n + kBandMaxBw - 1) / kBandMaxBw; }
 size_t band_reduce_work_doubles(int n);
 cudaError_t launch_band_reduce(const BandReduce &b, cudaStream_t st);

@@ -648,7 +648,7 @@ void dense_lowest_two_stage(dvr3d_ctx *ctx, double *A, long long lda, int n, int
     br.lda = lda;
     br.n = n;
     br.keep = vecs;
-    br.C = ctx->arena.get_t<double>(t + "bandC", band_compact_doubles(n));
+    br.C = ctx->arena.get_t<double>(t + "bandC", band_storage_doubles(n));
     br.T = ctx->arena.get_t<double>(t + "bandT", (size_t)band_reduce_panels(n) * kBandMaxBw * kBandMaxBw);
     br.work = ctx->arena.get_t<double>(t + "bandwork", band_reduce_work_doubles(n));
     if (time_panels) CK(cudaEventRecord(ctx->panel_ev[0], st));
@@ -657,9 +657,10 @@ void dense_lowest_two_stage(dvr3d_ctx *ctx, double *A, long long lda, int n, int
     const int reduce_launches = (int)(g_kernel_launches - launches0);
     if (time_panels) CK(cudaEventRecord(ctx->panel_ev[1], st));
     BandTri bt{};
-    bt.C = br.C;
     bt.n = n;
     bt.b = kBandMaxBw;
+    bt.slots = ctx->arena.get_t<double>(t + "bandslots", band_slot_doubles(n, bt.b));
+    CK(launch_band_slots(br.C, kBandLd - 1, n, bt.b, bt.slots, st));
     bt.d = ctx->arena.get_t<double>(t + "d", n);
     bt.e = ctx->arena.get_t<double>(t + "e", n);
     if (vecs) {
@@ -805,7 +806,7 @@ void dense_lowest(dvr3d_ctx *ctx, double *A, long long lda, int n, int nev, bool
 bool band_lowest(dvr3d_ctx *ctx, double *A, long long lda, int n, int b, int nev, double *w, double *Z,
                  long long ldz, double drop_rel, double *dropped_rel) {
     cudaStream_t st = ctx->stream;
-    if (b < 1 || b > kBandMaxBw || n < 3 || nev > n) return false;
+    if (b < 2 || b > kBandMaxBw || n < 3 || nev > n) return false;
     auto *mx = ctx->arena.get_t<unsigned long long>("bd_max", 2);
     CK(launch_band_prepare(A, lda, n, b, mx, st));
     unsigned long long hb[2] = {0, 0};
@@ -819,8 +820,8 @@ bool band_lowest(dvr3d_ctx *ctx, double *A, long long lda, int n, int b, int nev
     if (dropped_rel) *dropped_rel = rel;
     if (!(rel <= drop_rel)) return false;
     BandTri t{};
-    t.C = ctx->arena.get_t<double>("bd_C", band_compact_doubles(n));
-    CK(launch_band_compact(A, lda, n, b, t.C, st));
+    t.slots = ctx->arena.get_t<double>("bd_slots", band_slot_doubles(n, b));
+    CK(launch_band_slots(A, lda, n, b, t.slots, st));
     t.n = n;
     t.b = b;
     t.d = ctx->arena.get_t<double>("bd_d", n);
