@@ -123,7 +123,10 @@ void compute_wavefunctions(dvr3d_ctx *ctx, const BlockPlan &p, const Contracted 
     const long long nq = (long long)nb * P;
     double *Psi = ctx->arena.get_t<double>("wf_psi", (size_t)nq * nlev);
     for (int b = 0; b < nb; ++b) {
-        if (sz[b] == 0) continue;
+        if (sz[b] == 0) {  // no function there: zero amplitudes, whatever the buffer held before
+            CK(cudaMemset2DAsync(Psi + (size_t)b * P, sizeof(double) * nq, 0, sizeof(double) * P, nlev, st));
+            continue;
+        }
         GemmOp g;  // Psi[b P : (b+1) P, :] = Vt[:, col0 b ...] Zp[colp b ..., :]
         g.M = P;
         g.N = nlev;
