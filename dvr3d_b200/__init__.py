@@ -447,11 +447,9 @@ class Context:
         o = Options(precision=precision)
         need = C.c_size_t(0)
         needl = C.c_size_t(0)
-        # the first call sizes the text buffers (and writes no wavefunction file)
-        self._check(self._lib.dvr3d_b200_run_deck(self._h, text.encode(), C.byref(o), None, 0, C.byref(need),
-                                                  None, 0, C.byref(needl)))
-        out = C.create_string_buffer(need.value + 1)
-        lev = C.create_string_buffer(needl.value + 1)
+        # One run, with room for some 5 000 levels; a job with more text than that is run once more
+        # with the room it asked for (its wavefunction file is written by then).
+        out, lev = C.create_string_buffer(1 << 18), C.create_string_buffer(1 << 18)
         if wave_path is None:
             self._check(self._lib.dvr3d_b200_run_deck(self._h, text.encode(), C.byref(o), out, len(out),
                                                       C.byref(need), lev, len(lev), C.byref(needl)))
@@ -459,4 +457,8 @@ class Context:
             self._check(self._lib.dvr3d_b200_run_deck_wave(self._h, text.encode(), C.byref(o), out, len(out),
                                                            C.byref(need), lev, len(lev), C.byref(needl),
                                                            str(wave_path).encode()))
+        if need.value > len(out) or needl.value > len(lev):
+            out, lev = C.create_string_buffer(need.value + 1), C.create_string_buffer(needl.value + 1)
+            self._check(self._lib.dvr3d_b200_run_deck(self._h, text.encode(), C.byref(o), out, len(out),
+                                                      C.byref(need), lev, len(lev), C.byref(needl)))
         return out.value.decode(), lev.value.decode()

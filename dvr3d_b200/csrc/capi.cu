@@ -1,9 +1,13 @@
 // capi.cu -- extern "C" entry points declared in include/dvr3d_b200.h.
+#include <sys/stat.h>
+#include <unistd.h>
+
 #include <chrono>
 #include <cmath>
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
+#include <memory>
 #include <string>
 #include <vector>
 
@@ -604,19 +608,15 @@ struct FortranRecords {
         rec.insert(rec.end(), c, c + n);
     }
     void end() {
-        if (rec.size() > 0x7fffffffu) throw HostError{DVR3D_ERR_UNSUPPORTED, "wavefunction record above 2 GiB"};
-        const unsigned int n = (unsigned int)rec.size();
-        if (std::fwrite(&n, 4, 1, f) != 1 || (n && std::fwrite(rec.data(), 1, n, f) != n) ||
-            std::fwrite(&n, 4, 1, f) != 1)
-            throw HostError{DVR3D_ERR_ARG, "writing the wavefunction file failed"};
+        whole(rec.data(), rec.size());
         rec.clear();
     }
-};
-
-struct FileCloser {
-    FILE *f;
-    ~FileCloser() {
-        if (f) std::fclose(f);
+    // a record that lies in one piece already
+    void whole(const void *p, size_t bytes) {
+        if (bytes > 0x7fffffffu) throw HostError{DVR3D_ERR_UNSUPPORTED, "wavefunction record above 2 GiB"};
+        const unsigned int n = (unsigned int)bytes;
+        if (std::fwrite(&n, 4, 1, f) != 1 || (n && std::fwrite(p, 1, n, f) != n) || std::fwrite(&n, 4, 1, f) != 1)
+            throw HostError{DVR3D_ERR_ARG, "writing the wavefunction file failed"};
     }
 };
 
@@ -704,11 +704,55 @@ void write_wave_block(FortranRecords &wr, const dvr3d::BlockPlan &p, const dvr3d
     wr.end();
     wr.r8s(ev, r.meval);
     wr.end();
-    for (int l = 0; l < wave.nlev; ++l) {
-        wr.r8s(wave.psi.data() + (size_t)l * wave.len, (size_t)wave.len);
-        wr.end();
-    }
+    for (int l = 0; l < wave.nlev; ++l) wr.whole(wave.psi.data() + (size_t)l * wave.len, 8 * (size_t)wave.len);
 }
+
+// The wavefunction file of one job. It is opened for appending before the first solve, so that a
+// path that cannot be written is refused at once; a file that was there is emptied only when the
+// first block is written, and one that was not is taken away again if none ever is. Blocks wait
+// in memory (up to kHeld bytes) until the job's last solve, so that a job that fails leaves the
+// file of the run before it as it was: a caller needs no trial run to find that out.
+struct WaveFile {
+    static constexpr size_t kHeld = (size_t)1 << 30;
+    struct Block {
+        dvr3d::BlockPlan p;
+        dvr3d_result r;
+        std::vector<int> iv2;
+        std::vector<double> ev;
+        dvr3d::WaveOut wave;
+    };
+    std::string path;
+    FILE *f = nullptr;
+    bool fresh = false, begun = false;
+    size_t held = 0;
+    std::vector<Block> blocks;
+    FortranRecords wr;
+
+    explicit WaveFile(const char *p) : path(p) {
+        fresh = ::access(p, F_OK) != 0;
+        f = std::fopen(p, "ab");
+        if (!f) throw HostError{DVR3D_ERR_ARG, "cannot open " + path};
+        wr.f = f;
+    }
+    WaveFile(const WaveFile &) = delete;
+    ~WaveFile() {
+        std::fclose(f);
+        if (fresh && !begun) std::remove(path.c_str());
+    }
+    void write_held(const dvr3d_deck &d, int kd, int ku) {
+        if (!begun) {
+            // (a pipe or a device has no length to set)
+            struct stat sb;
+            if (::fstat(fileno(f), &sb) == 0 && S_ISREG(sb.st_mode) && ::ftruncate(fileno(f), 0) != 0)
+                throw HostError{DVR3D_ERR_ARG, "cannot empty " + path};
+            begun = true;
+            write_wave_header(wr, d, kd, ku);
+        }
+        for (const Block &b : blocks) write_wave_block(wr, b.p, b.r, b.iv2.data(), b.ev.data(), b.wave);
+        blocks.clear();
+        held = 0;
+    }
+};
 
 }  // namespace
 
@@ -727,14 +771,8 @@ static int run_deck_impl(dvr3d_ctx *ctx, const char *deck_text, const dvr3d_opti
         std::string s, lv;
         // the wavefunction file (unit IWAVE): written when the deck sets ZTRAN and a path is given
         const bool ztran = d.ztran && wave_path && wave_path[0];
-        FortranRecords wr;
-        FileCloser closer{nullptr};
-        if (ztran) {
-            closer.f = std::fopen(wave_path, "wb");
-            if (!closer.f) throw HostError{DVR3D_ERR_ARG, std::string("cannot open ") + wave_path};
-            wr.f = closer.f;
-            write_wave_header(wr, d, kd, ku);
-        }
+        std::unique_ptr<WaveFile> wf;
+        if (ztran) wf.reset(new WaveFile(wave_path));
         appendf(s, "     Program DVR3DRJZ (B200 hot path)\n\n     Title: %s\n", d.title);
         for (int kk = kd; kk <= ku; ++kk) {
             dvr3d::BlockPlan p;
@@ -748,7 +786,6 @@ static int run_deck_impl(dvr3d_ctx *ctx, const char *deck_text, const dvr3d_opti
             r.iv2_cap = (int)iv2.size();
             dvr3d::WaveOut wave;
             dvr3d::solve_block(ctx, d, kk, o, r, ztran ? &wave : nullptr);
-            if (ztran) write_wave_block(wr, p, r, iv2.data(), ev.data(), wave);
             if (d.jrot != 0 && p.zrot) appendf(s, "\n     Solutions with J =%3d k =%3d\n", p.jrot, p.kz);
             if (p.radau && d.jrot != 0 && p.zrot)
                 appendf(s, p.ipar == 0 ? "\n     even parity solutions\n" : "\n     odd parity solutions\n");
@@ -797,7 +834,13 @@ static int run_deck_impl(dvr3d_ctx *ctx, const char *deck_text, const dvr3d_opti
                     if (c % 5 == 4 || i == meval - 1) s += "\n\n";
                 }
             }
+            if (ztran) {
+                wf->held += 8 * wave.psi.size();
+                wf->blocks.push_back({std::move(p), r, std::move(iv2), std::move(ev), std::move(wave)});
+                if (wf->held > WaveFile::kHeld) wf->write_held(d, kd, ku);
+            }
         }
+        if (ztran) wf->write_held(d, kd, ku);
         copy_out(s, out, outcap, outlen);
         copy_out(lv, lev, levcap, levlen);
         return DVR3D_OK;

@@ -20,8 +20,6 @@
 #include <cstdint>
 #include <cstdio>
 #include <cstring>
-#include <fstream>
-#include <iterator>
 #include <string>
 #include <vector>
 
@@ -118,10 +116,42 @@ RotDeck parse_rot_deck(const char *text) {
     return d;
 }
 
-// Gauss-associated Legendre rule of ROTLEV3B's jacobi (:941-1007): zeros of the Jacobi
-// polynomial P_n^(k,k) found by a downward sign scan from x = 1 in steps of 1e-6, refined by
-// Newton (10 steps at most, |dx| <= 1e-12) with the derivative of the last evaluation; weights
-// from the recurrence constant. Returned over the full range, ascending (angin1 :760-764).
+// The points of ROTLEV3B's walk (:969-985): x_0 = 1, x_(i+1) = x_i - 1e-6 rounded to double, down
+// to -1.5e-6. Between two powers of two every subtraction rounds to the same step, a multiple of
+// the spacing there, so a run of points is start - m * step without error; the last thousand (and
+// the steps across a power of two) are taken one by one. The very points matter: Newton starts
+// from them, and the weights' last digits depend on where it started.
+struct RotWalk {
+    struct Run {
+        int i;
+        double x, step;
+    };
+    std::vector<Run> runs;
+    int size = 0;
+    RotWalk() {
+        const double h = 1.0e-6;
+        for (double x = 1.0; x > -1.5 * h;) {
+            const double y = x - h, low = x > 1.0e-3 ? std::ldexp(1.0, std::ilogb(x)) : x;
+            runs.push_back({size, x, x - y});
+            const int m = y >= low ? (int)((x - low) / (x - y)) : 0;
+            x = m > 0 ? x - m * (x - y) : y;
+            size += m > 0 ? m : 1;
+        }
+    }
+    double operator[](int i) const {
+        auto r = std::upper_bound(runs.begin(), runs.end(), i, [](int v, const Run &a) { return v < a.i; }) - 1;
+        return r->x - (i - r->i) * r->step;
+    }
+};
+
+// Gauss-associated Legendre rule of ROTLEV3B's jacobi (:941-1007): each zero of the Jacobi
+// polynomial P_n^(k,k) from the step of 1e-6, counted down from x = 1, that it lies in, refined
+// by Newton (10 steps at most, |dx| <= 1e-12) with the derivative of the last evaluation;
+// weights from the recurrence constant. Returned over the full range, ascending (angin1
+// :760-764). The reference walks all the steps and looks for changes of sign; here the steps are
+// bisected on the number of zeros above a point, the sign changes along the recurrence (P_0 ..
+// P_n is a Sturm sequence), which takes 20 evaluations a zero instead of 10^6 in all (a rule of
+// 40 points: 44 ms before, 0.1 now). A step with two zeros is refused as the walk refuses it.
 void rot_quadrature(int n, int k, std::vector<double> &x, std::vector<double> &w, double &cs, double &ts) {
     const double a = k, b = k;
     std::vector<double> c(n + 1, 0.0);
@@ -151,17 +181,35 @@ void rot_quadrature(int n, int k, std::vector<double> &x, std::vector<double> &w
     const int n2 = (n + 1) / 2;
     std::vector<double> xt;
     const double xstep = 1.0e-6;
-    double pm1 = 1.0, xx = 1.0;
-    for (;;) {
+    auto zeros_above = [&](double xx) {
+        double pa = 1.0, pb = xx + (a - b) / (a + b + 2.0);
+        bool neg = pb <= 0.0;  // a zero counts as a change of sign
+        int cnt = neg;
+        for (int j = 2; j <= n; ++j) {
+            const double q = xx * pb - c[j] * pa;
+            pa = pb;
+            pb = q;
+            const bool ng = pb < 0.0 || (pb == 0.0 && !neg);
+            cnt += ng != neg;
+            neg = ng;
+        }
+        return cnt;
+    };
+    const RotWalk walk;
+    int last = -1;  // the step of the zero before
+    for (int t = 1; t <= n2; ++t) {
+        int lo = last, hi = walk.size - 1;  // fewer than t zeros above point lo, t above hi
+        while (hi - lo > 1) {
+            const int mid = lo + (hi - lo) / 2;
+            (zeros_above(walk[mid]) >= t ? hi : lo) = mid;
+        }
+        const double xx = walk[hi];
         double p, dp, p1;
         recur(xx, p, dp, p1);
-        if (pm1 * p < 0.0) {
-            pm1 = -pm1;
-            xt.push_back(xx - 0.5 * xstep);
-        }
-        if ((int)xt.size() == n2) break;
-        xx -= xstep;
-        if (!(xx > -1.5 * xstep)) bad(DVR3D_ERR_QUADRATURE, "ROTLEV3B quadrature: wrong number of zeros found");
+        if (!((t % 2 ? p : -p) < 0.0 || (p == 0.0 && dp != 0.0)))
+            bad(DVR3D_ERR_QUADRATURE, "ROTLEV3B quadrature: wrong number of zeros found");
+        xt.push_back(xx - 0.5 * xstep);
+        last = hi;
     }
     std::vector<double> xh(n2), wh(n2);
     cs = 0.0;
@@ -246,10 +294,16 @@ std::vector<double> angular_block(int step, int k1, const KBlock &b1, const KBlo
     auto P1 = [&](int j, int i) { return b1.pleg[(size_t)i * ld1 + j]; };
     auto P2 = [&](int j, int i) { return b2.pleg[(size_t)i * ld2 + j]; };
     std::vector<double> ang((size_t)b1.iang * b2.iang, 0.0);  // column-major iang1 x iang2
+    std::vector<double> row(n2);
     const double kkp1 = (double)k1 * (k1 + 1), xkph = k1 + 0.5;
     int i1 = 0;
     for (int i = 0; i < n1; ++i) {
         if (b1.iv[i] == 0) continue;
+        for (int jp = 0; jp < n2; ++jp) {  // row i of P1^T fbr
+            double sum = 0.0;
+            for (int j = 0; j < n1; ++j) sum += P1(j, i) * fbr[(size_t)jp * n1 + j];
+            row[jp] = sum;
+        }
         int i2 = 0;
         for (int ip = 0; ip < n2; ++ip) {
             if (b2.iv[ip] == 0) continue;
@@ -259,8 +313,8 @@ std::vector<double> angular_block(int step, int k1, const KBlock &b1, const KBlo
                     const double jj = k1 + j;
                     sum1 += P1(j, i) * P2(j - 1, ip) * std::sqrt(jj * (jj + 1.0) - kkp1);
                 }
-                for (int jp = 0; jp < n2; ++jp) sum2 += P1(j, i) * P2(jp, ip) * fbr[(size_t)jp * n1 + j];
             }
+            for (int jp = 0; jp < n2; ++jp) sum2 += row[jp] * P2(jp, ip);
             ang[(size_t)i2 * b1.iang + i1] = (step == 1 ? sum1 + xkph * sum2 : sum2) * angfac;
             ++i2;
         }
@@ -425,9 +479,29 @@ void rotlev3b_solve(dvr3d_ctx *ctx, const char *deck_text, const char *wave_path
     const std::vector<double> radmee = mkrad(0, 0, 0), radmoo = mkrad(1, 0, 0), radmeo = mkrad(1, 1, 0),
                               radmoe = mkrad(1, 1, 1);
     cudaStream_t st = ctx->stream;
-    // first-step vectors of a block, on the device (ibass x nv)
-    auto upload_vectors = [&](const KBlock &b, int nv, const char *name) {
-        double *d = ctx->arena.get_t<double>(name, (size_t)b.ibass * std::max(nv, 1));
+    // first-step vectors of a block, on the device (ibass x nv). Every block meets its four
+    // neighbours, so the last three blocks stay, one in each of three buffers (the buffer of the
+    // block used longest ago is taken); sent anew for every pair, the vectors crossed to the device
+    // six to eight times.
+    struct Held {
+        const KBlock *b = nullptr;
+        int nv = 0;
+        long long used = 0;
+        double *d = nullptr;
+    } held[3];
+    long long uses = 0;
+    auto upload_vectors = [&](const KBlock &b, int nv) {
+        int s = 0;
+        for (int i = 0; i < 3; ++i) {
+            if (held[i].b == &b && held[i].nv == nv) {
+                held[i].used = ++uses;
+                return held[i].d;
+            }
+            if (held[i].used < held[s].used) s = i;
+        }
+        static const char *const names[3] = {"rt_c0", "rt_c1", "rt_c2"};
+        double *d = ctx->arena.get_t<double>(names[s], (size_t)b.ibass * std::max(nv, 1));
+        held[s] = Held{&b, nv, ++uses, d};
         for (int v = 0; v < nv; ++v)
             CK(cudaMemcpyAsync(d + (size_t)v * b.ibass, f.vec(b.vec0 + v, (size_t)b.ibass), sizeof(double) * b.ibass,
                                cudaMemcpyHostToDevice, st));
@@ -488,8 +562,8 @@ void rotlev3b_solve(dvr3d_ctx *ctx, const char *deck_text, const char *wave_path
             const int npair = (int)m1.size();
             if (ir1 > b1.ibass / b1.iang || ir2 > nrad2 || (int)rad.size() != npair)
                 bad(DVR3D_ERR_ARG, "wavefunction file: radial basis does not match the block parities");
-            double *C1 = upload_vectors(b1, n1, "rt_c1");
-            double *C2 = upload_vectors(b2, n2, "rt_c2");
+            double *C1 = upload_vectors(b1, n1);
+            double *C2 = upload_vectors(b2, n2);
             double *A = ctx->arena.get_t<double>("rt_ang", ang.size());
             CK(cudaMemcpyAsync(A, ang.data(), sizeof(double) * ang.size(), cudaMemcpyHostToDevice, st));
             const long long K = (long long)npair * b1.iang;
@@ -607,7 +681,7 @@ void rotlev3b_solve(dvr3d_ctx *ctx, const char *deck_text, const char *wave_path
             if (kk != b.iang) bad(DVR3D_ERR_ARG, "wavefunction file: kept angles differ from iang");
             double *Pd = ctx->arena.get_t<double>("rt_tp", pk.size());
             CK(cudaMemcpyAsync(Pd, pk.data(), sizeof(double) * pk.size(), cudaMemcpyHostToDevice, st));
-            double *V = upload_vectors(b, mvi, "rt_c1");
+            double *V = upload_vectors(b, mvi);
             double *Bm = ctx->arena.get_t<double>("rt_tb", (size_t)nkbas[i] * mvi);
             double *D = ctx->arena.get_t<double>("rt_td", (size_t)nkbas[i] * nval);
             launch_dgemm(false, false, nang, nrad * mvi, b.iang, 1.0, Pd, nang, V, b.iang, 0.0, Bm, nang, st);
