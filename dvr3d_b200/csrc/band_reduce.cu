@@ -9,9 +9,11 @@
 //   vtx_kernel       S = V^T X, M = -T^T S T / 2;
 //   w_kernel         W = X T + V M, and the next panel's columns of A2 - V W^T - W V^T;
 //   syr2k_kernel     the rest of A2 <- A2 - V W^T - W V^T (lower triangle).
-// 4/3 n^3 flop, nearly all in symm and syr2k on the FP64 tensor path (DMMA m16n8k16). At n = 12241
-// the whole reduction to tridiagonal form with the chase takes 305 ms against 970 ms in one stage
-// (symm 65, syr2k 65, panels 37, w 10, vtx 8, chase 119).
+// 4/3 n^3 flop, nearly all in symm and syr2k on the FP64 tensor path (DMMA m16n8k16). The next panel
+// needs only what w_kernel makes, so it runs beside syr2k, on 16 of the SMs. At n = 12202 the whole
+// reduction to tridiagonal form with the chase takes 210 ms against 970 ms in one stage (symm 65,
+// syr2k with the panels beside it 70, vtx 8, w 4, chase 49); one after the other, with a cluster
+// barrier in every column of a panel, the same took 250.
 #include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
@@ -20,6 +22,7 @@
 #include <cmath>
 
 #include "band_reduce.cuh"
+#include "cluster_dev.cuh"
 #include "common.cuh"
 #include "dmma.cuh"
 #include "gemm64.cuh"
@@ -55,6 +58,8 @@ struct PanelArgs {
     int j0, n;
     int nsm;            // blocks of a CTA in shared memory, the rest in `spill` (L2)
     double *spill;
+    int *err;           // set when a wait runs out
+    unsigned long long limit;
 };
 
 struct PanelShared {
@@ -64,15 +69,23 @@ struct PanelShared {
     double ppart[2][32];
     double w[32], z[32];
     double T[32][33];
-    double sc, tau, beta;
+    double sc, beta;
+    unsigned long long full[2];      // mbarriers: cpart and ppart are complete
 };
+constexpr unsigned kPanelBytes = (kCl + 1) * 32 * sizeof(double);  // what a column brings to each CTA
+constexpr unsigned long long kPanelPolls = 1ull << 26;  // of a wait, about a second
+constexpr int kBarPart = 1, kBarRow = 2;  // the warps' sums are there; the rank-1 update is known
 
 // One thread-block cluster factors the panel. Each warp keeps one 32 x 32 block of it in registers
 // (lane = (row mod 4, column mod 8): 8 x 4 elements) and, beyond 7680 rows, further blocks in
 // shared memory (beyond 19968 in L2). Per column one all-reduce of x^T [a_0 .. a_31] over the cluster, x the column
 // below its pivot, gives the norm, the row vector of the rank-1 update and the column of V^T V
-// that T needs; so a column costs one cluster barrier and two block barriers.
-// Latency bound: 2.4 us a column, 76 us a panel at 900 rows and 97 us on average from 12000 down.
+// that T needs. A control warp does all of the exchange: it adds up the warps' sums, stores them into
+// every CTA of the cluster (st.async: the mbarrier there counts the bytes, so nothing waits for the
+// stores to return and no cluster barrier follows), adds up what has come in and forms the scalars;
+// the others meet it at two named barriers a column, and T's column follows off the path.
+// Latency bound: 1.6 us a column; 59 us a panel on average from 3968 rows down (81 with a cluster
+// barrier a column and the exchange on a working warp).
 __global__ void __launch_bounds__((kPanelWarps + 1) * 32, 1) panel_qr_kernel(PanelArgs p) {
     extern __shared__ __align__(16) double psm[];
     PanelShared &S = *reinterpret_cast<PanelShared *>(psm);
@@ -80,7 +93,7 @@ __global__ void __launch_bounds__((kPanelWarps + 1) * 32, 1) panel_qr_kernel(Pan
     cg::cluster_group cluster = cg::this_cluster();
     const int rank = (int)cluster.block_rank();
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int NW = (int)(blockDim.x >> 5) - 1;
+    const int NW = (int)(blockDim.x >> 5) - 1, nthr = (int)blockDim.x;
     const bool worker = warp < NW;
     const int rl = lane & 3, cl = lane >> 2;
     const int nblk = (p.R + 31) / 32;
@@ -121,136 +134,165 @@ __global__ void __launch_bounds__((kPanelWarps + 1) * 32, 1) panel_qr_kernel(Pan
         }
     }
     for (int q = tid; q < 32 * 33; q += blockDim.x) (&S.T[0][0])[q] = 0.0;
+    const unsigned full0 = smem_u32(&S.full[0]);
+    if (tid == 0) {
+        for (int q = 0; q < 2; ++q) {
+            mbar_init(full0 + 8 * q, 1);
+            mbar_expect(full0 + 8 * q, kPanelBytes);
+        }
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
     cluster.sync();
+    // the control warp: lane = (half of the cluster, pair of columns)
+    const int hc = (lane >> 4) * (kCl / 2), cp2 = 2 * (lane & 15);
+    bool patient = true;  // until a wait has ended without its data; the rest then runs without waits
+    auto exchange = [&](int i) {
+        const int par = i & 1;
+        bar_sync(kBarPart, nthr);
+        double s0 = 0.0, s1 = 0.0, t0 = 0.0, t1 = 0.0;
+        int g = 0;
+        for (; g + 1 < NW; g += 2) {
+            const double2 p0 = *reinterpret_cast<const double2 *>(&S.wpart[g][cp2]);
+            const double2 p1 = *reinterpret_cast<const double2 *>(&S.wpart[g + 1][cp2]);
+            s0 += p0.x;
+            t0 += p0.y;
+            s1 += p1.x;
+            t1 += p1.y;
+        }
+        if (g < NW) {
+            const double2 p0 = *reinterpret_cast<const double2 *>(&S.wpart[g][cp2]);
+            s0 += p0.x;
+            t0 += p0.y;
+        }
+        s0 += s1;
+        t0 += t1;
+        const unsigned mine = smem_u32(&S.cpart[par][rank][cp2]), bar = full0 + 8 * par;
+#pragma unroll
+        for (int u = 0; u < kCl / 2; ++u) st_async2(map_rank(mine, hc + u), s0, t0, map_rank(bar, hc + u));
+        if (rank == 0) {
+            const double2 pv = *reinterpret_cast<const double2 *>(&S.prow[cp2]);
+            const unsigned piv = smem_u32(&S.ppart[par][cp2]);
+#pragma unroll
+            for (int u = 0; u < kCl / 2; ++u) st_async2(map_rank(piv, hc + u), pv.x, pv.y, map_rank(bar, hc + u));
+        }
+        // Past the limit the error is recorded; the wait itself goes on to the default limit, so that
+        // stores of this column do not arrive in a CTA that has left.
+        unsigned long long spins = 0;
+        while (patient && !mbar_test_cta(bar, (i >> 1) & 1)) {
+            if (++spins == p.limit) atomicExch(p.err, (int)kDevBarrierTimeout);
+            if (spins > p.limit && spins > kPanelPolls) patient = false;
+        }
+        __syncwarp();
+        // for column i + 2, which nobody sends before our i + 1
+        if (lane == 0 && patient) mbar_expect(bar, kPanelBytes);
+        double q0 = 0.0, q1 = 0.0;
+#pragma unroll
+        for (int u = 0; u < kCl; u += 2) {
+            q0 += S.cpart[par][u][lane];
+            q1 += S.cpart[par][u + 1][lane];
+        }
+        const double q = q0 + q1, pc = S.ppart[par][lane];
+        const double alpha = __shfl_sync(kFull, pc, i), sig = __shfl_sync(kFull, q, i);
+        double tau = 0.0, beta = alpha, sc = 0.0;
+        if (sig != 0.0) {
+            beta = -copysign(sqrt(alpha * alpha + sig), alpha);
+            sc = 1.0 / (alpha - beta);
+            tau = (beta - alpha) / beta;
+        }
+        const double vq = fma(sc, q, pc);  // a_c^T v (c > i), V_c^T v (c < i)
+        S.w[lane] = (lane > i) ? tau * vq : 0.0;
+        if (lane == 0) {
+            S.sc = sc;
+            S.beta = beta;
+        }
+        bar_arrive(kBarRow, nthr);
+        if (rank == kCl - 1) {
+            // T[0:i, i] = -tau T[0:i, 0:i] z, T[i][i] = tau (dlarft, forward, columnwise)
+            S.z[lane] = (lane < i) ? vq : 0.0;
+            __syncwarp();
+            double r0 = 0.0, r1 = 0.0;
+            for (int c = 0; c < i; c += 2) {
+                r0 = fma(S.T[lane][c], S.z[c], r0);
+                r1 = fma(S.T[lane][c + 1], S.z[c + 1], r1);  // z[i] = 0
+            }
+            S.T[lane][i] = (lane < i) ? -tau * (r0 + r1) : (lane == i ? tau : 0.0);
+            __syncwarp();
+        }
+    };
+    if (!worker)
+        for (int i = 0; i < p.nr; ++i) exchange(i);
 #pragma unroll
     for (int ph = 0; ph < 4; ++ph) {
+        if (!worker) break;
         for (int ii = 0; ii < 8; ++ii) {
-            const int i = 8 * ph + ii, par = i & 1;
+            const int i = 8 * ph + ii;
             if (i >= p.nr) break;
             const int src = ii * 4 + rl;
             double x[8];
-            if (worker) {
-                double q4[4] = {0.0, 0.0, 0.0, 0.0};
+            double q4[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+            for (int kk = 0; kk < 8; ++kk) {
+                x[kk] = __shfl_sync(kFull, a[kk][ph], src);
+                if (top && 4 * kk + rl <= i) x[kk] = 0.0;
+            }
+#pragma unroll
+            for (int kk = 0; kk < 8; ++kk)
+#pragma unroll
+                for (int nt = 0; nt < 4; ++nt) q4[nt] = fma(x[kk], a[kk][nt], q4[nt]);
+            beyond([&](const double *B, int) {
 #pragma unroll
                 for (int kk = 0; kk < 8; ++kk) {
-                    x[kk] = __shfl_sync(kFull, a[kk][ph], src);
-                    if (top && 4 * kk + rl <= i) x[kk] = 0.0;
+                    const double xs = B[(kk * 4 + ph) * 32 + src];
+#pragma unroll
+                    for (int nt = 0; nt < 4; ++nt) q4[nt] = fma(xs, B[(kk * 4 + nt) * 32 + lane], q4[nt]);
                 }
+            });
+            // sums over the four row lanes: lane rl ends with column 8 rl + cl
+            const bool hi = rl & 2, od = rl & 1;
+            double u0 = hi ? q4[0] : q4[2], u1 = hi ? q4[1] : q4[3];
+            u0 = __shfl_xor_sync(kFull, u0, 2);
+            u1 = __shfl_xor_sync(kFull, u1, 2);
+            const double v0 = (hi ? q4[2] : q4[0]) + u0, v1 = (hi ? q4[3] : q4[1]) + u1;
+            const double s = (od ? v1 : v0) + __shfl_xor_sync(kFull, od ? v0 : v1, 1);
+            S.wpart[warp][8 * rl + cl] = s;
+            if (top && rl == (i & 3)) {
 #pragma unroll
-                for (int kk = 0; kk < 8; ++kk)
+                for (int nt = 0; nt < 4; ++nt) S.prow[8 * nt + cl] = (ii >> 2) ? a[2 * ph + 1][nt] : a[2 * ph][nt];
+            }
+            bar_arrive(kBarPart, nthr);
+            bar_sync(kBarRow, nthr);
+            const double sc = S.sc;
+            double wn[4];
 #pragma unroll
-                    for (int nt = 0; nt < 4; ++nt) q4[nt] = fma(x[kk], a[kk][nt], q4[nt]);
-                beyond([&](const double *B, int) {
+            for (int nt = ph; nt < 4; ++nt) wn[nt] = S.w[8 * nt + cl];
 #pragma unroll
-                    for (int kk = 0; kk < 8; ++kk) {
-                        const double xs = B[(kk * 4 + ph) * 32 + src];
+            for (int kk = 0; kk < 8; ++kk) {
+                const double v = sc * x[kk];
+                if (top && 4 * kk + rl <= i) {
+                    if (4 * kk + rl == i) {  // the pivot row
 #pragma unroll
-                        for (int nt = 0; nt < 4; ++nt) q4[nt] = fma(xs, B[(kk * 4 + nt) * 32 + lane], q4[nt]);
+                        for (int nt = ph; nt < 4; ++nt) a[kk][nt] -= wn[nt];
+                        if (cl == ii) a[kk][ph] = S.beta;
                     }
-                });
-                // sums over the four row lanes: lane rl ends with column 8 rl + cl
-                const bool hi = rl & 2, od = rl & 1;
-                double u0 = hi ? q4[0] : q4[2], u1 = hi ? q4[1] : q4[3];
-                u0 = __shfl_xor_sync(kFull, u0, 2);
-                u1 = __shfl_xor_sync(kFull, u1, 2);
-                const double v0 = (hi ? q4[2] : q4[0]) + u0, v1 = (hi ? q4[3] : q4[1]) + u1;
-                const double s = (od ? v1 : v0) + __shfl_xor_sync(kFull, od ? v0 : v1, 1);
-                S.wpart[warp][8 * rl + cl] = s;
-                if (top && rl == (i & 3)) {
+                } else {
 #pragma unroll
-                    for (int nt = 0; nt < 4; ++nt) S.prow[8 * nt + cl] = (ii >> 2) ? a[2 * ph + 1][nt] : a[2 * ph][nt];
+                    for (int nt = ph; nt < 4; ++nt) a[kk][nt] = fma(-v, wn[nt], a[kk][nt]);
+                    if (cl == ii) a[kk][ph] = v;
                 }
             }
-            __syncthreads();
-            if (warp == 0) {
-                double s0 = 0.0, s1 = 0.0, s2 = 0.0, s3 = 0.0;
-                int g = 0;
-                for (; g + 3 < NW; g += 4) {
-                    s0 += S.wpart[g][lane];
-                    s1 += S.wpart[g + 1][lane];
-                    s2 += S.wpart[g + 2][lane];
-                    s3 += S.wpart[g + 3][lane];
-                }
-                for (; g < NW; ++g) s0 += S.wpart[g][lane];
-                const double s = (s0 + s1) + (s2 + s3);
-                double *mine = &S.cpart[par][rank][lane], *piv = &S.ppart[par][lane];
-                const double pv = (rank == 0) ? S.prow[lane] : 0.0;
-#pragma unroll
-                for (int u = 0; u < kCl; ++u) {
-                    *cluster.map_shared_rank(mine, u) = s;
-                    if (rank == 0) *cluster.map_shared_rank(piv, u) = pv;
-                }
-            }
-            cluster.sync();
-            if (warp == 0) {
-                double q0 = 0.0, q1 = 0.0;
-#pragma unroll
-                for (int u = 0; u < kCl; u += 2) {
-                    q0 += S.cpart[par][u][lane];
-                    q1 += S.cpart[par][u + 1][lane];
-                }
-                const double q = q0 + q1, pc = S.ppart[par][lane];
-                const double alpha = __shfl_sync(kFull, pc, i), sig = __shfl_sync(kFull, q, i);
-                double tau = 0.0, beta = alpha, sc = 0.0;
-                if (sig != 0.0) {
-                    beta = -copysign(sqrt(alpha * alpha + sig), alpha);
-                    sc = 1.0 / (alpha - beta);
-                    tau = (beta - alpha) / beta;
-                }
-                const double vq = fma(sc, q, pc);  // a_c^T v (c > i), V_c^T v (c < i)
-                S.w[lane] = (lane > i) ? tau * vq : 0.0;
-                S.z[lane] = (lane < i) ? vq : 0.0;
-                if (lane == 0) {
-                    S.sc = sc;
-                    S.tau = tau;
-                    S.beta = beta;
-                }
-            }
-            __syncthreads();
-            if (worker) {
-                const double sc = S.sc;
-                double wn[4];
-#pragma unroll
-                for (int nt = ph; nt < 4; ++nt) wn[nt] = S.w[8 * nt + cl];
+            beyond([&](double *B, int) {
 #pragma unroll
                 for (int kk = 0; kk < 8; ++kk) {
-                    const double v = sc * x[kk];
-                    if (top && 4 * kk + rl <= i) {
-                        if (4 * kk + rl == i) {  // the pivot row
-#pragma unroll
-                            for (int nt = ph; nt < 4; ++nt) a[kk][nt] -= wn[nt];
-                            if (cl == ii) a[kk][ph] = S.beta;
-                        }
-                    } else {
-#pragma unroll
-                        for (int nt = ph; nt < 4; ++nt) a[kk][nt] = fma(-v, wn[nt], a[kk][nt]);
-                        if (cl == ii) a[kk][ph] = v;
-                    }
-                }
-                beyond([&](double *B, int) {
-#pragma unroll
-                    for (int kk = 0; kk < 8; ++kk) {
-                        const double v = sc * B[(kk * 4 + ph) * 32 + src];
-                        __syncwarp();
-#pragma unroll
-                        for (int nt = ph; nt < 4; ++nt) {
-                            double *e = B + (kk * 4 + nt) * 32 + lane;
-                            *e = (nt == ph && cl == ii) ? v : fma(-v, wn[nt], *e);
-                        }
-                    }
+                    const double v = sc * B[(kk * 4 + ph) * 32 + src];
                     __syncwarp();
-                });
-            } else if (rank == kCl - 1) {
-                // T[0:i, i] = -tau T[0:i, 0:i] z, T[i][i] = tau (dlarft, forward, columnwise)
-                const double tau = S.tau;
-                double s0 = 0.0, s1 = 0.0;
-                for (int c = 0; c < i; c += 2) {
-                    s0 = fma(S.T[lane][c], S.z[c], s0);
-                    s1 = fma(S.T[lane][c + 1], S.z[c + 1], s1);  // z[i] = 0
+#pragma unroll
+                    for (int nt = ph; nt < 4; ++nt) {
+                        double *e = B + (kk * 4 + nt) * 32 + lane;
+                        *e = (nt == ph && cl == ii) ? v : fma(-v, wn[nt], *e);
+                    }
                 }
-                S.T[lane][i] = (lane < i) ? -tau * (s0 + s1) : (lane == i ? tau : 0.0);
                 __syncwarp();
-            }
+            });
         }
     }
     __syncthreads();
@@ -495,7 +537,9 @@ constexpr int kPS = 36;       // column stride of the 32-row ones
 constexpr size_t kWSmem = (size_t)(3 * 32 * kWS + 5 * 32 * kPS) * sizeof(double);
 
 // 64 rows a CTA: W = X T + V M (also for the first 32 rows, which every CTA needs), then the
-// next panel P = A2[:, 0:32] - V W_p^T - W V_p^T, W_p and V_p their first 32 rows.
+// next panel P = A2[:, 0:32] - V W_p^T - W V_p^T, W_p and V_p their first 32 rows. Bound by the
+// latency of its loads, which therefore all leave at once: 7.6 us a launch on average from 3968 rows
+// down (24 with loads of 8 bytes a few at a time).
 __global__ void __launch_bounds__(kThr) w_kernel(double *VWV, long long ldv, const double *X, long long ldx, const double *T,
                                                  const double *M, int R, const double *A2, long long lda, double *P,
                                                  long long ldp) {
@@ -504,18 +548,31 @@ __global__ void __launch_bounds__(kThr) w_kernel(double *VWV, long long ldv, con
     double *Xp = Ws + 32 * kWS, *Vp = Xp + 32 * kPS, *Wp = Vp + 32 * kPS, *Tm = Wp + 32 * kPS, *Mm = Tm + 32 * kPS;
     const int i0 = blockIdx.x * kBM;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, r = lane >> 2, c = lane & 3;
-    for (int q = tid; q < 32 * 64; q += kThr) {
-        const int j = q >> 6, i = q & 63;
-        Xs[j * kWS + i] = (i0 + i < R) ? X[(size_t)j * ldx + i0 + i] : 0.0;
-        Vs[j * kWS + i] = (i0 + i < R) ? VWV[(size_t)j * ldv + i0 + i] : 0.0;
+    // everything is asked for before anything is waited for
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+        const int e = tid + q * kThr, j = e >> 5, i = (e & 31) * 2, valid = min(max(R - i0 - i, 0), 2);
+        cp16(Xs + j * kWS + i, valid ? X + (size_t)j * ldx + i0 + i : X, valid * 8);
+        cp16(Vs + j * kWS + i, valid ? VWV + (size_t)j * ldv + i0 + i : VWV, valid * 8);
     }
-    for (int q = tid; q < 1024; q += kThr) {
-        const int j = q >> 5, i = q & 31;
-        Xp[j * kPS + i] = (i < R) ? X[(size_t)j * ldx + i] : 0.0;
-        Vp[j * kPS + i] = (i < R) ? VWV[(size_t)j * ldv + i] : 0.0;
-        Tm[j * kPS + i] = T[q];
-        Mm[j * kPS + i] = M[q];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        const int e = tid + q * kThr, j = e >> 4, i = (e & 15) * 2, valid = min(max(R - i, 0), 2);
+        cp16(Xp + j * kPS + i, valid ? X + (size_t)j * ldx + i : X, valid * 8);
+        cp16(Vp + j * kPS + i, valid ? VWV + (size_t)j * ldv + i : VWV, valid * 8);
+        cp16(Tm + j * kPS + i, T + 32 * j + i, 16);
+        cp16(Mm + j * kPS + i, M + 32 * j + i, 16);
     }
+    asm volatile("cp.async.commit_group;\n" ::);
+    double old[4][4];
+#pragma unroll
+    for (int b = 0; b < 4; ++b)
+#pragma unroll
+        for (int h = 0; h < 4; ++h) {
+            const int i = i0 + warp * 16 + r + 8 * (h >> 1), j = b * 8 + c * 2 + (h & 1);
+            old[b][h] = (i < R && i >= j) ? A2[(size_t)j * lda + i] : 0.0;
+        }
+    asm volatile("cp.async.wait_group 0;\n" ::);
     __syncthreads();
     // acc (16 rows m0.. of [column][row] tiles with stride s, nt column tiles from n0) += Lh Rh,
     // Lh(m, k) = L[k s + m], Rh(k, n) = B[n kPS + k] (bt: B[k kPS + n])
@@ -565,7 +622,7 @@ __global__ void __launch_bounds__(kThr) w_kernel(double *VWV, long long ldv, con
 #pragma unroll
         for (int h = 0; h < 4; ++h) {
             const int i = i0 + warp * 16 + r + 8 * (h >> 1), j = b * 8 + c * 2 + (h & 1);
-            if (i < R && i >= j) P[(size_t)j * ldp + i] = A2[(size_t)j * lda + i] - acc[b][h];
+            if (i < R && i >= j) P[(size_t)j * ldp + i] = old[b][h] - acc[b][h];
         }
 }
 
@@ -708,23 +765,39 @@ bool band_reduce_available() {
 
 size_t band_reduce_work_doubles(int n) {
     const size_t ld = (size_t)rup(n, 8);
-    return ld * (96 + 32 + 32) + 1024 + PanelPlan(n).spill_doubles();
+    return ld * (2 * 96 + 32 + 32) + 1024 + PanelPlan(n).spill_doubles();
 }
 
 cudaError_t launch_band_reduce(const BandReduce &b, cudaStream_t st) {
     const int n = b.n;
     const long long ld = rup(n, 8);
-    double *VWV = b.work, *X = VWV + 96 * ld, *P = X + 32 * ld, *M = P + 32 * ld;
+    double *X = b.work + 2 * 96 * ld, *P = X + 32 * ld, *M = P + 32 * ld;
     if (!band_reduce_available()) return cudaErrorNotSupported;
     cudaError_t e;
     if ((e = cudaMemsetAsync(b.C, 0, band_storage_doubles(n) * sizeof(double), st)) != cudaSuccess) return e;
     int dev = 0, nsm = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+    // The panel needs only what w_kernel has made of its columns, so panel j + 1 runs beside the
+    // update of step j, which goes to the side stream; V W V alternates between two buffers. Whichever
+    // way this function is left, `st` waits for the side stream.
+    struct Join {
+        const BandReduce &b;
+        cudaStream_t st;
+        bool open = false;
+        cudaError_t close() {
+            if (!open) return cudaSuccess;
+            open = false;
+            const cudaError_t e = cudaEventRecord(b.done, b.side);
+            return e == cudaSuccess ? cudaStreamWaitEvent(st, b.done, 0) : e;
+        }
+        ~Join() { close(); }
+    } update{b, st};
     DVR3D_COUNT_LAUNCH(1);
     copy_panel_kernel<<<(unsigned)(((long long)n * kB + 255) / 256), 256, 0, st>>>(b.A, b.lda, n, std::min(kB, n), P, ld);
     for (int j0 = 0; j0 < n; j0 += kB) {
         const int R = std::max(0, n - j0 - kB);
+        double *VWV = b.work + (j0 / kB & 1) * 96 * ld;
         PanelArgs pa{};
         pa.P = P;
         pa.ldp = ld;
@@ -741,12 +814,15 @@ cudaError_t launch_band_reduce(const BandReduce &b, cudaStream_t st) {
         const PanelPlan pp(R);
         pa.nsm = pp.nsm;
         pa.spill = M + 1024;
+        pa.err = b.err;
+        pa.limit = b.wait_limit ? b.wait_limit : kPanelPolls;
         {
             ClusterLaunch l(dim3(kCl), (pp.warps + 1) * 32, pp.smem, kCl, 1, st);
             DVR3D_COUNT_LAUNCH(1);
             if ((e = cudaLaunchKernelEx(&l.cfg, panel_qr_kernel, pa)) != cudaSuccess) return e;
         }
         if (R == 0) break;
+        if ((e = update.close()) != cudaSuccess) return e;
         double *A2 = b.A + (size_t)(j0 + kB) * b.lda + j0 + kB;
         if (pa.nr == 0) {  // one row left: it lies in the band
             DVR3D_COUNT_LAUNCH(1);
@@ -787,13 +863,16 @@ cudaError_t launch_band_reduce(const BandReduce &b, cudaStream_t st) {
         const int R2 = R - kB;
         if (R2 > 0) {
             const long long nt = (R2 + 63) / 64;
+            if ((e = cudaEventRecord(b.ready, st)) != cudaSuccess || (e = cudaStreamWaitEvent(b.side, b.ready, 0)) != cudaSuccess)
+                return e;
+            update.open = true;
             DVR3D_COUNT_LAUNCH(1);
-            syr2k_band_kernel<<<(unsigned)(nt * (nt + 1) / 2), kThr, kSyrSmem, st>>>(A2 + (size_t)kB * b.lda + kB, b.lda, R2,
-                                                                                  VWV + kB, ld);
+            syr2k_band_kernel<<<(unsigned)(nt * (nt + 1) / 2), kThr, kSyrSmem, b.side>>>(A2 + (size_t)kB * b.lda + kB, b.lda, R2,
+                                                                                      VWV + kB, ld);
             if ((e = cudaGetLastError()) != cudaSuccess) return e;
         }
     }
-    return cudaSuccess;
+    return update.close();
 }
 
 size_t band_reduce_back_doubles(int nev) { return (size_t)2 * kB * nev + gemm_splitk_work(kB, nev, 64); }

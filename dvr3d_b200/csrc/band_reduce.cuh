@@ -17,6 +17,10 @@ struct BandReduce {
                        // (band_storage_doubles(n))
     double *T;         // [band_reduce_panels(n)][32 x 32] triangular factors
     double *work;      // band_reduce_work_doubles(n)
+    cudaStream_t side; // the updates run here, beside the panels; joined before the call's last work on st
+    cudaEvent_t ready, done;  // of the caller's, timing disabled
+    int *err;          // cleared by the caller; set to kDevBarrierTimeout when a wait runs out
+    unsigned long long wait_limit;  // polls of a wait, 0: the default
 };
 
 // Whether the current device takes the panel kernel's cluster.

@@ -162,6 +162,9 @@ void dvr3d_b200_destroy(dvr3d_ctx *ctx) {
     for (auto &e : ctx->ev)
         if (e) cudaEventDestroy(e);
     for (auto &e : ctx->panel_ev) cudaEventDestroy(e);
+    for (auto &e : ctx->side_ev)
+        if (e) cudaEventDestroy(e);
+    if (ctx->side_stream) cudaStreamDestroy(ctx->side_stream);
     for (auto &e : ctx->gemm_ev) cudaEventDestroy(e);
     for (auto &g : ctx->graphs)
         if (g.second.exec) cudaGraphExecDestroy(g.second.exec);

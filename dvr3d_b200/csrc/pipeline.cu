@@ -651,6 +651,16 @@ void dense_lowest_two_stage(dvr3d_ctx *ctx, double *A, long long lda, int n, int
     br.C = ctx->arena.get_t<double>(t + "bandC", band_storage_doubles(n));
     br.T = ctx->arena.get_t<double>(t + "bandT", (size_t)band_reduce_panels(n) * kBandMaxBw * kBandMaxBw);
     br.work = ctx->arena.get_t<double>(t + "bandwork", band_reduce_work_doubles(n));
+    if (!ctx->side_stream) {
+        CK(cudaStreamCreateWithFlags(&ctx->side_stream, cudaStreamNonBlocking));
+        for (auto &e : ctx->side_ev) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+    }
+    br.side = ctx->side_stream;
+    br.ready = ctx->side_ev[0];
+    br.done = ctx->side_ev[1];
+    br.err = ctx->arena.get_t<int>(t + "err", 1);
+    br.wait_limit = ctx->wait_limit;
+    CK(cudaMemsetAsync(br.err, 0, sizeof(int), st));
     if (time_panels) CK(cudaEventRecord(ctx->panel_ev[0], st));
     const long long launches0 = g_kernel_launches;
     CK(launch_band_reduce(br, st));
@@ -668,9 +678,8 @@ void dense_lowest_two_stage(dvr3d_ctx *ctx, double *A, long long lda, int n, int
         bt.taus = ctx->arena.get_t<double>(t + "bandtau", band_tau_doubles(n, bt.b));
     }
     bt.progress = ctx->arena.get_t<unsigned int>(t + "bandprog", n);
-    bt.err = ctx->arena.get_t<int>(t + "err", 1);
+    bt.err = br.err;
     bt.wait_limit = ctx->wait_limit;
-    CK(cudaMemsetAsync(bt.err, 0, sizeof(int), st));
     CK(launch_band_chase(bt, st));
     double *e2s = ctx->arena.get_t<double>(t + "e2", n);
     double *info = ctx->arena.get_t<double>(t + "info", 4);

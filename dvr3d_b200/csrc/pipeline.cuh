@@ -62,6 +62,8 @@ struct dvr3d_ctx {
     cudaEvent_t ev[8] = {};
     int sm_count = 0;
     int dense_grid = 0;
+    cudaStream_t side_stream = nullptr;  // of the dense reduction's updates, made on first use
+    cudaEvent_t side_ev[2] = {};
     std::vector<cudaEvent_t> panel_ev;  // timing pool for the reduction panels
     unsigned long long wait_limit = 0;  // polls of each bounded device wait (0: kernel defaults)
     std::vector<cudaEvent_t> gemm_ev;   // timing pool of the GEMM launches of an iterative solve
