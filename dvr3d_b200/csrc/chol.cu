@@ -24,7 +24,6 @@ namespace dvr3d {
 namespace {
 
 constexpr int NB = kCholNb;
-constexpr int kLeafThreads = 256;
 
 __global__ void shift_copy_lower_kernel(const double *H, long long ldh, int n, double sigma, double *A,
                                         long long lda) {
@@ -37,34 +36,38 @@ __global__ void shift_copy_lower_kernel(const double *H, long long ldh, int n, d
     A[(size_t)j * lda + i] = v;
 }
 
-// Cholesky of the nb x nb block at (j0, j0) (nb <= 64, lower triangle read) and inverse of
-// its factor. in_place_inv = 0: the factor goes back into A; 1: the inverse replaces the
-// block's lower triangle. inv_out (optional): the inverse (ld 64, zeros above).
-// One right-looking sweep forms A = U D U^T (U unit lower) and, in the same steps, the
-// forward substitution X = inv(U) (row k of X is final when step k starts; step k
-// subtracts U[i][k] X[k] from the rows below); then L = U D^{1/2}, inv(L) = D^{-1/2} X.
-// Thread (row ti, group tg) keeps columns 16 tg .. 16 tg + 15 of the matrix and of X in
-// registers. The pivot column is published with zeros on and above the diagonal and row k
-// of X has zeros right of its diagonal, so every step is the same 32 unmasked FMAs per
-// thread (finished columns and the upper triangle take zero updates); one barrier per step.
-__global__ void __launch_bounds__(kLeafThreads, 1) potrf_leaf_kernel(double *A, long long lda, int j0, int nb,
-                                                                     double *inv_out, int in_place_inv,
-                                                                     double rel_tol, int *err) {
+// Cholesky of the nb x nb block A (nb <= N, lower triangle read) and inverse of its factor.
+// in_place_inv = 0: the factor goes back into A; 1: the inverse replaces the block's lower triangle.
+// inv_out (optional): the inverse (NB x NB, zeros above the diagonal and beyond nb).
+// One right-looking sweep forms A = U D U^T (U unit lower) and, in the same steps, the forward
+// substitution X = inv(U) (row k of X is final when step k starts; step k subtracts U[i][k] X[k]
+// from the rows below); then L = U D^{1/2}, inv(L) = D^{-1/2} X.
+// Thread (row ti, group tg) keeps W columns of the matrix and of X in registers. The pivot column is
+// published with zeros on and above the diagonal and row k of X has zeros right of its diagonal, so
+// the FMAs need no masks; a warp leaves out those that are zero for all of it (rows down to the
+// pivot, the matrix's columns up to it, X's beyond it).
+// A step is a chain (pivot's update, its reciprocal, a barrier, the column back from shared memory),
+// so a thread holds few columns (eight at N = 64, four at 32), the pivot's group forms and publishes
+// the next column before its share of X, and what else there is to do fits beside it. A leaf of 64
+// takes 25 us (36 with sixteen columns of each a thread and every FMA done), a block of up to 32 in
+// 32 rows 13 us (25 in one warp that broadcasts by shuffles).
+template <int N, int W>
+__global__ void __launch_bounds__(N *(N / W), 1) potrf_leaf_kernel(double *A, long long lda, int nb, double *inv_out,
+                                                                   int in_place_inv, double rel_tol, int *err) {
     if (*(volatile int *)err != 0) return;
-    __shared__ __align__(16) double colb[2][NB];
-    __shared__ __align__(16) double rowb[2][NB];
+    __shared__ __align__(16) double colb[2][N];
+    __shared__ __align__(16) double rowb[2][N];
     __shared__ double piv[2], rdb[2];
-    __shared__ double sq[NB], rsq[NB];
+    __shared__ double sq[N], rsq[N];
     __shared__ double s_thr;
     const int tid = threadIdx.x;
-    const int ti = tid & (NB - 1), tg = tid >> 6;
-    constexpr int U = NB / 4;
-    const int jb = tg * U;
-    double own[U], x[U];
+    const int ti = tid & (N - 1), tg = tid / N;
+    const int jb = tg * W, below = ti | 31;  // the warp's last row
+    double own[W], x[W];
 #pragma unroll
-    for (int u = 0; u < U; ++u) {
+    for (int u = 0; u < W; ++u) {
         const int j = jb + u;
-        own[u] = (ti < nb && j < nb && ti >= j) ? A[(size_t)(j0 + j) * lda + j0 + ti] : 0.0;
+        own[u] = (ti < nb && j < nb && ti >= j) ? A[(size_t)j * lda + ti] : 0.0;
         x[u] = (ti == j) ? 1.0 : 0.0;
         if (ti == j) sq[ti] = own[u];  // diagonal, for the pivot threshold
         if (ti == 0) rowb[0][j] = x[u];
@@ -85,52 +88,50 @@ __global__ void __launch_bounds__(kLeafThreads, 1) potrf_leaf_kernel(double *A, 
         if (tid == 0) s_thr = rel_tol * mx;
     }
     bool bad = false;
-    for (int k = 0; k < nb; ++k) {
-        const int cb = k & 1, nbuf = cb ^ 1;
+#pragma unroll 1
+    for (int k0 = 0; k0 < nb && !bad; k0 += W)
+#pragma unroll
+    for (int kk = 0; kk < W; ++kk) {
+        const int k = k0 + kk, cb = kk & 1, nbuf = cb ^ 1, kn = k + 1;
+        if (k >= nb || bad) break;
         __syncthreads();
         const double d = piv[cb];
-        if (!(d > s_thr) || !isfinite(d)) {  // uniform: every thread reads the same d
-            bad = true;
-            break;
-        }
+        bad = !(d > s_thr) || !isfinite(d);  // uniform: every thread reads the same d
+        if (bad || below <= k) continue;
         const double lik = colb[cb][ti] * rdb[cb];  // zero on and above the pivot
-        double cv[U], rv[U];
+        if (jb + W - 1 > k) {
+            double cv[W];
 #pragma unroll
-        for (int u = 0; u < U; u += 2) {
-            const double2 c2 = *reinterpret_cast<const double2 *>(&colb[cb][jb + u]);
-            const double2 r2 = *reinterpret_cast<const double2 *>(&rowb[cb][jb + u]);
-            cv[u] = c2.x;
-            cv[u + 1] = c2.y;
-            rv[u] = r2.x;
-            rv[u + 1] = r2.y;
-        }
+            for (int u = 0; u < W; u += 2) {
+                const double2 c2 = *reinterpret_cast<const double2 *>(&colb[cb][jb + u]);
+                cv[u] = c2.x;
+                cv[u + 1] = c2.y;
+            }
 #pragma unroll
-        for (int u = 0; u < U; ++u) {
-            own[u] = fma(-lik, cv[u], own[u]);
-            x[u] = fma(-lik, rv[u], x[u]);
+            for (int u = 0; u < W; ++u) own[u] = fma(-lik, cv[u], own[u]);
+            if (tg == kn / W) {  // column k+1 is final after this step
+                const double v = own[(kk + 1) % W];
+                if (ti == kn) {
+                    piv[nbuf] = v;
+                    rdb[nbuf] = 1.0 / v;
+                }
+                colb[nbuf][ti] = (ti > kn) ? v : 0.0;
+            }
         }
-        const int kn = k + 1;
-        if (tg == (kn >> 4) && kn < NB) {  // column k+1 is final after this step
-            double v = 0.0;
-            switch (kn & 15) {
-#define DVR3D_PICK(c) \
-    case c:           \
-        v = own[c];   \
-        break;
-                DVR3D_PICK(0) DVR3D_PICK(1) DVR3D_PICK(2) DVR3D_PICK(3) DVR3D_PICK(4) DVR3D_PICK(5) DVR3D_PICK(6)
-                DVR3D_PICK(7) DVR3D_PICK(8) DVR3D_PICK(9) DVR3D_PICK(10) DVR3D_PICK(11) DVR3D_PICK(12)
-                DVR3D_PICK(13) DVR3D_PICK(14) DVR3D_PICK(15)
-#undef DVR3D_PICK
+        if (jb <= k) {
+            double rv[W];
+#pragma unroll
+            for (int u = 0; u < W; u += 2) {
+                const double2 r2 = *reinterpret_cast<const double2 *>(&rowb[cb][jb + u]);
+                rv[u] = r2.x;
+                rv[u + 1] = r2.y;
             }
-            colb[nbuf][ti] = (ti > kn) ? v : 0.0;
-            if (ti == kn) {
-                piv[nbuf] = v;
-                rdb[nbuf] = 1.0 / v;
-            }
+#pragma unroll
+            for (int u = 0; u < W; ++u) x[u] = fma(-lik, rv[u], x[u]);
         }
         if (ti == kn) {  // so is row k+1 of X
 #pragma unroll
-            for (int u = 0; u < U; ++u) rowb[nbuf][jb + u] = x[u];
+            for (int u = 0; u < W; ++u) rowb[nbuf][jb + u] = x[u];
         }
     }
     if (bad) {
@@ -141,7 +142,7 @@ __global__ void __launch_bounds__(kLeafThreads, 1) potrf_leaf_kernel(double *A, 
     // inv(L) = D^{-1/2} X
     __syncthreads();
 #pragma unroll
-    for (int u = 0; u < U; ++u) {
+    for (int u = 0; u < W; ++u) {
         const int j = jb + u;
         if (ti == j && ti < nb) {
             const double r = sqrt(own[u]);
@@ -152,88 +153,22 @@ __global__ void __launch_bounds__(kLeafThreads, 1) potrf_leaf_kernel(double *A, 
     __syncthreads();
     const double rrow = (ti < nb) ? rsq[ti] : 0.0;
 #pragma unroll
-    for (int u = 0; u < U; ++u) {
+    for (int u = 0; u < W; ++u) {
         const int j = jb + u;
         const bool in = (ti < nb && j < nb && ti >= j);
-        const double l = (ti == j) ? sq[j] : own[u] * rsq[j];
-        const double xi = x[u] * rrow;
-        if (in) A[(size_t)(j0 + j) * lda + j0 + ti] = in_place_inv ? xi : l;
-        if (inv_out) inv_out[(size_t)j * NB + ti] = in ? xi : 0.0;
+        if (in) A[(size_t)j * lda + ti] = in_place_inv ? x[u] * rrow : ((ti == j) ? sq[j] : own[u] * rsq[j]);
+        if (inv_out) inv_out[(size_t)j * NB + ti] = in ? x[u] * rrow : 0.0;
     }
+    if (N < NB && inv_out)
+        for (int q = tid; q < NB * NB; q += blockDim.x)
+            if (q / NB >= N || q % NB >= N) inv_out[q] = 0.0;
 }
 
-// Cholesky and inverse of a b x b block (b <= 32) in one warp: lane i keeps row i of the
-// matrix and of X = inv(U) in registers; step k broadcasts the pivot and column k / row k
-// by shuffles (no barriers). Same results as the leaf kernel: G's lower triangle receives
-// L, inv_out (ld 64) the inverse with zeros above the diagonal.
-__global__ void __launch_bounds__(32) chol_warp_kernel(double *G, int b, double *inv_out, double rel_tol, int *err) {
-    if (*(volatile int *)err != 0) return;
-    const int i = threadIdx.x;
-    constexpr unsigned kAll = 0xffffffffu;
-    double own[32], x[32];
-#pragma unroll
-    for (int c = 0; c < 32; ++c) {
-        own[c] = (i < b && c < b && c <= i) ? G[(size_t)c * b + i] : 0.0;
-        x[c] = (c == i) ? 1.0 : 0.0;
-    }
-    double dmax = 0.0;
-#pragma unroll
-    for (int c = 0; c < 32; ++c)
-        if (c == i) dmax = own[c];
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) dmax = fmax(dmax, __shfl_xor_sync(kAll, dmax, o));
-    const double thr = rel_tol * dmax;
-    // the step loop stays a loop (a fully unrolled one is too long for the instruction cache);
-    // column k of this lane's row is picked by selects, the other rows' entries by shuffles
-    bool bad = false;
-#pragma unroll 1
-    for (int k = 0; k < b; ++k) {
-        double colk = 0.0;
-#pragma unroll
-        for (int c = 0; c < 32; ++c) colk = (c == k) ? own[c] : colk;
-        const double d = __shfl_sync(kAll, colk, k);
-        if (!(d > thr) || !isfinite(d)) {  // uniform: every lane holds the same d
-            bad = true;
-            break;
-        }
-        const double lik = (i > k && i < b) ? colk * (1.0 / d) : 0.0;
-#pragma unroll
-        for (int c = 0; c < 32; ++c) {
-            const double ack = __shfl_sync(kAll, colk, c);  // row c's entry of column k
-            own[c] -= (c > k) ? lik * ack : 0.0;
-            x[c] -= lik * __shfl_sync(kAll, x[c], k);      // row k of X (zero right of k)
-        }
-    }
-    if (bad) {
-        if (i == 0) atomicExch(err, (int)kDevNotPosDef);
-        return;
-    }
-    double di = 0.0;
-#pragma unroll
-    for (int c = 0; c < 32; ++c)
-        if (c == i) di = own[c];
-    const double sq = (i < b) ? sqrt(di) : 1.0;
-    const double rs = 1.0 / sq;
-#pragma unroll
-    for (int c = 0; c < 32; ++c) {
-        const double rsc = __shfl_sync(kAll, rs, c);
-        const double sqc = __shfl_sync(kAll, sq, c);
-        const bool in = (i < b && c < b && c <= i);
-        if (in) G[(size_t)c * b + i] = (c == i) ? sqc : own[c] * rsc;
-        if (inv_out && c < 64) inv_out[(size_t)c * NB + i] = in ? x[c] * rs : 0.0;
-    }
-    if (inv_out) {  // rows b..63 of the 64-row inverse block stay zero
-        for (int q = i; q < NB * NB; q += 32) {
-            const int c = q / NB, r = q % NB;
-            if (r >= 32 || c >= 32) inv_out[q] = 0.0;
-        }
-    }
-}
-
-cudaError_t leaf(double *A, long long lda, int j0, int nb, double *inv_out, int in_place, double rel_tol, int *err,
+cudaError_t leaf(double *A, long long lda, int nb, double *inv_out, int in_place, double rel_tol, int *err,
                  cudaStream_t st) {
     DVR3D_COUNT_LAUNCH(1);
-    potrf_leaf_kernel<<<1, kLeafThreads, 0, st>>>(A, lda, j0, nb, inv_out, in_place, rel_tol, err);
+    if (nb <= 32) potrf_leaf_kernel<32, 4><<<1, 256, 0, st>>>(A, lda, nb, inv_out, in_place, rel_tol, err);
+    else potrf_leaf_kernel<NB, 8><<<1, 512, 0, st>>>(A, lda, nb, inv_out, in_place, rel_tol, err);
     return cudaGetLastError();
 }
 
@@ -279,7 +214,7 @@ struct Rec {
 
     cudaError_t run(int off, int n, double *sp) {
         cudaError_t e;
-        if (n <= NB) return leaf(A, lda, off, n, nullptr, 1, 0.0, err, st);
+        if (n <= NB) return leaf(A + (size_t)off * lda + off, lda, n, nullptr, 1, 0.0, err, st);
         int n1 = ((n / 2 + NB - 1) / NB) * NB;
         if (n1 >= n) n1 = n - NB;
         const int n2 = n - n1;
@@ -407,12 +342,7 @@ cudaError_t launch_potrf_inv_lower(double *A, long long lda, int n, double *work
 
 cudaError_t launch_chol_small(double *G, int b, double *ginv, double rel_tol, int *err, cudaStream_t st) {
     if (b > NB) return cudaErrorInvalidValue;
-    if (b <= 32) {
-        DVR3D_COUNT_LAUNCH(1);
-        chol_warp_kernel<<<1, 32, 0, st>>>(G, b, ginv, rel_tol, err);
-        return cudaGetLastError();
-    }
-    return leaf(G, b, 0, b, ginv, 0, rel_tol, err, st);
+    return leaf(G, b, b, ginv, 0, rel_tol, err, st);
 }
 
 }  // namespace dvr3d
