@@ -587,11 +587,15 @@ __global__ void band_slots_kernel(const double *A, long long lda, int n, int b, 
 // Back-transformation, COLS eigenvector columns per CTA held in shared memory (column c at
 // zs + c ldzs, ldzs = 1 mod 16 so the lanes' rows and columns spread over the banks).
 // Sweeps are applied last first; the tasks of one sweep act on disjoint rows and are split
-// over the 8 warps (task w + 8 k of a chunk of kChunkTasks). In a warp, lane (rg, c) takes
+// over the warps (task w + kBtWarps k of a chunk of kChunkTasks). In a warp, lane (rg, c) takes
 // column c and rows COLS rg .. COLS rg + COLS - 1 of the reflector's window: COLS products,
 // a shuffle sum over the 32 / COLS row groups, COLS updates. The reflectors of the next
 // chunk are copied into shared memory (cp.async) while the current chunk is applied.
+// A task is a chain of loads, products, shuffles and stores (some 250 cycles), and a sweep a few of
+// them and a barrier; so a warp takes several tasks at once, loads first.
+// 500 vectors of order 2656 take 1.75 ms (2.1 with two columns a CTA and a task at a time).
 constexpr int kChunkTasks = 96;
+constexpr int kBtWarps = 8;
 
 __device__ __forceinline__ void cp_async8(double *dst, const double *src) {
     const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
@@ -599,7 +603,7 @@ __device__ __forceinline__ void cp_async8(double *dst, const double *src) {
 }
 
 template <int COLS>
-__global__ void __launch_bounds__(256) band_bt_kernel(BandTri t, double *Z, long long ldz, int nev, int ldzs) {
+__global__ void __launch_bounds__(32 * kBtWarps) band_bt_kernel(BandTri t, double *Z, long long ldz, int nev, int ldzs) {
     extern __shared__ double sm[];
     double *zs = sm;
     double *vb = sm + (size_t)COLS * ldzs;       // [2][kChunkTasks][kBW]
@@ -639,27 +643,34 @@ __global__ void __launch_bounds__(256) band_bt_kernel(BandTri t, double *Z, long
         const double *vd = vb + (size_t)cbuf * kChunkTasks * kBW;
         const double *td = tb + cbuf * kChunkTasks;
         const int nt = band_ntask(n, b, cj);
-        for (int s = cbase + warp; s < nt && s < cbase + kChunkTasks; s += 8) {
-            const double tau = td[s - cbase];
-            if (tau == 0.0) continue;
-            const int r0 = cj + 1 + s * b;
-            const double *v = vd + (size_t)(s - cbase) * kBW + rg * COLS;
-            double vv[COLS], zz[COLS];
-            double part = 0.0;
+        constexpr int U = COLS < 8 ? 3 : 2;  // tasks at once; kBtWarps U divides kChunkTasks
+        const int send = min(nt, cbase + kChunkTasks);
+        for (int s0 = cbase + warp; s0 < send; s0 += kBtWarps * U) {
+            double tau[U], vv[U][COLS], zz[U][COLS], part[U];
 #pragma unroll
-            for (int i = 0; i < COLS; ++i) {
-                const int r = min(r0 + rg * COLS + i, n - 1);
-                vv[i] = v[i];
-                zz[i] = zs[(size_t)cc * ldzs + r];
-                part += vv[i] * zz[i];
+            for (int u = 0; u < U; ++u) {
+                const int s = s0 + kBtWarps * u, r0 = cj + 1 + s * b + rg * COLS;
+                tau[u] = (s < send) ? td[s - cbase] : 0.0;
+                const double *v = vd + (size_t)(s - cbase) * kBW + rg * COLS;
+                part[u] = 0.0;
+#pragma unroll
+                for (int i = 0; i < COLS; ++i) {
+                    vv[u][i] = (tau[u] != 0.0) ? v[i] : 0.0;
+                    zz[u][i] = zs[(size_t)cc * ldzs + min(r0 + i, n - 1)];
+                    part[u] += vv[u][i] * zz[u][i];
+                }
             }
 #pragma unroll
-            for (int o = COLS; o < 32; o <<= 1) part += __shfl_xor_sync(kFull, part, o);
-            const double f = tau * part;
+            for (int o = COLS; o < 32; o <<= 1)
 #pragma unroll
-            for (int i = 0; i < COLS; ++i) {
-                const int r = r0 + rg * COLS + i;
-                if (vv[i] != 0.0 && r < n) zs[(size_t)cc * ldzs + r] = zz[i] - f * vv[i];
+                for (int u = 0; u < U; ++u) part[u] += __shfl_xor_sync(kFull, part[u], o);
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const int r0 = cj + 1 + (s0 + kBtWarps * u) * b + rg * COLS;
+                const double f = tau[u] * part[u];
+#pragma unroll
+                for (int i = 0; i < COLS; ++i)
+                    if (vv[u][i] != 0.0 && r0 + i < n) zs[(size_t)cc * ldzs + r0 + i] = zz[u][i] - f * vv[u][i];
             }
         }
     }
@@ -675,7 +686,7 @@ cudaError_t launch_bt(const BandTri &t, double *Z, long long ldz, int nev, int l
     cudaError_t e = cudaFuncSetAttribute(band_bt_kernel<COLS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     DVR3D_COUNT_LAUNCH(1);
-    band_bt_kernel<COLS><<<(unsigned)((nev + COLS - 1) / COLS), 256, smem, st>>>(t, Z, ldz, nev, ldzs);
+    band_bt_kernel<COLS><<<(unsigned)((nev + COLS - 1) / COLS), 32 * kBtWarps, smem, st>>>(t, Z, ldz, nev, ldzs);
     return cudaGetLastError();
 }
 
@@ -758,10 +769,20 @@ cudaError_t launch_band_backtransform(const BandTri &t, double *Z, long long ldz
     const int ldzs = (t.n + 15) / 16 * 16 + 1;
     const size_t fixed = (size_t)2 * kChunkTasks * (kBW + 1) * sizeof(double);
     auto need = [&](int cols) { return fixed + (size_t)cols * ldzs * sizeof(double); };
-    // widest slab that fits, but no wider than keeps every SM busy
-    int cols = 8;
-    while (cols > 1 && (need(cols) > (size_t)optin || (nev + cols - 1) / cols < nsm)) cols /= 2;
-    if (need(cols) > (size_t)optin) return cudaErrorInvalidValue;
+    // The kernel is bound by shared memory: a reflector costs a slab of 1, 2, 4, 8 columns some 16, 20,
+    // 30, 52 passes over it (loads, stores, shuffles), slabs on one SM add up. The width with the
+    // fewest passes on the fullest SM: 500 columns in slabs of 4, on 125 SMs (1.9 ms for order 2656; in slabs of 2 2.1),
+    // 100 columns one each.
+    static const int pass[4] = {16, 20, 30, 52};
+    int cols = 0, best = 0;
+    for (int q = 0; q < 4; ++q) {
+        const int c = 1 << q, slabs = (nev + c - 1) / c, cost = (slabs + nsm - 1) / nsm * pass[q];
+        if (need(c) <= (size_t)optin && (cols == 0 || cost < best)) {
+            cols = c;
+            best = cost;
+        }
+    }
+    if (cols == 0) return cudaErrorInvalidValue;
     switch (cols) {
         case 8: return launch_bt<8>(t, Z, ldz, nev, ldzs, need(8), st);
         case 4: return launch_bt<4>(t, Z, ldz, nev, ldzs, need(4), st);
