@@ -11,9 +11,9 @@
 //   syr2k_kernel     the rest of A2 <- A2 - V W^T - W V^T (lower triangle).
 // 4/3 n^3 flop, nearly all in symm and syr2k on the FP64 tensor path (DMMA m16n8k16). The next panel
 // needs only what w_kernel makes, so it runs beside syr2k, on 16 of the SMs. At n = 12202 the whole
-// reduction to tridiagonal form with the chase takes 210 ms against 970 ms in one stage (symm 65,
-// syr2k with the panels beside it 70, vtx 8, w 4, chase 49); one after the other, with a cluster
-// barrier in every column of a panel, the same took 250.
+// reduction to tridiagonal form with the chase takes 200 ms against 970 ms in one stage (symm 54,
+// syr2k with the panels beside it 69, vtx 8, w 4, chase 49); one after the other, with a cluster
+// barrier in every column of a panel, the same took 240.
 #include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
@@ -328,114 +328,166 @@ __global__ void __launch_bounds__((kPanelWarps + 1) * 32, 1) panel_qr_kernel(Pan
 }
 
 // ------------------------------------------------------------------ X = A2 V
-constexpr int kBM = 64, kBK = 16, kThr = 128, kStages = 4;
-constexpr int kSK = kBK + 4;         // [row][k] tiles
-constexpr int kSM = kBM + 4;         // [k][row] tiles
-constexpr int kATile = kBM * kSK;    // holds either layout
-constexpr int kBTile = kB * kSK;
+constexpr int kBM = 64, kBK = 16, kThr = 128, kStages = 4, kSymmPerSm = 4;
+constexpr int kSM = kBM + 4;         // column stride of the update's tiles
+constexpr int kATile = kBM * kBK;    // [row][k] or [k][row], unpadded: pairs of doubles change places
+constexpr int kBTile = kB * kBK;     // within a row by swz(pair, row), which spreads the fragments' reads
+__device__ __forceinline__ int swz(int pair, int row) { return (pair ^ ((row & 3) << 1)) << 1; }
 constexpr size_t kSymmSmem = (size_t)kStages * (kATile + kBTile) * sizeof(double);
-static_assert(kStages * (kATile + kBTile) >= kBM * kB, "staging of the reduction fits the operand buffers");
+constexpr int kSymmMost = 1024;  // CTAs
+// CTAs of X = A2 V: kSymmPerSm an SM, but at least four k tiles each (28 steps from 900 rows down take
+// 0.35 ms; with eight k tiles 0.43)
+inline int symm_ctas(int R, int nsm) {
+    const long long units = (long long)((R + kBM - 1) / kBM) * ((R + kBK - 1) / kBK);
+    return (int)std::max(1ll, std::min((long long)std::min(kSymmMost, kSymmPerSm * nsm), units / 4));
+}
 
 // X (R x 32) = A2 V, A2 symmetric with its lower triangle stored: a 64-row tile takes k tiles left
 // of its diagonal block as stored, those right of it transposed (from the rows below), and the
-// diagonal block element by element. K is split over a cluster of gridDim.y CTAs whose partial
-// tiles are summed in order through distributed shared memory. A2 is read twice (2/3 n^3 flop over
-// n^3 / 12 bytes): 18.8 TF/s over the reduction at n = 12241.
-__global__ void __launch_bounds__(kThr) symm_kernel(const double *A2, long long lda, int R, const double *V, long long ldv,
-                                                    double *X, long long ldx) {
+// diagonal block element by element. A2 is read twice (2/3 n^3 flop over n^3 / 12 bytes).
+// All CTAs get the same number of k tiles, counted through tile after tile: a CTA ends one row tile
+// and begins another, and whoever is last at a tile adds up its parts, in their order (a split of
+// every tile into S equal parts, in a cluster, leaves SMs idle unless tiles x S happens to fill them:
+// 48 -> 40 ms for the first 150 steps at n = 12202, 19.7 -> 23.8 TF/s for the first one). Four CTAs an
+// SM by their four stages of unpadded tiles; three with padded ones: 43 ms.
+__global__ void __launch_bounds__(kThr, kSymmPerSm) symm_kernel(const double *A2, long long lda, int R, const double *V, long long ldv,
+                                                    double *X, long long ldx, double *part, int *count) {
     extern __shared__ __align__(16) double sm[];
-    const int i0 = blockIdx.x * kBM;
-    const int ntk = (R + kBK - 1) / kBK;
-    const int S = gridDim.y, z = blockIdx.y;
-    const int t0 = (int)((long long)ntk * z / S), t1 = (int)((long long)ntk * (z + 1) / S);
+    __shared__ int s_old;
+    const int ntk = (R + kBK - 1) / kBK, G = gridDim.x;
+    const long long units = (long long)((R + kBM - 1) / kBM) * ntk;
+    long long u = units * blockIdx.x / G;
+    const long long u1 = units * (blockIdx.x + 1) / G;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int wm = (warp >> 1) * 32, wn = (warp & 1) * 16;
     const int r = lane >> 2, c = lane & 3;
-    double acc[2][2][4];
+    while (u < u1) {
+        const int tile = (int)(u / ntk), i0 = tile * kBM, t0 = (int)(u - (long long)tile * ntk);
+        const int t1 = (int)min((long long)ntk, t0 + (u1 - u));
+        double acc[2][2][4];
 #pragma unroll
-    for (int a = 0; a < 2; ++a)
+        for (int a = 0; a < 2; ++a)
 #pragma unroll
-        for (int b = 0; b < 2; ++b)
+            for (int b = 0; b < 2; ++b)
 #pragma unroll
-            for (int h = 0; h < 4; ++h) acc[a][b][h] = 0.0;
-    auto load = [&](int kt) {
-        double *As = sm + (kt - t0) % kStages * (kATile + kBTile), *Bs = As + kATile;
-        const int k0 = kt * kBK, kmax = R - k0;
+                for (int h = 0; h < 4; ++h) acc[a][b][h] = 0.0;
+        auto load = [&](int kt) {
+            double *As = sm + (kt - t0) % kStages * (kATile + kBTile), *Bs = As + kATile;
+            const int k0 = kt * kBK, kmax = R - k0;
 #pragma unroll
-        for (int q = 0; q < 2; ++q) {  // V rows k0.., 32 columns, k-contiguous
-            const int e = tid + q * kThr, j = e >> 3, k = (e & 7) * 2;
-            const int valid = min(max(kmax - k, 0), 2);
-            cp16(Bs + j * kSK + k, valid ? V + (size_t)j * ldv + k0 + k : V, valid * 8);
+            for (int q = 0; q < 2; ++q) {  // V rows k0.., 32 columns, k-contiguous
+                const int e = tid + q * kThr, j = e >> 3, k = (e & 7) * 2;
+                const int valid = min(max(kmax - k, 0), 2);
+                cp16(Bs + j * kBK + swz(k >> 1, j), valid ? V + (size_t)j * ldv + k0 + k : V, valid * 8);
+            }
+            if (k0 + kBK <= i0) {  // as stored: [k][row]
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    const int e = tid + q * kThr, k = e >> 5, i = (e & 31) * 2;
+                    const int valid = min(max(R - i0 - i, 0), 2);
+                    cp16(As + k * kBM + swz(i >> 1, k), valid ? A2 + (size_t)(k0 + k) * lda + i0 + i : A2, valid * 8);
+                }
+            } else if (k0 >= i0 + kBM) {  // transposed: [row][k]
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    const int e = tid + q * kThr, i = e >> 3, k = (e & 7) * 2;
+                    const int valid = (i0 + i < R) ? min(max(kmax - k, 0), 2) : 0;
+                    cp16(As + i * kBK + swz(k >> 1, i), valid ? A2 + (size_t)(i0 + i) * lda + k0 + k : A2, valid * 8);
+                }
+            } else {
+#pragma unroll
+                for (int q = 0; q < 8; ++q) {
+                    const int e = tid + q * kThr, k = e >> 6, i = e & 63;
+                    const int gi = i0 + i, gk = k0 + k;
+                    As[k * kBM + swz(i >> 1, k) + (i & 1)] = (gi < R && gk < R) ? A2[(size_t)min(gi, gk) * lda + max(gi, gk)] : 0.0;
+                }
+            }
+        };
+#pragma unroll
+        for (int q = 0; q < kStages - 1; ++q) {
+            if (t0 + q < t1) load(t0 + q);
+            asm volatile("cp.async.commit_group;\n" ::);
         }
-        if (k0 + kBK <= i0) {  // as stored: [k][row]
+        for (int kt = t0; kt < t1; ++kt) {
+            asm volatile("cp.async.wait_group %0;\n" ::"n"(kStages - 2));
+            __syncthreads();
+            if (kt + kStages - 1 < t1) load(kt + kStages - 1);
+            asm volatile("cp.async.commit_group;\n" ::);
+            const double *As = sm + (kt - t0) % kStages * (kATile + kBTile), *Bs = As + kATile;
+            const bool tr = kt * kBK >= i0 + kBM;
+            double af[2][8], bf[2][4];
+            if (tr) {
 #pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                const int e = tid + q * kThr, k = e >> 5, i = (e & 31) * 2;
-                const int valid = min(max(R - i0 - i, 0), 2);
-                cp16(As + k * kSM + i, valid ? A2 + (size_t)(k0 + k) * lda + i0 + i : A2, valid * 8);
-            }
-        } else if (k0 >= i0 + kBM) {  // transposed: [row][k]
+                for (int a = 0; a < 2; ++a)
 #pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                const int e = tid + q * kThr, i = e >> 3, k = (e & 7) * 2;
-                const int valid = (i0 + i < R) ? min(max(kmax - k, 0), 2) : 0;
-                cp16(As + i * kSK + k, valid ? A2 + (size_t)(i0 + i) * lda + k0 + k : A2, valid * 8);
-            }
-        } else {
+                    for (int i = 0; i < 8; ++i)
+                        af[a][i] = As[(wm + a * 16 + r + 8 * (i & 1)) * kBK + swz((c >> 1) + 2 * (i >> 1), r) + (c & 1)];
+            } else {
 #pragma unroll
-            for (int q = 0; q < 8; ++q) {
-                const int e = tid + q * kThr, k = e >> 6, i = e & 63;
-                const int gi = i0 + i, gk = k0 + k;
-                As[k * kSM + i] = (gi < R && gk < R) ? A2[(size_t)min(gi, gk) * lda + max(gi, gk)] : 0.0;
+                for (int a = 0; a < 2; ++a)
+#pragma unroll
+                    for (int i = 0; i < 8; ++i)
+                        af[a][i] = As[(c + 4 * (i >> 1)) * kBM + swz(((wm + r) >> 1) + a * 8 + 4 * (i & 1), c) + (r & 1)];
             }
+#pragma unroll
+            for (int b = 0; b < 2; ++b)
+#pragma unroll
+                for (int i = 0; i < 4; ++i) bf[b][i] = Bs[(wn + b * 8 + r) * kBK + swz((c >> 1) + 2 * i, r) + (c & 1)];
+#pragma unroll
+            for (int a = 0; a < 2; ++a)
+#pragma unroll
+                for (int b = 0; b < 2; ++b) dmma16(acc[a][b], af[a], bf[b]);
         }
-    };
-#pragma unroll
-    for (int q = 0; q < kStages - 1; ++q) {
-        if (t0 + q < t1) load(t0 + q);
-        asm volatile("cp.async.commit_group;\n" ::);
-    }
-    for (int kt = t0; kt < t1; ++kt) {
-        asm volatile("cp.async.wait_group %0;\n" ::"n"(kStages - 2));
+        asm volatile("cp.async.wait_group 0;\n" ::);
         __syncthreads();
-        if (kt + kStages - 1 < t1) load(kt + kStages - 1);
-        asm volatile("cp.async.commit_group;\n" ::);
-        const double *As = sm + (kt - t0) % kStages * (kATile + kBTile), *Bs = As + kATile;
-        const bool tr = kt * kBK >= i0 + kBM;
-        const int sr = tr ? kSK : 1, sk = tr ? 1 : kSM;
-        double af[2][8], bf[2][4];
+        const bool whole = t0 == 0 && t1 == ntk;
+        // a CTA has at most one part that begins its tile (the CTA's last) and one that does not
+        double *out = part + ((size_t)blockIdx.x * 2 + (t0 == 0)) * (kBM * kB);
 #pragma unroll
         for (int a = 0; a < 2; ++a)
 #pragma unroll
-            for (int i = 0; i < 8; ++i) af[a][i] = As[(wm + a * 16 + r + 8 * (i & 1)) * sr + (c + 4 * (i >> 1)) * sk];
+            for (int b = 0; b < 2; ++b)
 #pragma unroll
-        for (int b = 0; b < 2; ++b)
+                for (int h = 0; h < 4; ++h) {
+                    const int i = wm + a * 16 + r + 8 * (h >> 1), j = wn + b * 8 + c * 2 + (h & 1);
+                    if (!whole) __stcg(out + j * kBM + i, acc[a][b][h]);
+                    else if (i0 + i < R) X[(size_t)j * ldx + i0 + i] = acc[a][b][h];
+                }
+        if (!whole) {
+            // the CTAs of this tile's first and last unit
+            const long long f = (long long)tile * ntk;
+            const int qa = (int)(((f + 1) * G - 1) / units), qb = (int)(((f + ntk) * G - 1) / units);
+            __threadfence();
+            __syncthreads();
+            if (tid == 0) s_old = atomicAdd(count + tile, 1);
+            __syncthreads();
+            if (s_old == qb - qa) {
+                __threadfence();
+                double2 sum[8];
 #pragma unroll
-            for (int i = 0; i < 4; ++i) bf[b][i] = Bs[(wn + b * 8 + r) * kSK + c + 4 * i];
+                for (int e = 0; e < 8; ++e) sum[e] = make_double2(0.0, 0.0);
+                for (int q = qa; q <= qb; ++q) {
+                    const double2 *src = reinterpret_cast<const double2 *>(part + ((size_t)q * 2 + (q == qa)) * (kBM * kB));
 #pragma unroll
-        for (int a = 0; a < 2; ++a)
+                    for (int e = 0; e < 8; ++e) {
+                        const double2 v = __ldcg(src + tid + e * kThr);
+                        sum[e].x += v.x;
+                        sum[e].y += v.y;
+                    }
+                }
 #pragma unroll
-            for (int b = 0; b < 2; ++b) dmma16(acc[a][b], af[a], bf[b]);
+                for (int e = 0; e < 8; ++e) {
+                    const int o = 2 * (tid + e * kThr), i = i0 + o % kBM;
+                    double *x = X + (size_t)(o / kBM) * ldx + i;
+                    if (i < R) x[0] = sum[e].x;
+                    if (i + 1 < R) x[1] = sum[e].y;
+                }
+                if (tid == 0) count[tile] = 0;
+            }
+        }
+        u += t1 - t0;
+        __syncthreads();  // the operand buffers and s_old are free
     }
-    asm volatile("cp.async.wait_group 0;\n" ::);
-    __syncthreads();
-    cg::cluster_group cluster = cg::this_cluster();
-#pragma unroll
-    for (int a = 0; a < 2; ++a)
-#pragma unroll
-        for (int b = 0; b < 2; ++b)
-#pragma unroll
-            for (int h = 0; h < 4; ++h)
-                sm[(wn + b * 8 + c * 2 + (h & 1)) * kBM + wm + a * 16 + r + 8 * (h >> 1)] = acc[a][b][h];
-    cluster.sync();
-    const int j0 = z * kB / S, j1 = (z + 1) * kB / S;  // each CTA of the cluster finishes some columns
-    for (int q = tid; q < (j1 - j0) * kBM; q += kThr) {
-        const int j = j0 + q / kBM, i = q % kBM;
-        double s = 0.0;
-        for (int u = 0; u < S; ++u) s += cluster.map_shared_rank(sm, u)[j * kBM + i];
-        if (i0 + i < R) X[(size_t)j * ldx + i0 + i] = s;
-    }
-    cluster.sync();
 }
 
 // ------------------------------------------------------------------ S = V^T X, M = -T^T S T / 2
@@ -628,11 +680,13 @@ __global__ void __launch_bounds__(kThr) w_kernel(double *VWV, long long ldv, con
 
 // ------------------------------------------------------------------ A -= V W^T + W V^T
 constexpr size_t kSyrSmem = (size_t)2 * 64 * kSM * sizeof(double);
+constexpr int kSyrThr = 256;
 
 // One 64 x 64 tile of the lower triangle, K = 64: [V W] against [W V], which the buffer V W V
-// holds side by side. The accumulators start from -A, so A is read while the operands arrive:
-// 18.8 TF/s over the reduction at n = 12241, against 6.2 TF/s for the one-stage path's update.
-__global__ void __launch_bounds__(kThr, 3) syr2k_band_kernel(double *A, long long lda, int R, const double *VWV, long long ldv) {
+// holds side by side. The accumulators start from -A, so A is read while the operands arrive. Eight
+// warps of 32 x 16 (four of 32 x 32 left fewer in flight: 48.7 -> 47.1 ms for the first 150 steps at
+// n = 12202): 20 TF/s, against 6.2 for the one-stage path's update.
+__global__ void __launch_bounds__(kSyrThr, 2) syr2k_band_kernel(double *A, long long lda, int R, const double *VWV, long long ldv) {
     extern __shared__ __align__(16) double sm[];
     double *Xs = sm, *Ys = sm + 64 * kSM;
     const long long t = blockIdx.x;
@@ -641,20 +695,20 @@ __global__ void __launch_bounds__(kThr, 3) syr2k_band_kernel(double *A, long lon
     while ((long long)(ti + 1) * (ti + 2) / 2 <= t) ++ti;
     const int i0 = ti * 64, j0 = (int)(t - (long long)ti * (ti + 1) / 2) * 64;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, r = lane >> 2, c = lane & 3;
-    const int wm = (warp >> 1) * 32, wn = (warp & 1) * 32;
+    const int wm = (warp >> 2) * 32, wn = (warp & 3) * 16;
 #pragma unroll
-    for (int q = 0; q < 16; ++q) {
-        const int e = tid + q * kThr, k = e >> 5, i = (e & 31) * 2;
+    for (int q = 0; q < 8; ++q) {
+        const int e = tid + q * kSyrThr, k = e >> 5, i = (e & 31) * 2;
         const int vi = min(max(R - i0 - i, 0), 2), vj = min(max(R - j0 - i, 0), 2);
         cp16(Xs + k * kSM + i, vi ? VWV + (size_t)k * ldv + i0 + i : VWV, vi * 8);
         cp16(Ys + k * kSM + i, vj ? VWV + (size_t)(32 + k) * ldv + j0 + i : VWV, vj * 8);
     }
     asm volatile("cp.async.commit_group;\n" ::);
-    double acc[2][4][4];
+    double acc[2][2][4];
 #pragma unroll
     for (int a = 0; a < 2; ++a)
 #pragma unroll
-        for (int b = 0; b < 4; ++b)
+        for (int b = 0; b < 2; ++b)
 #pragma unroll
             for (int h = 0; h < 4; ++h) {
                 const int i = i0 + wm + a * 16 + r + 8 * (h >> 1), j = j0 + wn + b * 8 + c * 2 + (h & 1);
@@ -664,24 +718,24 @@ __global__ void __launch_bounds__(kThr, 3) syr2k_band_kernel(double *A, long lon
     __syncthreads();
 #pragma unroll
     for (int k0 = 0; k0 < 64; k0 += 16) {
-        double af[2][8], bf[4][4];
+        double af[2][8], bf[2][4];
 #pragma unroll
         for (int a = 0; a < 2; ++a)
 #pragma unroll
             for (int i = 0; i < 8; ++i) af[a][i] = Xs[(k0 + c + 4 * (i >> 1)) * kSM + wm + a * 16 + r + 8 * (i & 1)];
 #pragma unroll
-        for (int b = 0; b < 4; ++b)
+        for (int b = 0; b < 2; ++b)
 #pragma unroll
             for (int i = 0; i < 4; ++i) bf[b][i] = Ys[(k0 + c + 4 * i) * kSM + wn + b * 8 + r];
 #pragma unroll
         for (int a = 0; a < 2; ++a)
 #pragma unroll
-            for (int b = 0; b < 4; ++b) dmma16(acc[a][b], af[a], bf[b]);
+            for (int b = 0; b < 2; ++b) dmma16(acc[a][b], af[a], bf[b]);
     }
 #pragma unroll
     for (int a = 0; a < 2; ++a)
 #pragma unroll
-        for (int b = 0; b < 4; ++b)
+        for (int b = 0; b < 2; ++b)
 #pragma unroll
             for (int h = 0; h < 4; ++h) {
                 const int i = i0 + wm + a * 16 + r + 8 * (h >> 1), j = j0 + wn + b * 8 + c * 2 + (h & 1);
@@ -763,17 +817,24 @@ bool band_reduce_available() {
     return s == 1;
 }
 
+static size_t symm_count_doubles(int n) { return (size_t)rup((n + kBM - 1) / kBM, 4) / 2; }
+
 size_t band_reduce_work_doubles(int n) {
     const size_t ld = (size_t)rup(n, 8);
-    return ld * (2 * 96 + 32 + 32) + 1024 + PanelPlan(n).spill_doubles();
+    // V W V twice, X, P, M, the counters and parts of symm_kernel, the panel's blocks in L2
+    return ld * (2 * 96 + 32 + 32) + 1024 + symm_count_doubles(n) + (size_t)symm_ctas(n, kSymmMost) * 2 * kBM * kB +
+           PanelPlan(n).spill_doubles();
 }
 
 cudaError_t launch_band_reduce(const BandReduce &b, cudaStream_t st) {
     const int n = b.n;
     const long long ld = rup(n, 8);
     double *X = b.work + 2 * 96 * ld, *P = X + 32 * ld, *M = P + 32 * ld;
+    int *count = reinterpret_cast<int *>(M + 1024);
+    double *part = M + 1024 + symm_count_doubles(n), *spill = part + (size_t)symm_ctas(n, kSymmMost) * 2 * kBM * kB;
     if (!band_reduce_available()) return cudaErrorNotSupported;
     cudaError_t e;
+    if ((e = cudaMemsetAsync(count, 0, symm_count_doubles(n) * sizeof(double), st)) != cudaSuccess) return e;
     if ((e = cudaMemsetAsync(b.C, 0, band_storage_doubles(n) * sizeof(double), st)) != cudaSuccess) return e;
     int dev = 0, nsm = 0;
     cudaGetDevice(&dev);
@@ -813,7 +874,7 @@ cudaError_t launch_band_reduce(const BandReduce &b, cudaStream_t st) {
         pa.n = n;
         const PanelPlan pp(R);
         pa.nsm = pp.nsm;
-        pa.spill = M + 1024;
+        pa.spill = spill;
         pa.err = b.err;
         pa.limit = b.wait_limit ? b.wait_limit : kPanelPolls;
         {
@@ -830,26 +891,10 @@ cudaError_t launch_band_reduce(const BandReduce &b, cudaStream_t st) {
             if ((e = cudaGetLastError()) != cudaSuccess) return e;
             continue;
         }
-        const int tiles = (R + kBM - 1) / kBM, ntk = (R + kBK - 1) / kBK;
-        {
-            // three CTAs an SM; the split that leaves the last wave fullest, at least four k tiles each
-            const int slots = 3 * nsm;
-            int S = 1;
-            double best = 0.0;
-            for (int s = 1; s <= 8 && s * 4 <= std::max(4, ntk); ++s) {
-                const double waves = (double)tiles * s / slots;
-                const double eff = waves / std::ceil(waves) * (double)ntk / (ntk + 6.0 * s);
-                if (eff > best) {
-                    best = eff;
-                    S = s;
-                }
-            }
-            ClusterLaunch l(dim3(tiles, S), kThr, kSymmSmem, 1, S, st);
-            DVR3D_COUNT_LAUNCH(1);
-            if ((e = cudaLaunchKernelEx(&l.cfg, symm_kernel, (const double *)A2, b.lda, R, (const double *)VWV, ld, X, ld)) !=
-                cudaSuccess)
-                return e;
-        }
+        const int tiles = (R + kBM - 1) / kBM;
+        DVR3D_COUNT_LAUNCH(1);
+        symm_kernel<<<symm_ctas(R, nsm), kThr, kSymmSmem, st>>>(A2, b.lda, R, VWV, ld, X, ld, part, count);
+        if ((e = cudaGetLastError()) != cudaSuccess) return e;
         {
             ClusterLaunch l(dim3(kCl), 256, 0, kCl, 1, st);
             DVR3D_COUNT_LAUNCH(1);
@@ -867,7 +912,7 @@ cudaError_t launch_band_reduce(const BandReduce &b, cudaStream_t st) {
                 return e;
             update.open = true;
             DVR3D_COUNT_LAUNCH(1);
-            syr2k_band_kernel<<<(unsigned)(nt * (nt + 1) / 2), kThr, kSyrSmem, b.side>>>(A2 + (size_t)kB * b.lda + kB, b.lda, R2,
+            syr2k_band_kernel<<<(unsigned)(nt * (nt + 1) / 2), kSyrThr, kSyrSmem, b.side>>>(A2 + (size_t)kB * b.lda + kB, b.lda, R2,
                                                                                       VWV + kB, ld);
             if ((e = cudaGetLastError()) != cudaSuccess) return e;
         }
