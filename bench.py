@@ -449,8 +449,8 @@ def main() -> int:
     if args.profile_solve:
         # one solve of the workload and nothing else. The chosen form: the 1D/2D stage,
         # assembly, the Cholesky-inverse (764 GEMM launches at this size, counting the start
-        # block's Cholesky-QR), then the Krylov steps. --precision fp64: the plain path (one
-        # dense_panel_kernel launch per 32-column panel of the reduction).
+        # block's Cholesky-QR), then the Krylov steps. --precision fp64: the plain path (the
+        # reduction to a band in panels of 32 columns, the chase, the eigenvalues).
         import dvr3d_b200
         from dvr3d_b200 import configs, parse_deck
 
@@ -603,7 +603,7 @@ def main() -> int:
         traffic, traffic_note = None, None
         tp = ROOT / "profiles" / "traffic.json"
         if tp.exists():
-            ent = json.loads(tp.read_text()).get("gemm_pipe_kernel")
+            ent = json.loads(tp.read_text()).get(kern)
             if ent:
                 traffic = ent["dram_bytes_per_launch"]
                 traffic_note = ent["launch"]
@@ -612,10 +612,11 @@ def main() -> int:
                 "traffic_launch": traffic_note,
                 "peak_source": "measured in this run: cuBLAS DGEMM (torch.matmul float64) 8192^3, best of 5",
                 "alg_flops_per_step": dom_flops / nprof, "launches": dom_launch / nprof,
-                "note": "achieved = algorithmic flops of the DMMA GEMM launches of a solve (Cholesky-inverse, "
-                        "Krylov steps, Ritz vectors, H3 X; per launch from M, N, K and its triangular structure) "
-                        "/ the sum of their durations, each launch timed by a CUDA event pair on the solve's stream "
-                        "(one solve after the timed region)",
+                "note": ("achieved = algorithmic flops of the DMMA GEMM launches of a solve (Cholesky-inverse, "
+                         "Krylov steps, Ritz vectors, H3 X; per launch from M, N, K and its triangular structure) "
+                         "/ the sum of their durations, each launch timed by a CUDA event pair on the solve's stream "
+                         "(one solve after the timed region)") if kern == "gemm_pipe_kernel" else
+                        "achieved = 4/3 N^3 flop of the reduction to a band / its duration, panels included",
                 "share_of_step": (dom_ms / nprof) / (ms / args.steps) if ms > 0 else None}
     else:
         achieved = dom_bytes / (dom_ms / 1000.0) / 1e9 if dom_ms > 0 else None

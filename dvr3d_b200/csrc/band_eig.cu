@@ -593,7 +593,8 @@ __global__ void band_slots_kernel(const double *A, long long lda, int n, int b, 
 // chunk are copied into shared memory (cp.async) while the current chunk is applied.
 // A task is a chain of loads, products, shuffles and stores (some 250 cycles), and a sweep a few of
 // them and a barrier; so a warp takes several tasks at once, loads first.
-// 500 vectors of order 2656 take 1.75 ms (2.1 with two columns a CTA and a task at a time).
+// 330 vectors of order 1600 take 1.75 ms, 532 of order 2656 3.9 (2.1 and 5.1 with two columns a CTA
+// and a task at a time).
 constexpr int kChunkTasks = 96;
 constexpr int kBtWarps = 8;
 
@@ -771,8 +772,8 @@ cudaError_t launch_band_backtransform(const BandTri &t, double *Z, long long ldz
     auto need = [&](int cols) { return fixed + (size_t)cols * ldzs * sizeof(double); };
     // The kernel is bound by shared memory: a reflector costs a slab of 1, 2, 4, 8 columns some 16, 20,
     // 30, 52 passes over it (loads, stores, shuffles), slabs on one SM add up. The width with the
-    // fewest passes on the fullest SM: 500 columns in slabs of 4, on 125 SMs (1.9 ms for order 2656; in slabs of 2 2.1),
-    // 100 columns one each.
+    // fewest passes on the fullest SM: 330 columns in slabs of 4, on 83 SMs (order 1600: 1.9 ms; in
+    // slabs of 2, two on some SMs, 2.1), 100 columns one each.
     static const int pass[4] = {16, 20, 30, 52};
     int cols = 0, best = 0;
     for (int q = 0; q < 4; ++q) {

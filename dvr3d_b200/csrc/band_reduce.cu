@@ -10,7 +10,7 @@
 //   w_kernel         W = X T + V M, and the next panel's columns of A2 - V W^T - W V^T;
 //   syr2k_kernel     the rest of A2 <- A2 - V W^T - W V^T (lower triangle).
 // 4/3 n^3 flop, nearly all in symm and syr2k on the FP64 tensor path (DMMA m16n8k16). The next panel
-// needs only what w_kernel makes, so it runs beside syr2k, on 16 of the SMs. At n = 12202 the whole
+// needs only what w_kernel makes, so it runs beside syr2k, on 16 of the SMs. At n = 12241 the whole
 // reduction to tridiagonal form with the chase takes 200 ms against 970 ms in one stage (symm 54,
 // syr2k with the panels beside it 69, vtx 8, w 4, chase 49); one after the other, with a cluster
 // barrier in every column of a panel, the same took 240.
@@ -84,7 +84,7 @@ constexpr int kBarPart = 1, kBarRow = 2;  // the warps' sums are there; the rank
 // every CTA of the cluster (st.async: the mbarrier there counts the bytes, so nothing waits for the
 // stores to return and no cluster barrier follows), adds up what has come in and forms the scalars;
 // the others meet it at two named barriers a column, and T's column follows off the path.
-// Latency bound: 1.6 us a column; 59 us a panel on average from 3968 rows down (81 with a cluster
+// Latency bound: 1.6 us a column; 59 us a panel on average from 3960 rows down (81 with a cluster
 // barrier a column and the exchange on a working warp).
 __global__ void __launch_bounds__((kPanelWarps + 1) * 32, 1) panel_qr_kernel(PanelArgs p) {
     extern __shared__ __align__(16) double psm[];
@@ -348,7 +348,7 @@ inline int symm_ctas(int R, int nsm) {
 // All CTAs get the same number of k tiles, counted through tile after tile: a CTA ends one row tile
 // and begins another, and whoever is last at a tile adds up its parts, in their order (a split of
 // every tile into S equal parts, in a cluster, leaves SMs idle unless tiles x S happens to fill them:
-// 48 -> 40 ms for the first 150 steps at n = 12202, 19.7 -> 23.8 TF/s for the first one). Four CTAs an
+// 48 -> 40 ms for the first 150 steps at n = 12241, 19.7 -> 23.8 TF/s for the first one). Four CTAs an
 // SM by their four stages of unpadded tiles; three with padded ones: 43 ms.
 __global__ void __launch_bounds__(kThr, kSymmPerSm) symm_kernel(const double *A2, long long lda, int R, const double *V, long long ldv,
                                                     double *X, long long ldx, double *part, int *count) {
@@ -685,7 +685,7 @@ constexpr int kSyrThr = 256;
 // One 64 x 64 tile of the lower triangle, K = 64: [V W] against [W V], which the buffer V W V
 // holds side by side. The accumulators start from -A, so A is read while the operands arrive. Eight
 // warps of 32 x 16 (four of 32 x 32 left fewer in flight: 48.7 -> 47.1 ms for the first 150 steps at
-// n = 12202): 20 TF/s, against 6.2 for the one-stage path's update.
+// n = 12241): 20 TF/s, against 6.2 for the one-stage path's update.
 __global__ void __launch_bounds__(kSyrThr, 2) syr2k_band_kernel(double *A, long long lda, int R, const double *VWV, long long ldv) {
     extern __shared__ __align__(16) double sm[];
     double *Xs = sm, *Ys = sm + 64 * kSM;

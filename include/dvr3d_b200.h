@@ -182,10 +182,11 @@ const char *dvr3d_b200_last_error(const dvr3d_ctx *ctx);
 /* Use `stream` (a cudaStream_t) for all work of this context; NULL = the ctx's own. */
 int dvr3d_b200_set_stream(dvr3d_ctx *ctx, void *stream);
 
-/* Every device-side wait of the library is bounded: the grid barriers of the cooperative
- * dense reduction (default 2^26 polls) and the hand-off waits of the band reduction's bulge
- * chase (default 2^24 polls). A wait that runs out raises the kernel's error flag, every CTA
- * leaves its kernel, and the solve returns DVR3D_ERR_NOCONV with the context still usable.
+/* Every device-side wait of the library is bounded: the grid barriers of the one-stage dense
+ * reduction and the waits of the two-stage one's panels for a column's sums (default 2^26
+ * polls), the hand-off waits of the bulge chase (2^24 polls through global memory, 2^26 in
+ * shared memory). A wait that runs out raises the kernel's error flag, every CTA leaves its
+ * kernel, and the solve returns DVR3D_ERR_NOCONV with the context still usable.
  * This sets the poll limit of every such wait of later solves on the context (0 restores the
  * defaults); a small limit lets a caller check that the waits end. No counterpart in the
  * reference (which has no device waits). */
@@ -363,7 +364,9 @@ int dvr3d_b200_run_deck(dvr3d_ctx *ctx, const char *deck_text, const dvr3d_optio
  * levels and each level's amplitudes on the DVR grid from trans (Jacobi, psi(idvr, npnt1,
  * npnt2), :3733-3841) or transr (Radau, wvfunc(nbass), :3622-3641). Records are sequential
  * unformatted with a 4-byte length count before and after each; logicals are 4-byte with
- * .TRUE. = -1. Amplitudes are defined up to the sign of each eigenvector. The readers are
+ * .TRUE. = -1. Amplitudes are defined up to the sign of each eigenvector. The path is opened
+ * before the first solve and its file replaced after the last (from 1 GiB of amplitudes on,
+ * earlier): a job that fails leaves what was there. The readers are
  * ROTLEV3 / ROTLEV3B / DIPOLE3 (source/wfnread.f90:101-215 reads the same records). */
 int dvr3d_b200_run_deck_wave(dvr3d_ctx *ctx, const char *deck_text, const dvr3d_options *opt,
                              char *out, size_t outcap, size_t *outlen,
