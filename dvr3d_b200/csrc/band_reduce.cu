@@ -12,7 +12,7 @@
 // 4/3 n^3 flop, nearly all in symm and syr2k on the FP64 tensor path (DMMA m16n8k16). The next panel
 // needs only what w_kernel makes, so it runs beside syr2k, on 16 of the SMs. At n = 12241 the whole
 // reduction to tridiagonal form with the chase takes 200 ms against 970 ms in one stage (symm 54,
-// syr2k with the panels beside it 69, vtx 8, w 4, chase 49); one after the other, with a cluster
+// syr2k with the panels beside it 69, vtx 6, w 4, chase 49); one after the other, with a cluster
 // barrier in every column of a panel, the same took 240.
 #include <cooperative_groups.h>
 #include <cuda_runtime.h>
@@ -491,15 +491,21 @@ __global__ void __launch_bounds__(kThr, kSymmPerSm) symm_kernel(const double *A2
 }
 
 // ------------------------------------------------------------------ S = V^T X, M = -T^T S T / 2
-// One cluster; every warp takes k steps of 16 rows, operands straight from L2 as fragments.
+// One cluster; every warp takes k steps of 16 rows, operands straight from L2 as fragments. Bound by
+// latency: the warps' sums are added in two rounds and go to the first CTA in one store each, so that
+// what follows the loads is two block barriers and one of the cluster: 10.5 us a launch on average
+// from 900 rows down (13.7 with eight rounds and the first CTA reading the others' sums).
+constexpr int kVS = 32 * 33;  // a 32 x 32 tile, column-major, 33 a column
+constexpr size_t kVtxSmem = (size_t)(kCl + 4) * kVS * sizeof(double);
 __global__ void __launch_bounds__(256) vtx_kernel(const double *V, long long ldv, const double *X, long long ldx, int R,
                                                   const double *T, double *M) {
-    __shared__ double part[32 * 33];      // this CTA's sum, column-major, 33 a column
-    __shared__ double Ts[32 * 33], Y[32 * 33];
+    extern __shared__ __align__(16) double sm[];
+    double *recv = sm, *loc = sm + kCl * kVS;  // every CTA's sum (first CTA); of this one's warps
+    __shared__ double Ts[kVS], Y[kVS];
     cg::cluster_group cluster = cg::this_cluster();
+    cluster.barrier_arrive();  // the first CTA is there before anything is stored into it
     const int rank = (int)cluster.block_rank();
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, r = lane >> 2, c = lane & 3;
-    for (int q = tid; q < 32 * 33; q += 256) part[q] = 0.0;
     for (int q = tid; q < 1024; q += 256) Ts[(q >> 5) * 33 + (q & 31)] = T[q];
     double acc[2][4][4];
 #pragma unroll
@@ -531,24 +537,34 @@ __global__ void __launch_bounds__(256) vtx_kernel(const double *V, long long ldv
 #pragma unroll
             for (int b = 0; b < 4; ++b) dmma16(acc[a][b], af[a], bf[b]);
     }
-    for (int w = 0; w < 8; ++w) {  // in order: the sum does not depend on timing
-        __syncthreads();
-        if (warp == w) {
+#pragma unroll
+    for (int round = 0; round < 2; ++round) {  // warps 4..7 store, 0..3 add theirs
+        if ((warp < 4) == (round == 1)) {
+            double *l = loc + (warp & 3) * kVS;
 #pragma unroll
             for (int a = 0; a < 2; ++a)
 #pragma unroll
                 for (int b = 0; b < 4; ++b)
 #pragma unroll
-                    for (int h = 0; h < 4; ++h)
-                        part[(b * 8 + c * 2 + (h & 1)) * 33 + a * 16 + r + 8 * (h >> 1)] += acc[a][b][h];
+                    for (int h = 0; h < 4; ++h) {
+                        const int e = (b * 8 + c * 2 + (h & 1)) * 33 + a * 16 + r + 8 * (h >> 1);
+                        l[e] = round ? l[e] + acc[a][b][h] : acc[a][b][h];
+                    }
         }
+        __syncthreads();
+    }
+    cluster.barrier_wait();
+    for (int q = tid; q < 1024; q += 256) {
+        const int e = (q >> 5) * 33 + (q & 31);
+        *cluster.map_shared_rank(recv + rank * kVS + e, 0) = (loc[e] + loc[kVS + e]) + (loc[2 * kVS + e] + loc[3 * kVS + e]);
     }
     cluster.sync();
     if (rank == 0) {
         for (int q = tid; q < 1024; q += 256) {
             const int e = (q >> 5) * 33 + (q & 31);
             double s = 0.0;
-            for (int u = 0; u < kCl; ++u) s += cluster.map_shared_rank(part, u)[e];
+#pragma unroll
+            for (int u = 0; u < kCl; ++u) s += recv[u * kVS + e];
             Y[e] = s;  // S
         }
         __syncthreads();
@@ -580,7 +596,6 @@ __global__ void __launch_bounds__(256) vtx_kernel(const double *V, long long ldv
 #pragma unroll
         for (int h = 0; h < 4; ++h) M[(n0 + c * 2 + (h & 1)) * 32 + m0 + r + 8 * (h >> 1)] = -0.5 * h4[h];
     }
-    cluster.sync();
 }
 
 // ------------------------------------------------------------------ W and the next panel
@@ -790,6 +805,7 @@ cudaError_t set_attributes() {
     if ((e = cudaFuncSetAttribute(vtx_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1)) != cudaSuccess) return e;
     if ((e = cudaFuncSetAttribute(panel_qr_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most)) != cudaSuccess) return e;
     if ((e = cudaFuncSetAttribute(symm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSymmSmem)) != cudaSuccess) return e;
+    if ((e = cudaFuncSetAttribute(vtx_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kVtxSmem)) != cudaSuccess) return e;
     if ((e = cudaFuncSetAttribute(w_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kWSmem)) != cudaSuccess) return e;
     return cudaFuncSetAttribute(syr2k_band_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSyrSmem);
 }
@@ -896,7 +912,7 @@ cudaError_t launch_band_reduce(const BandReduce &b, cudaStream_t st) {
         symm_kernel<<<symm_ctas(R, nsm), kThr, kSymmSmem, st>>>(A2, b.lda, R, VWV, ld, X, ld, part, count);
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
         {
-            ClusterLaunch l(dim3(kCl), 256, 0, kCl, 1, st);
+            ClusterLaunch l(dim3(kCl), 256, kVtxSmem, kCl, 1, st);
             DVR3D_COUNT_LAUNCH(1);
             if ((e = cudaLaunchKernelEx(&l.cfg, vtx_kernel, (const double *)VWV, ld, (const double *)X, ld, R,
                                         (const double *)pa.T, M)) != cudaSuccess)
