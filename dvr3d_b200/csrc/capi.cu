@@ -732,7 +732,8 @@ struct WaveFile {
     FortranRecords wr;
 
     explicit WaveFile(const char *p) : path(p) {
-        fresh = ::access(p, F_OK) != 0;
+        struct stat sb;
+        fresh = ::lstat(p, &sb) != 0;  // not even a link that leads nowhere
         f = std::fopen(p, "ab");
         if (!f) throw HostError{DVR3D_ERR_ARG, "cannot open " + path};
         wr.f = f;
