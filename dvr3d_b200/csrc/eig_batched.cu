@@ -333,7 +333,7 @@ __global__ void __launch_bounds__(512) tridiag_small_kernel(BatchDesc bd, double
 // ------------------------------------------------------------------ eigenvalues
 constexpr int kEvThreads = 512;
 
-// Sturm-count multisection. Every CTA first counts at 512 equidistant points, which brackets each
+// Sturm-count multisection (by minors, or by quotients: tridiag_dev.cuh). Every CTA first counts at 512 equidistant points, which brackets each
 // eigenvalue to 1/513 of the Gershgorin interval in one pass; then groups of L lanes narrow one
 // eigenvalue each, L + 1 times a pass, L the largest power of two that keeps the CTA's threads busy.
 // gridDim.y CTAs share a block's eigenvalues. Bound by the FP64 issue of the counts (three
@@ -371,21 +371,41 @@ __global__ void __launch_bounds__(kEvThreads) eigvals_kernel(BatchDesc bd, const
     }
     // the matrix and its bounds in units of 1 / scale
     const double tnorm = fmax(fabs(s_min[0]), fabs(s_max[0]));
-    const double scale = sturm_scale(tnorm), unit = 1.0 / scale;
-    const double margin = 2.0 * DBL_EPSILON * (tnorm * scale) * n + 2.0 * DBL_MIN;
-    const double glo = s_min[0] * scale - margin, ghi = s_max[0] * scale + margin;
+    double scale = sturm_scale(tnorm), piv = DBL_MIN;
+    bool small = false;
     for (int i = tid; i < n; i += blockDim.x) {
         sd[i] = d[i] * scale;
-        if (i < n - 1) ne2[i] = sturm_off(e[i], scale);
+        if (i < n - 1) {
+            const double es = e[i] * scale;
+            ne2[i] = -es * es;
+            small |= !(es * es >= kSturmLeast);
+        }
     }
-    __syncthreads();
+    const bool quotients = __syncthreads_or(small);
+    if (quotients) {
+        scale = sturm_scale_quotients(tnorm);
+        for (int i = tid; i < n; i += blockDim.x) {
+            sd[i] = d[i] * scale;
+            if (i < n - 1) {
+                const double es = e[i] * scale;
+                ne2[i] = es * es;
+            }
+        }
+        __syncthreads();
+        double most = 1.0;
+        for (int i = 0; i < n - 1; ++i) most = fmax(most, ne2[i]);
+        piv = DBL_MIN * most;
+    }
+    auto count = [&](double x) { return quotients ? sturm_quotients(sd, ne2, n, x, 1.0, piv) : sturm_count(sd, ne2, n, x); };
+    const double unit = 1.0 / scale, margin = 2.0 * DBL_EPSILON * (tnorm * scale) * n + 2.0 * piv;
+    const double glo = s_min[0] * scale - margin, ghi = s_max[0] * scale + margin;
     const double h = (ghi - glo) / (double)(kEvThreads + 1);
-    s_cnt[tid] = sturm_count(sd, ne2, n, glo + h * (double)(tid + 1));
+    s_cnt[tid] = count(glo + h * (double)(tid + 1));
     if (mode != 0 && tid == 0) {
         double x = cut;
         if (mode == 2) x = nextafter(cut, DBL_MAX);  // count of eigenvalues <= cut
         x *= scale;
-        s_count = (x <= glo) ? 0 : (x >= ghi ? n : sturm_count(sd, ne2, n, x));
+        s_count = (x <= glo) ? 0 : (x >= ghi ? n : count(x));
     }
     __syncthreads();
     const int m = (mode != 0) ? s_count : n;
@@ -414,7 +434,7 @@ __global__ void __launch_bounds__(kEvThreads) eigvals_kernel(BatchDesc bd, const
             if (run && z - a <= 2.0 * DBL_EPSILON * fmax(fabs(a), fabs(z))) run = false;
             if (!__any_sync(0xffffffffu, run)) break;
             const double x = (L == 1) ? 0.5 * (a + z) : a + (z - a) * ((double)(sub + 1) / (double)(L + 1));
-            const bool above = sturm_count(sd, ne2, n, x) > j;
+            const bool above = count(x) > j;
             const unsigned bal = __ballot_sync(0xffffffffu, above) & gmask;
             const int f = bal ? __ffs(bal) - 1 - g0 : L;  // first lane above
             const double xl = __shfl_sync(0xffffffffu, x, g0 + (f > 0 ? f - 1 : 0));

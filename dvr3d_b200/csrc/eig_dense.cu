@@ -595,14 +595,37 @@ __global__ void __launch_bounds__(1024) tri_bounds_kernel(const double *d, const
         }
         __syncthreads();
     }
-    const double tnorm = fmax(fabs(smin[0]), fabs(smax[0])), scale = sturm_scale(tnorm);
-    for (int i = tid; i + 1 < n; i += blockDim.x) ne2[i] = sturm_off(e[i], scale);
+    const double low = smin[0], high = smax[0], tnorm = fmax(fabs(low), fabs(high));
+    double scale = sturm_scale(tnorm), piv = 0.0;
+    bool small = false;
+    for (int i = tid; i + 1 < n; i += blockDim.x) {
+        const double es = e[i] * scale;
+        ne2[i] = -es * es;
+        small |= !(es * es >= kSturmLeast);
+    }
+    if (__syncthreads_or(small)) {  // the counts go by quotients
+        scale = sturm_scale_quotients(tnorm);
+        double most = 1.0;
+        for (int i = tid; i + 1 < n; i += blockDim.x) {
+            const double es = e[i] * scale;
+            ne2[i] = es * es;
+            most = fmax(most, es * es);
+        }
+        smax[tid] = most;
+        __syncthreads();
+        for (int s = blockDim.x / 2; s > 0; s >>= 1) {
+            if (tid < s) smax[tid] = fmax(smax[tid], smax[tid + s]);
+            __syncthreads();
+        }
+        piv = DBL_MIN * smax[0];
+    }
     if (tid == 0) {
-        const double margin = 2.0 * DBL_EPSILON * tnorm * n + 2.0 * DBL_MIN;
-        info[0] = smin[0] - margin;
-        info[1] = smax[0] + margin;
+        const double margin = 2.0 * DBL_EPSILON * tnorm * n + 2.0 * fmax(piv / scale, DBL_MIN);
+        info[0] = low - margin;
+        info[1] = high + margin;
         info[2] = scale;
         info[3] = fmax(tnorm, DBL_MIN);
+        info[4] = piv;
     }
 }
 
@@ -615,41 +638,46 @@ __global__ void __launch_bounds__(128) multisect_kernel(const double *d, const d
     const int lane = threadIdx.x & 31;
     if (gw >= nev) return;
     const int j = gw;
-    const double scale = info[2], unit = 1.0 / scale;
+    const double scale = info[2], unit = 1.0 / scale, piv = info[4];
     double lo = info[0] * scale, hi = info[1] * scale;
     for (int pass = 0; pass < 64; ++pass) {
         if (hi - lo <= 2.0 * DBL_EPSILON * fmax(fabs(lo), fabs(hi))) break;
         const double x = lo + (hi - lo) * (double)(lane + 1) / 33.0;
-        SturmCount s;
-        s.start(fma(d[0], scale, -x));
-        int i = 1;
-        if (n >= 9) {
-            double dd[8], ee[8];
-#pragma unroll
-            for (int u = 0; u < 8; ++u) {
-                dd[u] = d[i + u];
-                ee[u] = ne2[i + u - 1];
-            }
-            for (; i + 8 <= n; i += 8) {
-                double dn[8], en[8];
-                const int q = (i + 16 <= n) ? i + 8 : i;  // the next eight rows, if there are
+        int c;
+        if (piv > 0.0) {
+            c = sturm_quotients(d, ne2, n, x, scale, piv);
+        } else {
+            SturmCount s;
+            s.start(fma(d[0], scale, -x));
+            int i = 1;
+            if (n >= 9) {
+                double dd[8], ee[8];
 #pragma unroll
                 for (int u = 0; u < 8; ++u) {
-                    dn[u] = d[q + u];
-                    en[u] = ne2[q + u - 1];
+                    dd[u] = d[i + u];
+                    ee[u] = ne2[i + u - 1];
                 }
+                for (; i + 8 <= n; i += 8) {
+                    double dn[8], en[8];
+                    const int q = (i + 16 <= n) ? i + 8 : i;  // the next eight rows, if there are
 #pragma unroll
-                for (int u = 0; u < 8; ++u) s.step(fma(dd[u], scale, -x), ee[u]);
-                s.rescale();
+                    for (int u = 0; u < 8; ++u) {
+                        dn[u] = d[q + u];
+                        en[u] = ne2[q + u - 1];
+                    }
 #pragma unroll
-                for (int u = 0; u < 8; ++u) {
-                    dd[u] = dn[u];
-                    ee[u] = en[u];
+                    for (int u = 0; u < 8; ++u) s.step(fma(dd[u], scale, -x), ee[u]);
+                    s.rescale();
+#pragma unroll
+                    for (int u = 0; u < 8; ++u) {
+                        dd[u] = dn[u];
+                        ee[u] = en[u];
+                    }
                 }
             }
+            for (; i < n; ++i) s.step(fma(d[i], scale, -x), ne2[i - 1]);
+            c = s.c;
         }
-        for (; i < n; ++i) s.step(fma(d[i], scale, -x), ne2[i - 1]);
-        const int c = s.c;
         const unsigned bal = __ballot_sync(0xffffffffu, c > j);
         const int l = bal ? (__ffs(bal) - 1) : 32;
         const double xl = __shfl_sync(0xffffffffu, x, l > 0 ? l - 1 : 0);

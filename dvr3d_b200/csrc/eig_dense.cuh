@@ -36,7 +36,9 @@ int dense_resident_plan(int device, int n, int *grid);
 int dense_tridiag_grid(int device);
 int dense_panel_width();
 cudaError_t launch_dense_tridiag(DenseTri &t, int grid, cudaStream_t st);
-// info[0..3] = lower bound, upper bound, pivmin, ||T||
+// info[kTriInfo]: lower bound, upper bound, scale of the Sturm counts, ||T||, and the least quotient
+// where the counts go by quotients (zero: by minors)
+constexpr int kTriInfo = 5;
 void launch_dense_eigvals(const double *d, const double *e, int n, int nev, double *e2, double *info,
                           double *w, cudaStream_t st);
 // Eigenvectors of the reduced matrix for the nev eigenvalues w, back-transformed into Z.

@@ -682,7 +682,7 @@ void dense_lowest_two_stage(dvr3d_ctx *ctx, double *A, long long lda, int n, int
     bt.wait_limit = ctx->wait_limit;
     CK(launch_band_chase(bt, st));
     double *e2s = ctx->arena.get_t<double>(t + "e2", n);
-    double *info = ctx->arena.get_t<double>(t + "info", 4);
+    double *info = ctx->arena.get_t<double>(t + "info", kTriInfo);
     launch_dense_eigvals(bt.d, bt.e, n, nev, e2s, info, w, st);
     CK(cudaGetLastError());
     if (vecs) {
@@ -785,7 +785,7 @@ void dense_lowest(dvr3d_ctx *ctx, double *A, long long lda, int n, int nev, bool
         std::fprintf(stderr, "\n");
     }
     double *e2s = ctx->arena.get_t<double>(t + "e2", n);
-    double *info = ctx->arena.get_t<double>(t + "info", 4);
+    double *info = ctx->arena.get_t<double>(t + "info", kTriInfo);
     launch_dense_eigvals(dt.d, dt.e, n, nev, e2s, info, w, st);
     CK(cudaGetLastError());
     if (vecs) {
@@ -844,7 +844,7 @@ bool band_lowest(dvr3d_ctx *ctx, double *A, long long lda, int n, int b, int nev
     CK(launch_band_chase(t, st));
     check_dev_err(ctx, t.err, "band reduction");
     double *e2s = ctx->arena.get_t<double>("bd_e2", n);
-    double *info = ctx->arena.get_t<double>("bd_info", 4);
+    double *info = ctx->arena.get_t<double>("bd_info", kTriInfo);
     launch_dense_eigvals(t.d, t.e, n, nev, e2s, info, w, st);
     CK(cudaGetLastError());
     const int T = std::min(nev, 1024);

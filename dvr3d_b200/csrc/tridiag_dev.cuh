@@ -13,10 +13,11 @@ namespace dvr3d {
 // principal minors p_0 = 1, p_i = (d_i - x) p_{i-1} - e_{i-1}^2 p_{i-2} (Givens). Unlike the
 // quotients p_i / p_{i-1} of dstebz this needs no division: one dependent multiply-add a row (about
 // 8 cycles against 110). T is scaled to norm below one by a power of two, so a pair of minors grows
-// at most threefold a row; squared off-diagonals below 2^-120 (a perturbation of 2^-60 ||T||) are
-// raised to it, so no two consecutive minors vanish; and the pair is brought back to magnitude one
-// every eight rows, between which it cannot leave the exponent range.
-constexpr double kSturmFloor = 7.52316384526264e-37;  // 2^-120
+// at most threefold a row; and the pair is brought back to magnitude one every eight rows, between
+// which it cannot leave the exponent range as long as no squared off-diagonal is below 2^-120. A
+// matrix that has one (decoupled, or graded over more than 2^60) is counted by the quotients,
+// which keep each decoupled part's eigenvalues accurate relative to that part.
+constexpr double kSturmLeast = 7.52316384526264e-37;  // 2^-120
 
 // power of two that brings ||T|| = tnorm below one
 static __device__ __forceinline__ double sturm_scale(double tnorm) {
@@ -25,10 +26,24 @@ static __device__ __forceinline__ double sturm_scale(double tnorm) {
     frexp(tnorm, &ex);
     return ldexp(1.0, -max(-1000, min(1000, ex)));
 }
-// the off-diagonal term of the recurrence, -e^2 of the scaled matrix
-static __device__ __forceinline__ double sturm_off(double e, double scale) {
-    const double es = e * scale;
-    return -fmax(es * es, kSturmFloor);
+// the same for the quotients, whose small entries keep their exponents: only norms whose squares
+// leave the range are scaled
+static __device__ __forceinline__ double sturm_scale_quotients(double tnorm) {
+    return (tnorm < 1.0e150 && tnorm > 1.0e-150) ? 1.0 : sturm_scale(tnorm);
+}
+
+// Number of eigenvalues of T strictly below x by the quotients (a zero one counts as negative): d, x
+// and e2, the squared off-diagonals, in units of 1 / scale.
+static __device__ __noinline__ int sturm_quotients(const double *d, const double *e2, int n, double x, double scale, double pivmin) {
+    double q = fma(d[0], scale, -x);
+    if (fabs(q) < pivmin) q = -pivmin;
+    int c = (q < 0.0);
+    for (int i = 1; i < n; ++i) {
+        q = fma(d[i], scale, -x) - e2[i - 1] / q;
+        if (fabs(q) < pivmin) q = -pivmin;
+        c += (q < 0.0);
+    }
+    return c;
 }
 
 // Running count: rows are fed in order with step(), eight at most between calls of rescale().
@@ -54,7 +69,8 @@ struct SturmCount {
     }
 };
 
-// Number of eigenvalues of T strictly below x; d and x scaled, ne2 from sturm_off.
+// Number of eigenvalues of T strictly below x; by the minors: d, x and ne2, the negative
+// squared off-diagonals, in units of 1 / scale.
 static __device__ __forceinline__ int sturm_count(const double *d, const double *ne2, int n, double x) {
     SturmCount s;
     s.start(d[0] - x);
