@@ -333,9 +333,10 @@ __global__ void __launch_bounds__(512) tridiag_small_kernel(BatchDesc bd, double
 // ------------------------------------------------------------------ eigenvalues
 constexpr int kEvThreads = 512;
 
-// Sturm-count multisection (by minors, or by quotients: tridiag_dev.cuh). Every CTA first counts at 512 equidistant points, which brackets each
-// eigenvalue to 1/513 of the Gershgorin interval in one pass; then groups of L lanes narrow one
-// eigenvalue each, L + 1 times a pass, L the largest power of two that keeps the CTA's threads busy.
+// Sturm-count multisection (by minors, or by quotients: tridiag_dev.cuh). Every CTA first counts at
+// 512 equidistant points, which brackets each eigenvalue to 1/513 of the Gershgorin interval in one
+// pass; then groups of L lanes narrow one eigenvalue each, L + 1 times a pass, L the largest power of
+// two that keeps the CTA's threads busy.
 // gridDim.y CTAs share a block's eigenvalues. Bound by the FP64 issue of the counts (three
 // operations a row): 64 blocks of order 465, 62 eigenvalues each: 0.21 ms (one thread an eigenvalue
 // with a division a row: 2.2 ms).
