@@ -43,6 +43,7 @@ __global__ void __launch_bounds__(1024) tridiag_kernel(BatchDesc bd, double *A, 
     extern __shared__ double sm[];
     double *V = sm, *W = V + kTriNb * ns, *xs = W + kTriNb * ns, *sp0 = xs + ns;
     __shared__ double part[32], part2[32], zs[2 * kTriNb];
+    if constexpr (C > 1) cg::this_cluster().barrier_arrive();
     const int T = blockDim.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = T >> 5;
     auto get = [&](int r, int c) { return __ldcg(ag + (unsigned)(c * n + r)); };
     auto exchange = [&]() {
@@ -53,6 +54,7 @@ __global__ void __launch_bounds__(1024) tridiag_kernel(BatchDesc bd, double *A, 
     __syncthreads();
     const int row = tid;  // the row of this thread in the vector steps
     double acol = (row < n) ? get(row, 0) : 0.0, x = 0.0;
+    if constexpr (C > 1) cg::this_cluster().barrier_wait();  // the others are there: partial sums go into them
     for (int k = 0; k + 2 < n; ++k) {
         const int i = k % kTriNb;
         if (i == 0 && k > 0) {
