@@ -173,6 +173,7 @@ struct alignas(128) ChaseSmem {
     unsigned long long credit[kRing];       // staged slots free again, here and at the next CTA
     volatile int tasks, refl;               // tasks begun; reflectors known, their betas staged
     volatile int abort;
+    int slots_in, firsts_in;                // slots and first columns sent to this CTA in all
 };
 
 __global__ void __launch_bounds__(kChaseThreads, 1) band_chase_kernel(BandTri t) {
@@ -193,7 +194,7 @@ __global__ void __launch_bounds__(kChaseThreads, 1) band_chase_kernel(BandTri t)
     for (int q = tid; q < (int)(2 * kRing * sizeof(ChaseSlot) / 8); q += kChaseThreads) reinterpret_cast<double *>(S.raw)[q] = 0.0;
     if (tid < kBW) S.xin[tid] = S.xout[tid] = 0.0;
     if (tid == 0) {
-        S.abort = 0;
+        S.abort = S.slots_in = S.firsts_in = 0;
         for (int q = 0; q < kRing; ++q) {
             mbar_init(smem_u32(&S.full[q]), 1);
             mbar_init(smem_u32(&S.own[q]), 1);
@@ -230,6 +231,8 @@ __global__ void __launch_bounds__(kChaseThreads, 1) band_chase_kernel(BandTri t)
     int in0 = 0;     // slots of this CTA's ring consumed by earlier sweeps
     int out0 = 0;    // slots sent by earlier sweeps
     int sweeps = 0;  // sweeps so far
+    int blocks = 0, betas = 0, firsts = 0;  // sent to the next CTA by this thread
+    int expected = 1;                       // first columns that this thread has told fullx to expect
     for (int j = (int)(blockIdx.x / K) * K + rank; j <= n - 3; j += gridDim.x, ++sweeps) {
         const int nt = band_ntask(n, b, j);
         const int ntp = (j > 0) ? band_ntask(n, b, j - 1) : 0;
@@ -280,6 +283,7 @@ __global__ void __launch_bounds__(kChaseThreads, 1) band_chase_kernel(BandTri t)
                             mbar_expect(smem_u32(&S.full[sl]), slot_bytes);
                             fence_async();
                             bulk_load(smem_u32(&S.raw[sl]), G + 1 + s, slot_bytes, smem_u32(&S.full[sl]));
+                            S.slots_in = m + 1;
                         }
                     }
                 }
@@ -289,8 +293,12 @@ __global__ void __launch_bounds__(kChaseThreads, 1) band_chase_kernel(BandTri t)
                 for (int s = -1; s + 1 < nt && !S.abort; ++s) {
                     while (S.tasks < s + 2 && !S.abort) {}
                     if (S.abort) break;
-                    if (s < 0) mbar_expect(smem_u32(&S.fullx), x_bytes);  // the first column, for the next sweep
-                    else give_back(in0 + s);
+                    if (s < 0) {  // the first column, for the next sweep
+                        mbar_expect(smem_u32(&S.fullx), x_bytes);
+                        ++expected;
+                    } else {
+                        give_back(in0 + s);
+                    }
                 }
             }
         } else if (role == 0 && w == 1) {
@@ -302,6 +310,7 @@ __global__ void __launch_bounds__(kChaseThreads, 1) band_chase_kernel(BandTri t)
                     const int u = (out0 + s) % kRing;
                     fence_async();
                     bulk_to_cta(rem(&S.raw[u]), smem_u32(&S.stage[u]), block_bytes, rem(&S.full[u]));
+                    blocks = out0 + s + 1;
                 }
             } else if (far && lane == 0) {
                 // the first column is known with task 1's beta, slot s with task s + 2's
@@ -493,9 +502,13 @@ __global__ void __launch_bounds__(kChaseThreads, 1) band_chase_kernel(BandTri t)
                     __syncwarp();
 #pragma unroll
                     for (int g = 1; g <= 3; ++g) bar_arrive(kBarY + g, 5 * 32);
-                    if (near && !S.abort) {
-                        if (s == 1 && lane < b) st_async(rem(&S.xin[lane]), (lane == b - 1) ? beta : S.xout[lane], rem(&S.fullx));
-                        if (s >= 2 && lane == 0) st_async(rem(&S.raw[so2].beta), beta, rem(&S.full[so2]));
+                    if (near && s == 1 && __all_sync(kFull, !S.abort)) {  // all of it or nothing
+                        if (lane < b) st_async(rem(&S.xin[lane]), (lane == b - 1) ? beta : S.xout[lane], rem(&S.fullx));
+                        ++firsts;
+                    }
+                    if (near && s >= 2 && lane == 0 && !S.abort) {
+                        st_async(rem(&S.raw[so2].beta), beta, rem(&S.full[so2]));
+                        betas = o - 1;
                     }
                     if (far && lane == 0) {
                         if (s == 1) S.xout[b - 1] = beta;
@@ -519,8 +532,11 @@ __global__ void __launch_bounds__(kChaseThreads, 1) band_chase_kernel(BandTri t)
         __syncthreads();
         // the last two slots (and the first column of a sweep of one task); the betas of tasks nt and
         // nt + 1 are zero
-        if (near && warp == 2 && !S.abort) {
-            if (nt == 1 && lane < b) st_async(rem(&S.xin[lane]), (lane == b - 1) ? 0.0 : S.xout[lane], rem(&S.fullx));
+        if (near && warp == 2 && __all_sync(kFull, !S.abort)) {
+            if (nt == 1) {
+                if (lane < b) st_async(rem(&S.xin[lane]), (lane == b - 1) ? 0.0 : S.xout[lane], rem(&S.fullx));
+                ++firsts;
+            }
             if (lane == 0) {
                 fence_async();
                 for (int s = max(0, nt - 2); s < nt; ++s) {
@@ -528,6 +544,7 @@ __global__ void __launch_bounds__(kChaseThreads, 1) band_chase_kernel(BandTri t)
                     bulk_to_cta(rem(&S.raw[u]), smem_u32(&S.stage[u]), block_bytes, rem(&S.full[u]));
                     st_async(rem(&S.raw[u].beta), 0.0, rem(&S.full[u]));
                 }
+                blocks = betas = out0 + nt;
             }
         }
         if (far && warp == 1 && lane == 0 && !S.abort) {
@@ -547,6 +564,7 @@ __global__ void __launch_bounds__(kChaseThreads, 1) band_chase_kernel(BandTri t)
                 for (int s = nt - 1; s < ntp; ++s) {
                     const int m = in0 + s;
                     if (s >= nt) wait(&S.full[m % kRing], (m / kRing) & 1);
+                    if (S.abort) break;
                     give_back(m);
                 }
         }
@@ -554,7 +572,34 @@ __global__ void __launch_bounds__(kChaseThreads, 1) band_chase_kernel(BandTri t)
         in0 += first ? nt : ntp;
         if (send) out0 += nt;
     }
-    if (S.abort) __nanosleep(20000);  // copies of a neighbour that gave up may still be on their way
+    // Nobody leaves with a copy into its shared memory on the way, given up or not: a sender makes whole
+    // what it has begun (a slot of which only the block or only the beta has gone: the receiver has
+    // given its credit, so it expects the other part too) and says how much that was; then the
+    // receiver waits for the last phases of these barriers, whether or not it has read the slots.
+    if (warp == 1 && lane == 0) S.tasks = blocks;
+    __syncthreads();
+    if (warp == 2 && lane == 0 && !last) {
+        blocks = max(blocks, S.tasks);
+        const int whole = max(blocks, betas);
+        fence_async();
+        for (int m = min(blocks, betas); m < whole; ++m) {
+            const int u = m % kRing;
+            if (m >= blocks) bulk_to_cta(rem(&S.raw[u]), smem_u32(&S.stage[u]), block_bytes, rem(&S.full[u]));
+            else st_async(rem(&S.raw[u].beta), 0.0, rem(&S.full[u]));
+        }
+        *cluster.map_shared_rank(&S.slots_in, rank + 1) = whole;
+        *cluster.map_shared_rank(&S.firsts_in, rank + 1) = firsts;
+    }
+    cluster.sync();
+    if (tid == 0) {
+        auto arrived = [&](unsigned long long *bar, unsigned phase) {
+            for (unsigned long long spins = 0; spins < 4 * kSpinLimit && !mbar_test(smem_u32(bar), phase & 1); ++spins) {}
+        };
+        const int slots = S.slots_in;
+        for (int m = max(0, slots - kRing); m < slots; ++m) arrived(&S.full[m % kRing], m / kRing);
+        if (S.firsts_in > expected) mbar_expect(smem_u32(&S.fullx), x_bytes);  // gave up before it came to that
+        if (S.firsts_in > 0) arrived(&S.fullx, S.firsts_in - 1);
+    }
     cluster.sync();
 }
 
