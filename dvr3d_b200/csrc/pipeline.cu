@@ -1329,9 +1329,9 @@ void solve_contracted(dvr3d_ctx *ctx, const BlockPlan &p, const Contracted &C, c
     if (wave) compute_wavefunctions(ctx, p, C, Z, N, meval, *wave);
     double ms1, ms2, ms3;
     finish_times(ms1, ms2, ms3);
-    // dominant kernel: the panel kernel of the Householder reduction; its algorithmic
-    // traffic is one read of the trailing lower triangle per column
-    // (one-stage), or the 4/3 N^3 flop of the reduction to band form (two-stage)
+    // dominant work: one-stage, the panel kernel of the Householder reduction, whose algorithmic
+    // traffic is one read of the trailing lower triangle per column; two-stage, the reduction to band
+    // form as a whole (panel_qr, symm, vtx, w and syr2k_band: 4/3 N^3 flop), whose kernels overlap
     double bytes = 0.0;
     for (int k = 0; k + 2 < N; ++k) {
         const double m = (double)(N - k - 1);
@@ -1341,7 +1341,7 @@ void solve_contracted(dvr3d_ctx *ctx, const BlockPlan &p, const Contracted &C, c
     res.dom_bytes = dout.two_stage ? 0.0 : bytes;
     res.dom_flops = dout.two_stage ? 4.0 / 3.0 * (double)N * N * N : 0.0;
     res.dom_launches = dout.npanel;
-    std::snprintf(res.dom_kernel, sizeof(res.dom_kernel), dout.two_stage ? "syr2k_band_kernel" : "dense_panel_kernel");
+    std::snprintf(res.dom_kernel, sizeof(res.dom_kernel), dout.two_stage ? "band_reduction" : "dense_panel_kernel");
     res.launches = (int)(g_kernel_launches - launches0);
     res.h2d_bytes = t_h2d;
     res.d2h_bytes = t_d2h;

@@ -153,7 +153,9 @@ typedef struct dvr3d_result {
     int launches;           /* kernels launched by the library for this solve               */
     long long h2d_bytes;    /* host -> device bytes copied by this solve                    */
     long long d2h_bytes;    /* device -> host bytes copied by this solve                    */
-    char dom_kernel[48];    /* name of the dominant kernel                                  */
+    char dom_kernel[48];    /* name of the dominant kernel, or "band_reduction": dom_ms,
+                               dom_flops and dom_launches are of all kernels of the dense
+                               reduction to a band                                          */
     /* caller-provided buffers (may be NULL / 0) */
     double *eval;   int eval_cap;     /* levels (Eh), ascending                               */
     int *iv2;       int iv2_cap;      /* per-block selection counts (blocks in solve order)   */
