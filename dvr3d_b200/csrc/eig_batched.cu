@@ -961,7 +961,7 @@ void launch_eigvecs_batched(const BatchDesc &bd, double *A, const double *d, con
     int nwarp = 8;
     auto invit_smem = [&](int k) { return ((size_t)2 * np + (size_t)k * (5 * np + np / 8)) * sizeof(double); };
     while (nwarp > 1 && invit_smem(nwarp) > cap) --nwarp;
-    // 32 columns of Z a CTA where they fit (orders up to 536), else 16
+    // 32 columns of Z a CTA where they fit (orders up to 527), else 16
     auto bt_smem = [&](int nc, int zs) { return ((size_t)nc * zs + 8 * nc * 33 + 2 * nc * 36) * sizeof(double); };
     const int zs = (nmax + 32) / 16 * 16 + 4;  // 16-row tiles run past the end
     const bool wide = bt_smem(32, zs) <= cap + 24 * 1024;
