@@ -2,14 +2,14 @@
 // of DVR3DRJZ and ROTLEV3B): records framed by a 4-byte length before and after.
 #pragma once
 
+#include <climits>
 #include <cstdint>
+#include <cstdio>
 #include <cstring>
 #include <memory>
 #include <string>
 #include <utility>
 #include <vector>
-
-#include <cstdio>
 
 #include "../../include/dvr3d_b200.h"
 #include "host_setup.h"
@@ -24,10 +24,13 @@ struct Records {
     [[noreturn]] static void bad(const std::string &m) { throw HostError{DVR3D_ERR_ARG, m}; }
 
     explicit Records(const std::string &path) {
-        FILE *f = std::fopen(path.c_str(), "rb");
+        struct Close {
+            void operator()(FILE *f) const { std::fclose(f); }
+        };
+        const std::unique_ptr<FILE, Close> f(std::fopen(path.c_str(), "rb"));
         if (!f) bad("cannot open the wavefunction file " + path);
-        const size_t size = slurp(f);
-        std::fclose(f);
+        const size_t size = slurp(f.get());
+        if (std::ferror(f.get())) bad("cannot read the wavefunction file " + path);
         size_t pos = 0;
         while (pos + 8 <= size) {
             int32_t n = 0, m = 0;
@@ -47,7 +50,7 @@ struct Records {
         size_t cap = 1 << 16, size = 0;
         if (std::fseek(f, 0, SEEK_END) == 0) {
             const long end = std::ftell(f);
-            if (end > 0) cap = (size_t)end + 1;
+            if (end > 0 && end < LONG_MAX) cap = (size_t)end + 1;  // (a directory says LONG_MAX)
             std::rewind(f);
         }
         buf.reset(new unsigned char[cap]);
