@@ -817,8 +817,8 @@ cudaError_t launch_band_backtransform(const BandTri &t, double *Z, long long ldz
     auto need = [&](int cols) { return fixed + (size_t)cols * ldzs * sizeof(double); };
     // The kernel is bound by shared memory: a reflector costs a slab of 1, 2, 4, 8 columns some 16, 20,
     // 30, 52 passes over it (loads, stores, shuffles), slabs on one SM add up. The width with the
-    // fewest passes on the fullest SM: 330 columns in slabs of 4, on 83 SMs (order 1600: 1.9 ms; in
-    // slabs of 2, two on some SMs, 2.1), 100 columns one each.
+    // fewest passes on the fullest SM: 330 columns in slabs of 4, on 83 SMs (order 1600, a reflector at
+    // a time: 1.9 ms; in slabs of 2, two on some SMs, 2.1), 100 columns one each.
     static const int pass[4] = {16, 20, 30, 52};
     int cols = 0, best = 0;
     for (int q = 0; q < 4; ++q) {

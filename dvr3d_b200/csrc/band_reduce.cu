@@ -10,10 +10,10 @@
 //   w_kernel         W = X T + V M, and the next panel's columns of A2 - V W^T - W V^T;
 //   syr2k_kernel     the rest of A2 <- A2 - V W^T - W V^T (lower triangle).
 // 4/3 n^3 flop, nearly all in symm and syr2k on the FP64 tensor path (DMMA m16n8k16). The next panel
-// needs only what w_kernel makes, so it runs beside syr2k, on 16 of the SMs. At n = 12241 the whole
-// reduction to tridiagonal form with the chase takes 200 ms against 970 ms in one stage (symm 54,
-// syr2k with the panels beside it 69, vtx 6, w 4, chase 49); one after the other, with a cluster
-// barrier in every column of a panel, the same took 240.
+// needs only what w_kernel makes, so it runs beside syr2k, on 16 of the SMs. At n = 12202 the
+// reduction to the band takes 128 ms (symm 54, syr2k with the panels beside it 69, vtx 6, w 4) and the
+// chase 49, against 950 ms in one stage; one after the other, with a cluster barrier in every column
+// of a panel, the two stages took 240.
 #include <cooperative_groups.h>
 #include <cuda_runtime.h>
 

@@ -1,4 +1,5 @@
-// eig_batched.cu -- batched FP64 symmetric eigensolver kernels (one CTA per block).
+// eig_batched.cu -- batched FP64 symmetric eigensolver kernels: one or two CTAs a block in the
+// reduction, up to eight for the eigenvalues and sixteen for the inverse iteration.
 // See eig_batched.cuh for the role of each stage and the reference routines replaced.
 #include <cooperative_groups.h>
 
@@ -459,7 +460,7 @@ __global__ void __launch_bounds__(kEvThreads) eigvals_kernel(BatchDesc bd, const
 __device__ int g_invit_fail[4];
 
 // Eigenvectors of the tridiagonal matrices for the selected eigenvalues, as dstein: LU factors of
-// T - lambda I with partial pivoting, up to four solves, modified Gram-Schmidt inside clusters of
+// T - lambda I with partial pivoting, four solves, modified Gram-Schmidt inside clusters of
 // eigenvalues closer than 1e-6 ||T||. One warp per cluster with the factors and the iterate in its
 // slice of shared memory; lane 0 runs the recurrences eight rows at a time, operands first, so that
 // a row costs its dependent operations only. gridDim.y CTAs share a block's clusters. Bound by that

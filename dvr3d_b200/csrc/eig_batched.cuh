@@ -4,10 +4,10 @@
 // dsyev('V','L') (source/dvr3drjz_segmented.f90:2638-2659) in the 1D (jhmain :1987) and 2D
 // (jhmain :2030, nfmain :3077) stages. Only the eigenpairs that the energy cut-off keeps
 // are needed downstream, so the solver is split the way dsyevx is:
-//   1. Householder tridiagonalisation, one CTA per block (reflectors kept in the block);
-//   2. Sturm-count bisection: either the eigenvalues below a cut-off or all of them;
+//   1. Householder tridiagonalisation, one or two CTAs a block (reflectors kept in the block);
+//   2. Sturm-count multisection: either the eigenvalues below a cut-off or all of them;
 //   3. inverse iteration (with modified Gram-Schmidt inside clusters of close eigenvalues)
-//      for the selected eigenvalues only, then back-transformation by the reflectors.
+//      for the selected eigenvalues only, then back-transformation by block reflectors.
 // Every block lives in global memory (L2-resident for the sizes of the 1D/2D stages).
 #pragma once
 
