@@ -11,7 +11,7 @@
 //   syr2k_kernel     the rest of A2 <- A2 - V W^T - W V^T (lower triangle).
 // 4/3 n^3 flop, nearly all in symm and syr2k on the FP64 tensor path (DMMA m16n8k16). The next panel
 // needs only what w_kernel makes, so it runs beside syr2k, on 16 of the SMs. At n = 12202 the
-// reduction to the band takes 128 ms (symm 54, syr2k with the panels beside it 69, vtx 6, w 4) and the
+// reduction to the band takes 125 ms (symm 54, syr2k with the panels beside it 66, vtx 6, w 4) and the
 // chase 49, against 950 ms in one stage; one after the other, with a cluster barrier in every column
 // of a panel, the two stages took 240.
 #include <cooperative_groups.h>
@@ -694,16 +694,18 @@ __global__ void __launch_bounds__(kThr) w_kernel(double *VWV, long long ldv, con
 }
 
 // ------------------------------------------------------------------ A -= V W^T + W V^T
-constexpr size_t kSyrSmem = (size_t)2 * 64 * kSM * sizeof(double);
+constexpr size_t kSyrSmem = (size_t)3 * 64 * kSM * sizeof(double);
 constexpr int kSyrThr = 256;
 
 // One 64 x 64 tile of the lower triangle, K = 64: [V W] against [W V], which the buffer V W V
-// holds side by side. The accumulators start from -A, so A is read while the operands arrive. Eight
-// warps of 32 x 16 (four of 32 x 32 left fewer in flight: 48.7 -> 47.1 ms for the first 150 steps at
-// n = 12241): 20 TF/s, against 6.2 for the one-stage path's update.
+// holds side by side. The tile of A comes into shared memory behind the operands and the products'
+// sum is subtracted from it once: accumulators that start from -A round at its magnitude 64 times
+// (levels of order 3984: 2.1e-16 hartree rms against 1.1e-16), and no faster (128 -> 125 ms for the
+// reduction at n = 12202). Eight warps of 32 x 16 (four of 32 x 32 left fewer in flight: 48.7 -> 47.1
+// ms for the first 150 steps at n = 12241): 20 TF/s, against 6.2 for the one-stage path's update.
 __global__ void __launch_bounds__(kSyrThr, 2) syr2k_band_kernel(double *A, long long lda, int R, const double *VWV, long long ldv) {
     extern __shared__ __align__(16) double sm[];
-    double *Xs = sm, *Ys = sm + 64 * kSM;
+    double *Xs = sm, *Ys = sm + 64 * kSM, *As = Ys + 64 * kSM;
     const long long t = blockIdx.x;
     int ti = (int)((sqrt(8.0 * (double)t + 1.0) - 1.0) * 0.5);
     while ((long long)ti * (ti + 1) / 2 > t) --ti;
@@ -719,17 +721,21 @@ __global__ void __launch_bounds__(kSyrThr, 2) syr2k_band_kernel(double *A, long 
         cp16(Ys + k * kSM + i, vj ? VWV + (size_t)(32 + k) * ldv + j0 + i : VWV, vj * 8);
     }
     asm volatile("cp.async.commit_group;\n" ::);
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+        const int e = tid + q * kSyrThr, j = e >> 5, i = (e & 31) * 2;
+        const int valid = (j0 + j < R) ? min(max(R - i0 - i, 0), 2) : 0;
+        cp16(As + j * kSM + i, valid ? A + (size_t)(j0 + j) * lda + i0 + i : A, valid * 8);
+    }
+    asm volatile("cp.async.commit_group;\n" ::);
     double acc[2][2][4];
 #pragma unroll
     for (int a = 0; a < 2; ++a)
 #pragma unroll
         for (int b = 0; b < 2; ++b)
 #pragma unroll
-            for (int h = 0; h < 4; ++h) {
-                const int i = i0 + wm + a * 16 + r + 8 * (h >> 1), j = j0 + wn + b * 8 + c * 2 + (h & 1);
-                acc[a][b][h] = (i < R && j <= i) ? -A[(size_t)j * lda + i] : 0.0;
-            }
-    asm volatile("cp.async.wait_group 0;\n" ::);
+            for (int h = 0; h < 4; ++h) acc[a][b][h] = 0.0;
+    asm volatile("cp.async.wait_group 1;\n" ::);
     __syncthreads();
 #pragma unroll
     for (int k0 = 0; k0 < 64; k0 += 16) {
@@ -747,14 +753,16 @@ __global__ void __launch_bounds__(kSyrThr, 2) syr2k_band_kernel(double *A, long 
 #pragma unroll
             for (int b = 0; b < 2; ++b) dmma16(acc[a][b], af[a], bf[b]);
     }
+    asm volatile("cp.async.wait_group 0;\n" ::);
+    __syncthreads();
 #pragma unroll
     for (int a = 0; a < 2; ++a)
 #pragma unroll
         for (int b = 0; b < 2; ++b)
 #pragma unroll
             for (int h = 0; h < 4; ++h) {
-                const int i = i0 + wm + a * 16 + r + 8 * (h >> 1), j = j0 + wn + b * 8 + c * 2 + (h & 1);
-                if (i < R && j <= i) A[(size_t)j * lda + i] = -acc[a][b][h];
+                const int i = wm + a * 16 + r + 8 * (h >> 1), j = wn + b * 8 + c * 2 + (h & 1);
+                if (i0 + i < R && j0 + j <= i0 + i) A[(size_t)(j0 + j) * lda + i0 + i] = As[j * kSM + i] - acc[a][b][h];
             }
 }
 

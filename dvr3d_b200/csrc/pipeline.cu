@@ -718,10 +718,10 @@ void dense_lowest_two_stage(dvr3d_ctx *ctx, double *A, long long lda, int n, int
 void dense_lowest(dvr3d_ctx *ctx, double *A, long long lda, int n, int nev, bool vecs, double *w, double *Z,
                   long long ldz, const char *tag, bool time_panels, DenseOut *out) {
     // Two stages at every order (levels only; order 12: 0.18 -> 0.09 ms, 40: 0.56 -> 0.20, 128: 1.85 ->
-    // 0.67, 924: 14.4 -> 5.8, 3984: 102 -> 28.6, 12202: 953 -> 181 ms); one stage for orders that need
+    // 0.67, 924: 14.4 -> 5.8, 3984: 102 -> 28.6, 12202: 953 -> 179 ms); one stage for orders that need
     // no reflector, and for vectors whose columns the chase's back-transformation cannot hold in shared
     // memory (over kBandBackMax). The levels' rounding is coarser by the chase, which transforms every
-    // band element once a sweep: 4.0e-16 hartree rms at order 12202 where one stage has 0.7e-16, 2.1e-16
+    // band element once a sweep: 3e-16 hartree rms at order 12202 where one stage has 0.7e-16, 1.1e-16
     // against 0.3e-16 at 3984 (LAPACK's dsyevd there: 12e-16), all far below eps ||H||.
     if (n >= 3 && (!vecs || n <= kBandBackMax) && band_reduce_available()) {
         dense_lowest_two_stage(ctx, A, lda, n, nev, vecs, w, Z, ldz, tag, time_panels, out);
