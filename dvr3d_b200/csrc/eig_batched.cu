@@ -20,7 +20,9 @@ namespace {
 // Lower Householder reduction as dsytd2('L'): for k = 0..n-3 the reflector H_k = I - tau_k v v^T,
 // v = (0..0, 1, v_{k+2..n-1}), annihilates A[k+2:, k]. Columns are formed in panels of eight from the
 // panel-start matrix (the dlatrd scheme: A v needs one read of the trailing matrix and no write; the
-// matrix itself is updated once a panel, a rank-16 DMMA product over both triangles). A column k is a
+// matrix itself is updated once a panel, a rank-16 DMMA product over both triangles, subtracted from it
+// as a whole: accumulators that start from the matrix round at its magnitude sixteen times, which
+// doubled the vectors' errors, 9.8e-14 against 4.4e-14 rms for orders 160 to 459). A column k is a
 // chain, kept short: the product with the trailing matrix and the panel's dot products use the
 // column x itself and run beside its norm (v = e_{k+1} + sc x), every thread forms the reflector's
 // scalars, and three block barriers and one exchange are left. A cluster of C CTAs shares a block:
@@ -66,28 +68,26 @@ __global__ void __launch_bounds__(1024) tridiag_kernel(BatchDesc bd, double *A, 
                 double af[8];
 #pragma unroll
                 for (int h = 0; h < 8; ++h) af[h] = ((h >> 2) ? W : V)[(t + 4 * ((h >> 1) & 1)) * ns + r0 + g + 8 * (h & 1)];
-                double acc[2][4];
+                double old[2][4];
 #pragma unroll
                 for (int y = 0; y < 2; ++y)
 #pragma unroll
                     for (int h = 0; h < 4; ++h) {
                         const int r = r0 + g + 8 * (h >> 1), c = c0 + 8 * y + 2 * t + (h & 1);
-                        acc[y][h] = (r < n && c < n) ? -get(r, c) : 0.0;
+                        old[y][h] = (r < n && c < n) ? get(r, c) : 0.0;
                     }
 #pragma unroll
                 for (int y = 0; y < 2; ++y) {
-                    double bf[4];
+                    double bf[4], acc[4] = {0.0, 0.0, 0.0, 0.0};
 #pragma unroll
                     for (int h = 0; h < 4; ++h) bf[h] = ((h >> 1) ? V : W)[(t + 4 * (h & 1)) * ns + c0 + 8 * y + g];
-                    dmma16(acc[y], af, bf);
-                }
-#pragma unroll
-                for (int y = 0; y < 2; ++y)
+                    dmma16(acc, af, bf);
 #pragma unroll
                     for (int h = 0; h < 4; ++h) {
                         const int r = r0 + g + 8 * (h >> 1), c = c0 + 8 * y + 2 * t + (h & 1);
-                        if (r < n && c < n) ag[(size_t)c * n + r] = -acc[y][h];
+                        if (r < n && c < n) ag[(size_t)c * n + r] = old[y][h] - acc[h];
                     }
+                }
             }
             exchange();
             acol = (row >= k && row < n) ? get(row, k) : 0.0;
