@@ -757,7 +757,8 @@ __global__ void __launch_bounds__(128) bt_factor_kernel(BatchDesc bd, double *A,
 }
 
 // NC columns of Z a CTA, kept in shared memory ([column][row], stride 4 mod 16) through all panels:
-// W = V^T Z (rows split over the eight warps), W2 = T W, Z -= V W2.
+// W = V^T Z (rows split over the eight warps), W2 = T W, Z -= V W2 (the products summed first: Z is
+// rounded once a panel, not once a reflector).
 template <int NC>
 __global__ void __launch_bounds__(256) bt_apply_kernel(BatchDesc bd, const double *A, const int *sel, const long long *zoff,
                                                        const int *zld, double *Z, int zs) {
@@ -840,7 +841,7 @@ __global__ void __launch_bounds__(256) bt_apply_kernel(BatchDesc bd, const doubl
 #pragma unroll
             for (int y = 0; y < NT; ++y)
 #pragma unroll
-                for (int h = 0; h < 4; ++h) acc[y][h] = zt[(size_t)(y * 8 + c * 2 + (h & 1)) * zs + i0 + r + 8 * (h >> 1)];
+                for (int h = 0; h < 4; ++h) acc[y][h] = 0.0;
 #pragma unroll
             for (int k0 = 0; k0 < 32; k0 += 16) {
                 double af[8];
@@ -857,7 +858,7 @@ __global__ void __launch_bounds__(256) bt_apply_kernel(BatchDesc bd, const doubl
 #pragma unroll
             for (int y = 0; y < NT; ++y)
 #pragma unroll
-                for (int h = 0; h < 4; ++h) zt[(size_t)(y * 8 + c * 2 + (h & 1)) * zs + i0 + r + 8 * (h >> 1)] = acc[y][h];
+                for (int h = 0; h < 4; ++h) zt[(size_t)(y * 8 + c * 2 + (h & 1)) * zs + i0 + r + 8 * (h >> 1)] += acc[y][h];
         }
         __syncthreads();
     }

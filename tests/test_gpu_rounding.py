@@ -105,3 +105,10 @@ def test_vectors_of_blocks(batched):
     every column of the panel)."""
     ours, theirs = batched
     assert ours[0] <= 1.5 * theirs[0]
+
+
+def test_residuals_of_blocks(batched):
+    """The back-transformation rounds a vector once a panel of 32 reflectors: residuals of 0.43 times
+    torch's measured, 0.48 and 0.50 where it rounds once a reflector."""
+    ours, theirs = batched
+    assert ours[1] <= 0.46 * theirs[1]
